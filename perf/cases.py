@@ -181,3 +181,70 @@ def tolerance(case):
     if case["router"] == "inside":
         return {"rel": 5e-3, "max": 0.9}
     return {"rel": 4e-3, "max": 4e-2}
+
+
+EXACT_FLOPS = 2.2e11                         # beyond this the 64-bit computation takes too long
+
+
+def exact(case, seed):
+    """The layer in 64 bits with the quantisation points that the FP8 path has by definition (activations and
+    intermediate to e4m3 per 128 columns); nothing else is rounded."""
+    if work(case)["flops"] > EXACT_FLOPS:
+        return None
+    spec, width, local = GEOMETRY[case["variant"]]
+    s = prepare(case, seed)
+    mode = ROUTER_MODE.get(case["variant"], spec.router_mode)
+    hs, layer = s["hs"].double(), s["layer"]
+    logits = s["logits"].double() if s["rw"] is None else hs @ s["rw"].double().t()
+    ids, weights = _route(logits, mode, s["bias"], spec)
+    x = _through_e4m3(hs)
+    owner = s["emap"].long() if s["emap"] is not None else torch.arange(spec.experts, device=hs.device)
+    ids = owner[ids]
+    out = torch.zeros_like(hs)
+    for e in torch.unique(ids).tolist():
+        if e >= 0:
+            tok, slot = (ids == e).nonzero(as_tuple=True)
+            y = _expert(x[tok], layer["w13"][e], layer["w13_scale"][e], layer["w2"][e], layer["w2_scale"][e])
+            out.index_add_(0, tok, y * weights[tok, slot, None])
+    out *= s["scale"] if s["shared"] is not None else 1.0
+    if s["shared"] is not None:
+        sh, (part, parts) = s["shared"], s["part"]
+        tok = (torch.arange(len(hs), device=hs.device) // 128 % parts == part).nonzero(as_tuple=True)[0]
+        y = _expert(x[tok], sh["w13"], sh["w13_scale"], sh["w2"], sh["w2_scale"])
+        if sh.get("gate") is not None:
+            y *= torch.sigmoid(hs[tok] @ sh["gate"].double())[:, None]
+        out.index_add_(0, tok, y)
+    return out
+
+
+def _route(logits, mode, bias, spec):
+    if mode == 0:
+        score = sel = torch.softmax(logits, dim=-1)
+    else:
+        score = torch.sigmoid(logits)
+        sel = score + bias.double()
+    if mode == 2:
+        groups = sel.unflatten(1, (spec.n_group, -1))
+        best = groups.topk(2, dim=-1).values.sum(-1).topk(spec.topk_group, dim=-1).indices
+        keep = torch.zeros(groups.shape[:2], dtype=torch.bool, device=sel.device).scatter_(1, best, True)
+        sel = groups.masked_fill(~keep[..., None], -math.inf).flatten(1)
+    ids = sel.topk(spec.top_k, dim=-1).indices
+    w = score.gather(1, ids)
+    return ids, w / w.sum(-1, keepdim=True)
+
+
+def _through_e4m3(x):
+    g = x.unflatten(-1, (-1, 128))
+    amax = g.abs().amax(-1, keepdim=True)
+    amax = torch.where(amax > 0, amax, 1.0)
+    return ((g * (448.0 / amax)).float().to(torch.float8_e4m3fn).double() * (amax / 448.0)).flatten(-2)
+
+
+def _weight(w, scale):
+    w = w.view(torch.float8_e4m3fn).double().unflatten(0, (-1, 128)).unflatten(2, (-1, 128))
+    return (w * scale.double()[:, None, :, None]).flatten(2).flatten(0, 1)
+
+
+def _expert(x, w13, s13, w2, s2):
+    gate, up = (x @ _weight(w13, s13).t()).chunk(2, dim=-1)
+    return _through_e4m3(torch.nn.functional.silu(gate) * up) @ _weight(w2, s2).t()
