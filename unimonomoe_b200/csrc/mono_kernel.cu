@@ -180,6 +180,13 @@ constexpr int TCOLS = NSPLIT * WC;       // accumulator columns (fp32 registers)
 constexpr int PASS_STRIDE = 128 / NSPLIT;  // intermediate columns covered by one buffer in the up projection
 constexpr int LDW = (WC <= 64) ? WC : HCB;  // TMEM columns per tcgen05.ld
 constexpr int NLD = WC / LDW;
+// One TMA request per weight stage where a stage is one MMA operand: for one SM alone the copy engine takes 861 cycles for
+// 32 KB as one box of 256 rows of 128 bytes and 1142 as four boxes of 64 rows. (The layer gains 0.5 % from it at every
+// batch size: with three stages a step is otherwise bound by what an SM takes in from L2, 48 KB of weights and rows.) A
+// box cannot interleave gate and up rows, so a stage of the up projection holds the pass's 128 gate rows and then its 128
+// up rows, and a warpgroup's columns of such a buffer are two pieces BC / 2 apart.
+constexpr bool ONE_BOX = !PAIR && NSPLIT == 1 && EPI_WGS == 2;
+constexpr int DOWN_BOX = ONE_BOX ? 256 : HCB;  // rows of a box of the down projection's weights
 static_assert(HCB == 32 || HCB == 64, "unsupported split of the accumulator between warpgroups");
 static_assert(LDW == 32 || LDW == 64, "TMEM loads are 32 or 64 columns wide");
 constexpr int N_EPI = EPI_WGS * 128;
@@ -1024,6 +1031,11 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
               }
               mbar_arrive_expect_tx(&S.fullB[st], (MONO_ABLATE & 16) ? 0 : B_STAGE_BYTES);
               if constexpr ((MONO_ABLATE & 16) != 0) { ++nb; continue; }
+              if constexpr (ONE_BOX) {
+                tma_load_3d(map_up, x, static_cast<uint32_t>(ch * CHUNK_COLS + ps * 128), static_cast<uint32_t>(2 * e), dst, &S.fullB[st]);
+                ++nb;
+                continue;
+              }
               // shared rows of buffer j, warpgroup h: [j*BC + h*WC, +HCB) gate columns c + j*PASS_STRIDE + h*HCB ..,
               // then the HCB matching up columns
 #pragma unroll
@@ -1056,7 +1068,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
               mbar_arrive_expect_tx(&S.fullB[st], (MONO_ABLATE & 16) ? 0 : B_STAGE_BYTES);
               if constexpr ((MONO_ABLATE & 16) != 0) { ++nb; continue; }
 #pragma unroll
-              for (int j = 0; j < 256 / HCB; ++j) tma_load_2d(map_down, x, y + j * HCB, dst + j * HCB * 128, &S.fullB[st]);
+              for (int j = 0; j < 256 / DOWN_BOX; ++j) tma_load_2d(map_down, x, y + j * DOWN_BOX, dst + j * DOWN_BOX * 128, &S.fullB[st]);
               ++nb;
             }
           }
@@ -1284,7 +1296,10 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       const int h = et >> 7;               // warpgroup: which WC columns of every accumulator buffer
       const int q = warp & 3;              // TMEM lane quarter this warp may read
       const int r = q * 32 + lane;         // row of the tile
-      const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(h * WC);
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+      // first column of piece c (LDW columns) of this warpgroup's part of an up- / down-projection buffer
+      auto up_col = [&](int c) -> uint32_t { return static_cast<uint32_t>(ONE_BOX ? h * HCB + c * (BC / 2) : h * WC + c * LDW); };
+      auto down_col = [&](int c) -> uint32_t { return static_cast<uint32_t>(h * WC + c * LDW); };
       uint32_t nt = 0;
       bool dead = false;  // after an abort: keep the loop structure (named barriers stay matched), skip the work
       // Accumulators, pairs of adjacent columns. Buffer j of a slab owns acc[j*WC/2, (j+1)*WC/2):
@@ -1301,7 +1316,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       // Read one accumulator buffer out of tensor memory and fold it into part j of the register
       // accumulators: acc += D * scale (s_lo for the first HCB columns, s_hi for the rest). The
       // buffer goes back to the MMA thread as soon as its contents are in registers.
-      auto promote = [&](int j, uint32_t buf, float s_lo, float s_hi) {
+      auto promote = [&](int j, uint32_t buf, float s_lo, float s_hi, auto col) {
         tc_fence_after();
         if constexpr ((MONO_ABLATE & 1) != 0) {
           tc_fence_before();
@@ -1312,7 +1327,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
 #pragma unroll
         for (int c = 0; c < NLD; ++c) {
           uint32_t v[LDW];
-          tmem_ld_n<LDW>(t_lane + buf * BC + c * LDW, v);
+          tmem_ld_n<LDW>(t_row + buf * BC + col(c), v);
           tmem_ld_wait();
           if (c == NLD - 1) {
             // one arrival per warp: per-thread arrivals on one shared-memory word serialise
@@ -1428,7 +1443,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
               PROF_ADD(pe_wait); PROF_HIST(0, (ks < 16 ? ks : 15), et == 0); }
               TRACE_E(1);
               PROF_T0();
-              if (!dead) promote(j, buf, s_g, s_u);
+              if (!dead) promote(j, buf, s_g, s_u, up_col);
               PROF_ADD(pe_up);
               TRACE_E(3);
               ++nt;
@@ -1526,7 +1541,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
               PROF_ADD(pe_wait); PROF_HIST(0, 16 + dk, et == 0); }
               TRACE_E(1);
               PROF_T0();
-              if (!dead) promote(j, buf, sc, sc);
+              if (!dead) promote(j, buf, sc, sc, down_col);
               PROF_ADD(pe_down);
               TRACE_E(3);
               ++nt;
@@ -1893,6 +1908,20 @@ int make_u8_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, 
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
+// Up-projection weights [experts][gate | up][N_HALF][K]: a box takes 128 gate rows and the 128 matching up rows.
+int make_up_map(CUtensorMap* m, const void* base, uint64_t rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return -1;
+  cuuint64_t gd[3] = {K_DIM, N_HALF, rows / N_HALF};
+  cuuint64_t gs[2] = {K_DIM, static_cast<cuuint64_t>(K_DIM) * N_HALF};
+  cuuint32_t bx[3] = {128u, 128u, 2u};
+  cuuint32_t es[3] = {1u, 1u, 1u};
+  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), gd, gs, bx, es,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
+}
+
 // 2-D bf16 tensor [rows, cols] row-major, box box_rows x 64 elements (128 bytes), 128-byte swizzle;
 // rows past the end read as zero.
 int make_bf16_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
@@ -1942,7 +1971,9 @@ int cached_map(CUtensorMap* dst, int kind, const void* base, uint64_t rows, uint
   }
   ++g_map_misses;
   CUtensorMap m;
-  const int rc = (kind <= 1) ? make_u8_map(&m, base, rows, cols, box_rows) : make_bf16_map(&m, base, rows, cols, box_rows);
+  const int rc = (ONE_BOX && kind == 0) ? make_up_map(&m, base, rows)
+                 : (kind <= 1)          ? make_u8_map(&m, base, rows, cols, box_rows)
+                                        : make_bf16_map(&m, base, rows, cols, box_rows);
   if (rc != 0) return rc;
   if (g_maps.size() >= kMaxCachedMaps) g_maps.clear();
   g_maps.emplace(key, m);
@@ -2031,7 +2062,7 @@ int prefill_wgmma_plan_prepare(const uint8_t* up_w_fp8, const uint8_t* down_w_fp
   if (up_w_fp8 == nullptr || down_w_fp8 == nullptr) return -104;
   CUtensorMap tmp;
   if (cached_map(&tmp, 0, up_w_fp8, static_cast<uint64_t>(E_LOCAL) * N_UP, K_DIM, HCB) != 0) return -2;
-  if (cached_map(&tmp, 1, down_w_fp8, static_cast<uint64_t>(E_LOCAL) * H_DIM, N_HALF, HCB) != 0) return -3;
+  if (cached_map(&tmp, 1, down_w_fp8, static_cast<uint64_t>(E_LOCAL) * H_DIM, N_HALF, DOWN_BOX) != 0) return -3;
   int dev = 0;
   cudaError_t err = cudaGetDevice(&dev);
   if (err == cudaSuccess) err = ensure_kernel_attribute(dev);
@@ -2149,7 +2180,7 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
     fprintf(stderr, "up-projection tensor map failed: %d\n", rc);
     return -2;
   }
-  rc = cached_map(&p.tm_down, 1, down_w_fp8, static_cast<uint64_t>(E_LOCAL) * H_DIM, N_HALF, HCB);
+  rc = cached_map(&p.tm_down, 1, down_w_fp8, static_cast<uint64_t>(E_LOCAL) * H_DIM, N_HALF, DOWN_BOX);
   if (rc != 0) {
     fprintf(stderr, "down-projection tensor map failed: %d\n", rc);
     return -3;
@@ -2163,7 +2194,7 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
     p.sh_part = sh->part;
     p.sh_parts = sh->parts;
     rc = cached_map(&p.tm_sh_up, 0, sh->up_w_fp8, static_cast<uint64_t>(N_UP), K_DIM, HCB);
-    if (rc == 0) rc = cached_map(&p.tm_sh_down, 1, sh->down_w_fp8, static_cast<uint64_t>(H_DIM), N_HALF, HCB);
+    if (rc == 0) rc = cached_map(&p.tm_sh_down, 1, sh->down_w_fp8, static_cast<uint64_t>(H_DIM), N_HALF, DOWN_BOX);
     if (rc != 0) {
       fprintf(stderr, "shared-expert tensor map failed: %d\n", rc);
       return -5;

@@ -82,6 +82,16 @@ __device__ __forceinline__ void tma_load_2d(const CUtensorMap* m, uint32_t x, ui
       : "memory");
 }
 
+// Three-dimensional form of tma_load_2d: one request for rows that are not adjacent in global memory.
+__device__ __forceinline__ void tma_load_3d(const CUtensorMap* m, uint32_t x, uint32_t y, uint32_t z, void* dst,
+                                            uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
+}
+
 // ---------------------------------------------------------------- cp.async (16 B, L2 only)
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
