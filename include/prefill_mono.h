@@ -15,7 +15,7 @@
  *
  * Return codes of the launch entry points (Q:1569-1599, Q:1621-1638, EP:1658-1659):
  *     0      launched
- *  -100      workspace null or smaller than prefill_wgmma_workspace_bytes()
+ *  -100      workspace null or smaller than every launch needs (230 KB)
  *  -101      num_tokens <= 0
  *  -102      num_tokens*top_k/128 + local experts exceeds prefill_wgmma_max_tiles()
  *  -103      device has fewer SMs than prefill_wgmma_grid_size()
@@ -32,7 +32,10 @@
  *
  * Buffers (T = num_tokens, k = top_k = 8, E = 256 routed experts, El = local experts):
  *   logits            fp32 [T, E]                      in
- *   workspace         >= prefill_wgmma_workspace_bytes(); zeroed by the launch itself
+ *   workspace         prefill_wgmma_workspace_bytes(); zeroed by the launch itself as far as it has to be. The part
+ *                     behind the first 230 KB holds the intermediate of the split form (short batches); a smaller
+ *                     workspace, or one that is not 16-byte aligned, is accepted and does without that form: the same
+ *                     bits, later
  *   act_bf16          bf16 [T, K]                      in
  *   act_fp8           u8   [T, K]                      scratch/out: e4m3 activations
  *   act_scales        fp32 [T, K/128]                  scratch/out

@@ -38,6 +38,7 @@
 #include <cuda_runtime.h>
 
 #include <cfloat>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -197,6 +198,18 @@ constexpr int N_GATHER = 64;
 constexpr int MAX_MY_TILES = 32 * NCH;
 constexpr int MAX_TILES = MAX_MY_TILES * kGrid;
 
+// ------------------------------------------------------------------ the split form of the expert phase
+// A unit of the schedule (one tile, all of its passes) keeps one CTA busy for NP * NK + NHB * NP slab steps. That is
+// right for long batches. In a short one there are fewer units than SMs (one token: 8 units of 148), or a second round
+// of them that is nearly empty, and a unit of a few rows is bound by how fast its one CTA can load weights.
+// The split form cuts the units into their passes and deals those evenly over all CTAs, twice: first every (unit,
+// 128-column pass of the up projection), whose e4m3 result and scales go to global memory; then, behind a grid-wide
+// counter, every (unit, 256-column pass of the down projection). The intermediate leaves shared memory, and the weight
+// ring takes its place. The operations on a row and their order are those of the whole unit: the same bits come out.
+constexpr bool SPLIT_BUILD = ONE_BOX && MONO_ABLATE == 0;
+constexpr size_t SPLIT_ROW_BYTES = N_HALF + NPT * sizeof(float);  // e4m3 intermediate and its scales, one row
+constexpr int SPLIT_ROWS = SPLIT_BUILD ? kGrid * TILE_M : 0;      // rows of the global intermediate
+
 // ------------------------------------------------------------------ shared memory plan
 constexpr int A_STAGE_BYTES = TILE_M * 128;  // 128 rows x 128 B
 constexpr int B_ROWS = PAIR ? 128 : 256;     // weight rows of a stage kept by one CTA
@@ -222,6 +235,14 @@ constexpr int SA = SA_RAW > STAGE_CAP ? STAGE_CAP : SA_RAW;
 static_assert(SB >= 2 && SA >= 2, "intermediate too wide for shared memory: shard N_HALF further");
 constexpr int DYN_SMEM = 1024 + INTER_BYTES + SA * A_STAGE_BYTES + SB * B_STAGE_BYTES + SCALE_BYTES;
 static_assert(NWARPS * E * 4 <= SA * A_STAGE_BYTES, "phase-0 histograms live in the activation ring");
+// split form: no intermediate and no scale staging in shared memory, so the weight ring is deeper
+constexpr int SPLIT_SA = 3;
+constexpr int SPLIT_SB = (SMEM_CAP - SMEM_STATIC_RESERVE - 1024 - SPLIT_SA * A_STAGE_BYTES) / B_STAGE_BYTES;
+constexpr int SPLIT_DYN_SMEM = 1024 + SPLIT_SA * A_STAGE_BYTES + SPLIT_SB * B_STAGE_BYTES;
+constexpr int A_STAGE_CAP = SPLIT_SA > STAGE_CAP ? SPLIT_SA : STAGE_CAP;
+constexpr int B_STAGE_CAP = SPLIT_SB > STAGE_CAP ? SPLIT_SB : STAGE_CAP;
+static_assert(!SPLIT_BUILD || (NWARPS * E * 4 <= SPLIT_SA * A_STAGE_BYTES && SPLIT_SB >= 3),
+              "phases R to 1 use the rings of the split form as they use the others");
 
 // Register budget (setmaxnreg). The kernel launches with REGS_LAUNCH registers per thread; the
 // producer warpgroup gives registers back and the epilogue warpgroups take them. The
@@ -242,7 +263,8 @@ constexpr uint32_t IDESC = umma_idesc_e4m3_f32(PAIR ? 256 : 128, BC);
 // router GEMV: one [128 tokens x 256 experts] accumulator, K slabs of 64 bf16 (128 bytes)
 constexpr uint32_t IDESC_ROUTER = umma_idesc_bf16_f32(128, E);
 constexpr int RK = K_DIM / 64;
-constexpr int RS = (SA < SB) ? SA : SB;
+
+constexpr uint32_t kSplitCounter = 3;  // workspace counter between the halves of the split form (0-2: grid barriers)
 
 // wait sites reported in the status word
 enum Site : uint32_t {
@@ -276,6 +298,10 @@ struct Params {
   const __nv_bfloat16* residual;
   float out_scale;
   uint64_t timeout_ns;
+  // split form: intermediate rows [sp_rows, N_HALF] e4m3 and their scales [sp_rows, N_HALF / 128]
+  uint8_t* sp_inter;
+  float* sp_scale;
+  int sp_rows;
   // optional debug dump (null in production): raw gate|up accumulators, e4m3 intermediate, its scales
   float* dbg_acc;
   uint8_t* dbg_inter;
@@ -570,7 +596,7 @@ __device__ __forceinline__ size_t wsd_index(int e, int chunk, int i) {
 
 // ------------------------------------------------------------------ shared state
 struct __align__(16) SharedState {
-  uint64_t fullA[STAGE_CAP], emptyA[STAGE_CAP], fullB[STAGE_CAP], emptyB[STAGE_CAP];
+  uint64_t fullA[A_STAGE_CAP], emptyA[A_STAGE_CAP], fullB[B_STAGE_CAP], emptyB[B_STAGE_CAP];
   uint64_t tmem_full[NBUF], tmem_empty[NBUF];
   uint64_t inter_ready[4];  // one per 128-column pass of the intermediate (NP <= 4)
   uint64_t rfull[4], rempty[4], racc_full, racc_empty;  // phase R only
@@ -578,7 +604,10 @@ struct __align__(16) SharedState {
   uint32_t flag;          // grid_sync result broadcast
   int n_my_tiles;
   int total_tiles;
+  int sp_units, sp_wave_units;   // split form: units in all, and units whose intermediate fits at a time
+  uint32_t sp_flag, sp_gflag;    // split form: counter reached (epilogue, gather warps)
   TileInfo tiles[MAX_MY_TILES];
+  int sp_row0[MAX_MY_TILES];     // split form: the tile's first row in the global intermediate
   float rowmax[2][EPI_WGS][TILE_M];
   alignas(16) int gather_tok[2][8][TILE_M / 8];  // token of row gr + 8 i of the tile being gathered, [tile parity][gr][i]
 #ifdef MONO_PROFILE
@@ -589,7 +618,416 @@ struct __align__(16) SharedState {
 };
 static_assert(sizeof(SharedState) <= SMEM_STATIC_RESERVE, "static shared state exceeds its reserve");
 
+// ------------------------------------------------------------------ pieces of the split form's epilogue
+// (The whole-unit loop has the same sections in line: with these functions called there the expert phase of the H = 7168
+// build took 3 % longer at 16384 tokens, its loop has no register to spare.)
+// SiLU(gate) * up (kernel/qwen_tp/src/prefill_mono_final_nb.cu:678), written over the gate columns; returns the amax
+// of this thread's columns.
+__device__ __forceinline__ float silu_mul(float2 (&acc)[TCOLS / 2]) {
+  float mx = 0.f;
+#pragma unroll
+  for (int j = 0; j < ((MONO_ABLATE & 2) ? 0 : NSPLIT); ++j) {
+#pragma unroll
+    for (int i = 0; i < HCB / 2; ++i) {
+      const float2 g = acc[j * (WC / 2) + i], u = acc[j * (WC / 2) + HCB / 2 + i];
+      // the reference's form (exp and division on the special-function unit). A tanh.approx form needs one
+      // special-function operation instead of two and is 15 us faster per layer, but its 2^-11 relative error
+      // moves enough e4m3 codes of the intermediate to push about one output in 10^5 beyond 2e-2 rms
+      const float v0 = __fdividef(u.x * g.x, 1.0f + __expf(-g.x));
+      const float v1 = __fdividef(u.y * g.y, 1.0f + __expf(-g.y));
+      acc[j * (WC / 2) + i] = make_float2(v0, v1);
+      mx = fmaxf(mx, fmaxf(fabsf(v0), fabsf(v1)));
+    }
+  }
+  return mx;
+}
+__device__ __forceinline__ uint4 pack_e4m3x16(const float2* a, float inv) {
+  uint4 qv;
+  qv.x = pack_e4m3x4(a[0].x * inv, a[0].y * inv, a[1].x * inv, a[1].y * inv);
+  qv.y = pack_e4m3x4(a[2].x * inv, a[2].y * inv, a[3].x * inv, a[3].y * inv);
+  qv.z = pack_e4m3x4(a[4].x * inv, a[4].y * inv, a[5].x * inv, a[5].y * inv);
+  qv.w = pack_e4m3x4(a[6].x * inv, a[6].y * inv, a[7].x * inv, a[7].y * inv);
+  return qv;
+}
+// The accumulators of a down pass times the routing weight, as bf16 into columns col0 .. of the partial row.
+__device__ __forceinline__ void store_rows(const Params& p, const float2 (&acc)[TCOLS / 2], int fi, float2 rw2, int chunk, int col0, bool ok) {
+  const int lane = threadIdx.x & 31;
+  // Neighbouring lanes swap half of their 32-byte pieces first, so that in every store instruction
+  // lanes 2i and 2i+1 write 64 contiguous bytes of ONE row: 16 lines per instruction instead of 32.
+  // (the guard is made warp-uniform: the shuffles below need every lane of the warp)
+  if (__all_sync(0xFFFFFFFFu, ok) && (MONO_ABLATE & 4) == 0) {
+    const bool odd = (lane & 1) != 0;
+    const int fi_even = __shfl_sync(0xFFFFFFFFu, fi, lane & ~1), fi_odd = __shfl_sync(0xFFFFFFFFu, fi, lane | 1);
+    __nv_bfloat16* row_even = p.partial + (static_cast<size_t>(fi_even < 0 ? 0 : fi_even) * NCH + chunk) * H_DIM + col0;
+    __nv_bfloat16* row_odd = p.partial + (static_cast<size_t>(fi_odd < 0 ? 0 : fi_odd) * NCH + chunk) * H_DIM + col0;
+#pragma unroll
+    for (int j = 0; j < NSPLIT; ++j) {
+      __nv_bfloat16* dst_even = row_even + j * BC;
+      __nv_bfloat16* dst_odd = row_odd + j * BC;
+#pragma unroll
+      for (int k2 = 0; k2 < WC / 32; ++k2) {   // pieces 2*k2 and 2*k2+1 of this thread's WC columns of buffer j
+        uint32_t lo[8], hi[8], mine[8], theirs[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float2 a = __fmul2_rn(acc[j * (WC / 2) + (2 * k2) * 8 + i], rw2);
+          const float2 b = __fmul2_rn(acc[j * (WC / 2) + (2 * k2 + 1) * 8 + i], rw2);
+          lo[i] = cvt_bf16x2_satfinite(a.x, a.y);
+          hi[i] = cvt_bf16x2_satfinite(b.x, b.y);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          // an even lane keeps its piece 2*k2 and gives away 2*k2+1; an odd lane the other way round
+          const uint32_t send = odd ? lo[i] : hi[i];
+          theirs[i] = (MONO_ABLATE & 256) ? send : __shfl_xor_sync(0xFFFFFFFFu, send, 1);
+          mine[i] = odd ? hi[i] : lo[i];
+        }
+        const int piece = 2 * k2 + (odd ? 1 : 0);
+        // row of the even lane: its own piece from the even lane, the received one from the odd lane
+        if (fi_even >= 0) st_global_256_stream(dst_even + piece * 16, odd ? theirs : mine);
+        if (fi_odd >= 0) st_global_256_stream(dst_odd + piece * 16, odd ? mine : theirs);
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------ the split form
+// What CTA `bid` takes of wave w: the units [lo, hi) of the wave its passes belong to (kept from slot0 of its list),
+// the passes [a0, a1) of the up and [b0, b1) of the down projection, counted over the wave's units. Contiguous shares
+// that differ by at most one pass: the passes of one unit mostly follow one another on one CTA.
+struct SplitShare {
+  int lo, hi, slot0, a0, a1, b0, b1;
+};
+__device__ __forceinline__ SplitShare split_share(int w, int wave_units, int units, int bid) {
+  const int n = min(wave_units, units - w * wave_units);
+  SplitShare s;
+  s.lo = bid * n / kGrid;
+  s.hi = ((bid + 1) * n + kGrid - 1) / kGrid;
+  s.slot0 = w * (((bid + 1) * wave_units + kGrid - 1) / kGrid - bid * wave_units / kGrid);  // the waves before w are full
+  s.a0 = bid * (n * NP) / kGrid;
+  s.a1 = (bid + 1) * (n * NP) / kGrid;
+  s.b0 = bid * (n * NHB) / kGrid;
+  s.b1 = (bid + 1) * (n * NHB) / kGrid;
+  return s;
+}
+
+// Phase 2 in the split form, with the roles of the whole-unit form. Both halves are the same slab step (weights
+// through one ring, rows through the other). The weights of the down passes do not depend on the up passes, so the
+// TMA and the MMA warp run through the counter between the halves; the gather warps and the epilogue wait at it.
+__device__ __forceinline__ void split_phase(const Params& p, SharedState& S, const WaitCtx& wc, uint8_t* a_ring, uint8_t* b_ring,
+                                            uint32_t tmem_base) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, bid = blockIdx.x;
+  const int units = S.sp_units, wave_units = S.sp_wave_units;
+  const int waves = (units + wave_units - 1) / wave_units;
+  const int numel = p.num_tokens * TOP_K;
+  Workspace* ws = p.ws;
+  const uint32_t a_ring_u32 = smem_u32(a_ring), b_ring_u32 = smem_u32(b_ring);
+  if (warp < 4) {
+    reg_dec<REGS_PRODUCER>();
+    if (warp == WARP_TMA) {
+      if (lane == 0) {
+        tma_prefetch_desc(&p.tm_up);
+        tma_prefetch_desc(&p.tm_down);
+        uint32_t nb = 0;
+        auto stage = [&]() -> uint8_t* {   // the next free stage, its bytes announced; null on abort
+          const uint32_t st = nb % SPLIT_SB;
+          if (!mbar_wait(&S.emptyB[st], ((nb / SPLIT_SB) & 1u) ^ 1u, wc, kSiteEmptyB)) return nullptr;
+          mbar_arrive_expect_tx(&S.fullB[st], B_STAGE_BYTES);
+          return b_ring + st * B_STAGE_BYTES;
+        };
+        bool ok = true;
+        for (int w = 0; w < waves && ok; ++w) {
+          const SplitShare my = split_share(w, wave_units, units, bid);
+          for (int u = my.a0; u < my.a1 && ok; ++u) {
+            const TileInfo ti = S.tiles[my.slot0 + u / NP - my.lo];
+            const bool sh = ti.e == SHARED_E;
+            for (int ks = 0; ks < NK; ++ks, ++nb) {
+              uint8_t* dst = stage();
+              if (dst == nullptr) { ok = false; break; }
+              tma_load_3d(sh ? &p.tm_sh_up : &p.tm_up, ks * 128, ti.chunk * CHUNK_COLS + u % NP * 128, sh ? 0 : 2 * ti.e, dst,
+                          &S.fullB[nb % SPLIT_SB]);
+            }
+          }
+          for (int u = my.b0; u < my.b1 && ok; ++u) {
+            const TileInfo ti = S.tiles[my.slot0 + u / NHB - my.lo];
+            const bool sh = ti.e == SHARED_E;
+            for (int dk = 0; dk < NP; ++dk, ++nb) {
+              uint8_t* dst = stage();
+              if (dst == nullptr) { ok = false; break; }
+              tma_load_2d(sh ? &p.tm_sh_down : &p.tm_down, (ti.chunk * NP + dk) * 128, (sh ? 0 : ti.e) * H_DIM + u % NHB * 256,
+                          dst, &S.fullB[nb % SPLIT_SB]);
+            }
+          }
+        }
+      }
+    } else if (warp == WARP_MMA) {
+      int steps = 0;
+      for (int w = 0; w < waves; ++w) {
+        const SplitShare my = split_share(w, wave_units, units, bid);
+        steps += (my.a1 - my.a0) * NK + (my.b1 - my.b0) * NP;
+      }
+      for (uint32_t n = 0; n < static_cast<uint32_t>(steps); ++n) {
+        const uint32_t sb = n % SPLIT_SB, sa = n % SPLIT_SA, buf = n % NBUF;
+        if (!mbar_wait_warp(&S.fullB[sb], (n / SPLIT_SB) & 1u, wc, kSiteFullB) ||
+            !mbar_wait_warp(&S.fullA[sa], (n / SPLIT_SA) & 1u, wc, kSiteFullA) ||
+            !mbar_wait_warp(&S.tmem_empty[buf], ((n / NBUF) & 1u) ^ 1u, wc, kSiteTmemEmpty))
+          break;
+        // the gathered rows were written by cp.async (generic proxy); the tensor core reads them through the async proxy
+        fence_proxy_async_smem();
+        tc_fence_after();
+        const uint64_t da = umma_desc_sw128(a_ring_u32 + sa * A_STAGE_BYTES);
+        const uint64_t db = umma_desc_sw128(b_ring_u32 + sb * B_STAGE_BYTES);
+        if (elect_one_sync()) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_f8(tmem_base + buf * BC, da + 2u * k, db + 2u * k, IDESC, k > 0 ? 1u : 0u);
+          umma_commit(&S.tmem_full[buf]);
+          umma_commit(&S.emptyA[sa]);
+          umma_commit(&S.emptyB[sb]);
+        }
+        __syncwarp();
+      }
+    } else {
+      // gather, lanes and swizzle as in the whole-unit form: thread g copies 16-byte piece g % 8 of rows g / 8 + 8 i
+      const int gt = tid - WARP_GATHER0 * 32, gc = gt & 7, gr = gt >> 3;
+      constexpr int ROWS_PER_THREAD = TILE_M / 8;
+      const uint32_t dst0 = a_ring_u32 + gr * 128 + ((gc ^ gr) << 4);
+      uint32_t na = 0;
+      int fills = 0;
+      bool dead = false;  // after an abort: the named barriers stay matched, the work is skipped
+      for (int w = 0; w < waves; ++w) {
+        const SplitShare my = split_share(w, wave_units, units, bid);
+        int cur = -1;
+        for (int u = my.a0; u < my.a1; ++u) {
+          const int slot = my.slot0 + u / NP - my.lo;
+          if (slot != cur) {   // the passes of one unit follow one another: its tokens are looked up once
+            cur = slot;
+            ++fills;
+            const TileInfo ti = S.tiles[slot];
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+              const int r = gt + hh * 64;
+              int t = -1;
+              if (r < ti.rows) {
+                if (ti.e == SHARED_E) {
+                  t = ti.row0 + r;
+                } else {
+                  const int fi = __ldcg(&p.sorted_ids[ti.row0 + r]);
+                  if (fi >= 0 && fi < numel) t = fi / TOP_K;
+                }
+              }
+              S.gather_tok[fills & 1][r & 7][r >> 3] = t;
+            }
+            named_bar_sync(2, N_GATHER);
+          }
+          for (int ks = 0; ks < NK; ++ks) {
+            const uint32_t sa = na % SPLIT_SA;
+            if (!dead && !mbar_wait(&S.emptyA[sa], ((na / SPLIT_SA) & 1u) ^ 1u, wc, kSiteEmptyA)) dead = true;
+            if (dead) continue;
+            const uint8_t* g0 = p.act_fp8 + ks * 128 + gc * 16;
+#pragma unroll
+            for (int i4 = 0; i4 < ROWS_PER_THREAD / 4; ++i4) {
+              const int4 t4 = *reinterpret_cast<const int4*>(&S.gather_tok[fills & 1][gr][4 * i4]);
+              const int tok[4] = {t4.x, t4.y, t4.z, t4.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (tok[i] >= 0) cp_async16(dst0 + sa * A_STAGE_BYTES + (4 * i4 + i) * 1024, g0 + static_cast<size_t>(tok[i]) * K_DIM);
+            }
+            cp_async_arrive_noinc(&S.fullA[sa]);
+            ++na;
+          }
+        }
+        if (gt == 0) {   // the intermediate of every unit of the wave is in global memory
+          S.sp_gflag = wait_counter_ge(&ws->barrier[kSplitCounter], static_cast<uint32_t>((2 * w + 1) * kGrid), wc, kErrGridBarrier,
+                                       kSplitCounter) ? 1u : 0u;
+          __threadfence();
+        }
+        named_bar_sync(2, N_GATHER);
+        if (S.sp_gflag == 0u) dead = true;
+        for (int u = my.b0; u < my.b1; ++u) {
+          const TileInfo ti = S.tiles[my.slot0 + u / NHB - my.lo];
+          const uint8_t* g0 = p.sp_inter + static_cast<size_t>(S.sp_row0[my.slot0 + u / NHB - my.lo]) * N_HALF + ti.chunk * CHUNK_COLS + gc * 16;
+          for (int dk = 0; dk < NP; ++dk) {
+            const uint32_t sa = na % SPLIT_SA;
+            if (!dead && !mbar_wait(&S.emptyA[sa], ((na / SPLIT_SA) & 1u) ^ 1u, wc, kSiteEmptyA)) dead = true;
+            if (dead) continue;
+#pragma unroll
+            for (int i = 0; i < ROWS_PER_THREAD; ++i) {
+              const int r = gr + 8 * i;
+              if (r < ti.rows) cp_async16(dst0 + sa * A_STAGE_BYTES + i * 1024, g0 + static_cast<size_t>(r) * N_HALF + dk * 128);
+            }
+            cp_async_arrive_noinc(&S.fullA[sa]);
+            ++na;
+          }
+        }
+        named_bar_sync(2, N_GATHER);  // sp_gflag and the token table have been read
+      }
+      cp_async_commit();
+      cp_async_wait<0>();
+    }
+  } else {
+    // epilogue: the columns and rows of a thread are those of the whole-unit form
+    reg_inc<REGS_EPILOGUE>();
+    const int et = tid - 128, h = et >> 7, q = warp & 3, r = q * 32 + lane;
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    auto up_col = [&](int c) -> uint32_t { return h * HCB + c * (BC / 2); };
+    auto down_col = [&](int c) -> uint32_t { return h * WC + c * HCB; };
+    uint32_t nt = 0;
+    bool dead = false;
+    auto full = [&]() -> uint32_t {   // the next accumulator buffer, once it is full
+      const uint32_t buf = nt % NBUF;
+      if (!dead && !mbar_wait(&S.tmem_full[buf], (nt / NBUF) & 1u, wc, kSiteTmemFull)) dead = true;
+      ++nt;
+      dead = __any_sync(0xFFFFFFFFu, dead);
+      return buf;
+    };
+    // One slab step: acc += D * scale (s_lo for the first HCB columns, s_hi for the rest).
+    auto promote = [&](float2 (&acc)[TCOLS / 2], float s_lo, float s_hi, auto col) {
+      const uint32_t buf = full();
+      if (dead) return;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t v[HCB];
+        tmem_ld_n<HCB>(t_row + buf * BC + col(c), v);
+        tmem_ld_wait();
+        if (c == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&S.tmem_empty[buf]);
+        }
+        const float sc = (c == 0) ? s_lo : s_hi;
+#pragma unroll
+        for (int i = 0; i < HCB / 2; ++i)
+          acc[c * (HCB / 2) + i] = __ffma2_rn(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])),
+                                              make_float2(sc, sc), acc[c * (HCB / 2) + i]);
+      }
+    };
+    // A warp none of whose 32 rows belongs to the tile only hands the buffers back: in the short tiles of a short batch
+    // the other warps then have the issue slots and the special-function unit to themselves.
+    auto pass_on = [&](int n) {
+#pragma unroll 1
+      for (int i = 0; i < n; ++i) {
+        const uint32_t buf = full();
+        if (lane == 0 && !dead) mbar_arrive(&S.tmem_empty[buf]);
+      }
+    };
+    // index of this thread's partial row in tile ti (-1: no row) and its token
+    auto take_row = [&](const TileInfo& ti, int& fi, int& tok) {
+      fi = -1;
+      tok = 0;
+      if (r < ti.rows) {
+        if (ti.e == SHARED_E) {
+          tok = ti.row0 + r;
+          fi = numel + tok;
+        } else {
+          fi = __ldcg(&p.sorted_ids[ti.row0 + r]);
+          if (fi < 0 || fi >= numel) fi = -1;
+          else tok = fi / TOP_K;
+        }
+      }
+    };
+    // all epilogue threads: arrive at the counter and wait until it stands at `target`
+    auto meet = [&](uint32_t target) {
+      named_bar_sync(1, N_EPI);
+      if (et == 0) {
+        __threadfence();
+        atomicAdd(&ws->barrier[kSplitCounter], 1u);
+        S.sp_flag = wait_counter_ge(&ws->barrier[kSplitCounter], target, wc, kErrGridBarrier, kSplitCounter) ? 1u : 0u;
+        __threadfence();
+      }
+      named_bar_sync(1, N_EPI);
+      if (S.sp_flag == 0u) dead = true;
+    };
+    for (int w = 0; w < waves; ++w) {
+      const SplitShare my = split_share(w, wave_units, units, bid);
+      // ---------------- up projection + SiLU*mul + requantisation
+      int cur = -1, fi = -1, tok = 0;
+      for (int u = my.a0; u < my.a1; ++u) {
+        const int ps = u % NP, slot = my.slot0 + u / NP - my.lo;
+        const TileInfo ti = S.tiles[slot];
+        if (q * 32 >= ti.rows) { pass_on(NK); continue; }
+        if (slot != cur) { cur = slot; take_row(ti, fi, tok); }
+        const bool sh = ti.e == SHARED_E;
+        const float* su = sh ? p.sh_up_scales : p.up_w_scales;
+        // the pass's weight scales, spread over the lanes; the row's activation scale is loaded two slabs ahead
+        constexpr int WR = (NK + 31) / 32;
+        float wg[WR], wu[WR];
+#pragma unroll
+        for (int j = 0; j < WR; ++j) {
+          const int ks = lane + 32 * j;
+          wg[j] = (ks < NK) ? __ldg(su + wsu_index(sh ? 0 : ti.e, ti.chunk, ps * NK + ks)) : 0.f;
+          wu[j] = (ks < NK) ? __ldg(su + wsu_index(sh ? 0 : ti.e, ti.chunk, (NP + ps) * NK + ks)) : 0.f;
+        }
+        const float* as_row = p.act_scales + static_cast<size_t>(tok) * NK;
+        float a_n1 = (fi >= 0) ? __ldcg(as_row) : 0.f, a_n2 = (fi >= 0) ? __ldcg(as_row + 1) : 0.f;
+        float2 acc[TCOLS / 2];
+#pragma unroll
+        for (int i = 0; i < TCOLS / 2; ++i) acc[i] = make_float2(0.f, 0.f);
+#pragma unroll 1
+        for (int ks = 0; ks < NK; ++ks) {
+          const float a_s = a_n1;
+          a_n1 = a_n2;
+          if (ks + 2 < NK && fi >= 0) a_n2 = __ldcg(as_row + ks + 2);
+          const float s_g = __fmul_rn(__shfl_sync(0xFFFFFFFFu, (WR > 1 && ks >= 32) ? wg[WR - 1] : wg[0], ks & 31), a_s);
+          const float s_u = __fmul_rn(__shfl_sync(0xFFFFFFFFu, (WR > 1 && ks >= 32) ? wu[WR - 1] : wu[0], ks & 31), a_s);
+          promote(acc, s_g, s_u, up_col);
+        }
+        // the row's amax over the pass's 128 columns: the two warps of these rows hold half of them each
+        float mx = silu_mul(acc);
+        S.rowmax[u & 1][h][r] = mx;
+        named_bar_sync(4 + q, 64);
+        mx = fmaxf(S.rowmax[u & 1][0][r], S.rowmax[u & 1][1][r]);
+        const bool nz = mx > FLT_MIN;
+        const float inv = nz ? __fdiv_rn(448.0f, mx) : 0.f;
+        if (fi >= 0 && !dead) {
+          const size_t srow = static_cast<size_t>(S.sp_row0[slot] + r);
+          uint8_t* irow = p.sp_inter + srow * N_HALF + ti.chunk * CHUNK_COLS + ps * 128 + h * HCB;
+#pragma unroll
+          for (int c = 0; c < HCB / 16; ++c) *reinterpret_cast<uint4*>(irow + c * 16) = pack_e4m3x16(&acc[c * 8], inv);
+          if (h == 0) p.sp_scale[srow * NPT + ti.chunk * NP + ps] = nz ? __fdiv_rn(mx, 448.0f) : (1.0f / 448.0f);
+        }
+      }
+      meet(static_cast<uint32_t>((2 * w + 1) * kGrid));  // every row of the wave's intermediate is written
+      if (bid == 0 && et == 0) ws->phase_ns[6] = globaltimer_ns();
+      // ---------------- down projection, routing weight, bf16 partial rows
+      cur = -1;
+      float rw = 0.f, isc[NP];
+      for (int u = my.b0; u < my.b1; ++u) {
+        const int hb = u % NHB, slot = my.slot0 + u / NHB - my.lo;
+        const TileInfo ti = S.tiles[slot];
+        if (q * 32 >= ti.rows) { pass_on(NP); continue; }
+        const bool sh = ti.e == SHARED_E;
+        if (slot != cur) {
+          cur = slot;
+          take_row(ti, fi, tok);
+          rw = 0.f;
+#pragma unroll
+          for (int dk = 0; dk < NP; ++dk) isc[dk] = 0.f;
+          if (fi >= 0) {
+            rw = !sh ? __ldcg(&p.topk_weights[fi]) : (p.sh_gate != nullptr) ? __ldcg(&p.sh_gate_w[tok]) : 1.f;
+#pragma unroll
+            for (int dk = 0; dk < NP; ++dk)
+              isc[dk] = __ldcg(&p.sp_scale[static_cast<size_t>(S.sp_row0[slot] + r) * NPT + ti.chunk * NP + dk]);
+          }
+        }
+        float sc[NP];
+#pragma unroll
+        for (int dk = 0; dk < NP; ++dk)
+          sc[dk] = __fmul_rn(__ldg((sh ? p.sh_down_scales : p.down_w_scales) + wsd_index(sh ? 0 : ti.e, ti.chunk, (hb * 2 + h) * NP + dk)),
+                             isc[dk]);
+        float2 acc[TCOLS / 2];
+#pragma unroll
+        for (int i = 0; i < TCOLS / 2; ++i) acc[i] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int dk = 0; dk < NP; ++dk) promote(acc, sc[dk], sc[dk], down_col);
+        store_rows(p, acc, fi, make_float2(rw, rw), ti.chunk, hb * 256 + h * WC, !dead);
+      }
+      if (w + 1 < waves) meet(static_cast<uint32_t>((2 * w + 2) * kGrid));  // the intermediate may be overwritten
+    }
+  }
+}
+
 // ------------------------------------------------------------------ the kernel
+template <bool SPLIT>
 __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t dyn_raw[];
   __shared__ SharedState S;
@@ -601,12 +1039,13 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   const int T = p.num_tokens;
   const int numel = T * TOP_K;
 
+  constexpr int RS = SPLIT ? 3 : (SA < SB) ? SA : SB;  // stages of the router linear's ring
   // 1024-byte aligned base of the operand buffers
   const uint32_t dyn_u32 = (smem_u32(dyn_raw) + 1023u) & ~1023u;
   uint8_t* dyn = dyn_raw + (dyn_u32 - smem_u32(dyn_raw));
   uint8_t* inter = dyn;
-  uint8_t* a_ring = dyn + INTER_BYTES;
-  uint8_t* b_ring = a_ring + SA * A_STAGE_BYTES;
+  uint8_t* a_ring = SPLIT ? dyn : dyn + INTER_BYTES;
+  uint8_t* b_ring = a_ring + (SPLIT ? SPLIT_SA : SA) * A_STAGE_BYTES;
   float* as_sm = reinterpret_cast<float*>(b_ring + SB * B_STAGE_BYTES);  // [NK][128]
   float* wsu_sm = as_sm + NK * TILE_M;                                    // [2][WSU_N]
   float* wsd_sm = wsu_sm + 2 * WSU_N;                                     // [2][WSD_N]
@@ -865,6 +1304,27 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       if (tid < E) { scan_cnt[tid] += vc; scan_tile[tid] += vt; }
       __syncthreads();
     }
+    // the shared expert's units follow the routed ones in the deal: token tile j (128 tokens), chunk fastest
+    int sh_units = 0;
+    if (p.sh_on) {
+      const int tok_tiles = (T + TILE_M - 1) / TILE_M;
+      sh_units = ((tok_tiles > p.sh_part) ? (tok_tiles - p.sh_part + p.sh_parts - 1) / p.sh_parts : 0) * NCH;
+    }
+    const int tt_routed = scan_tile[E - 1], rows_routed = scan_cnt[E - 1];
+    // Split form: every row of the batch in the intermediate at once where they fit (a row's place is its sorted
+    // position), otherwise waves of as many units as fit (its place is the unit's place in the wave).
+    const bool one_wave = !SPLIT || rows_routed + sh_units / NCH * TILE_M <= p.sp_rows;
+    const int wave_units = one_wave ? max(1, tt_routed + sh_units) : max(1, p.sp_rows / TILE_M * NCH);
+    // place of unit g in this CTA's list, or -1; whole units are dealt round-robin
+    auto slot_of = [&](int g) -> int {
+      if constexpr (SPLIT) {
+        const SplitShare mine = split_share(g / wave_units, wave_units, tt_routed + sh_units, bid);
+        const int l = g % wave_units;
+        return (l >= mine.lo && l < mine.hi) ? mine.slot0 + l - mine.lo : -1;
+      } else {
+        return (g % SCHED_UNITS == sched_me) ? g / SCHED_UNITS : -1;
+      }
+    };
     if (tid < E) {
       const int off_e = scan_cnt[tid] - cnt;
       const int tbase = scan_tile[tid] - tiles_e;
@@ -879,8 +1339,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       }
       for (int i = 0; i < tiles_e; ++i) {
         const int g = tbase + i;
-        if (g % SCHED_UNITS == sched_me) {
-          const int slot = g / SCHED_UNITS;
+        const int slot = slot_of(g);
+        if (slot >= 0) {
           if (slot < MAX_MY_TILES) {
             TileInfo ti;
             ti.e = tid;
@@ -889,6 +1349,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             ti.rows = max(0, min(TILE_M, off_e + cnt - ti.row0));
             ti.chunk = i % NCH;
             S.tiles[slot] = ti;
+            if constexpr (SPLIT) S.sp_row0[slot] = one_wave ? ti.row0 : g % wave_units / NCH * TILE_M;
           } else {
             report_error(ws, kErrBounds, 1, static_cast<uint32_t>(g), static_cast<uint32_t>(slot));
           }
@@ -904,17 +1365,11 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       }
     }
     __syncthreads();
-    // the shared expert's units follow the routed ones in the deal: token tile j (128 tokens), chunk fastest
-    int sh_units = 0;
     if (p.sh_on) {
-      const int tok_tiles = (T + TILE_M - 1) / TILE_M;
-      const int mine = (tok_tiles > p.sh_part) ? (tok_tiles - p.sh_part + p.sh_parts - 1) / p.sh_parts : 0;
-      sh_units = mine * NCH;
-      const int tt_routed = S.total_tiles;
       for (int i = tid; i < sh_units; i += BLOCK) {
         const int g = tt_routed + i;
-        if (g % SCHED_UNITS == sched_me) {
-          const int slot = g / SCHED_UNITS;
+        const int slot = slot_of(g);
+        if (slot >= 0) {
           if (slot < MAX_MY_TILES) {
             TileInfo ti;
             ti.e = SHARED_E;
@@ -922,6 +1377,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             ti.rows = max(0, min(TILE_M, T - ti.row0));
             ti.chunk = i % NCH;
             S.tiles[slot] = ti;
+            if constexpr (SPLIT) S.sp_row0[slot] = one_wave ? rows_routed + i / NCH * TILE_M : g % wave_units / NCH * TILE_M;
           } else {
             report_error(ws, kErrBounds, 3, static_cast<uint32_t>(g), static_cast<uint32_t>(slot));
           }
@@ -929,7 +1385,9 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       }
     }
     if (tid == 0) {
-      const int tt = S.total_tiles + sh_units;
+      const int tt = tt_routed + sh_units;
+      S.sp_units = tt;
+      S.sp_wave_units = wave_units;
       S.n_my_tiles = (tt > sched_me) ? min(MAX_MY_TILES, (tt - sched_me + SCHED_UNITS - 1) / SCHED_UNITS) : 0;
     }
     // stable scatter: each warp re-walks its own tokens in ascending order
@@ -959,12 +1417,13 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   const uint32_t crank = PAIR ? cluster_ctarank() : 0u;
   const bool leader = crank == 0u;
   if (tid == 0) {
+    if (SPLIT && !alive) { S.sp_units = 0; S.sp_wave_units = 1; }
     const uint32_t both = PAIR ? 2u : 1u;
-    for (int s = 0; s < SA; ++s) {
+    for (int s = 0; s < (SPLIT ? SPLIT_SA : SA); ++s) {
       mbar_init(&S.fullA[s], N_GATHER + ((PAIR && leader) ? 1u : 0u));
       mbar_init(&S.emptyA[s], 1);
     }
-    for (int s = 0; s < SB; ++s) { mbar_init(&S.fullB[s], 1); mbar_init(&S.emptyB[s], 1); }
+    for (int s = 0; s < (SPLIT ? SPLIT_SB : SB); ++s) { mbar_init(&S.fullB[s], 1); mbar_init(&S.emptyB[s], 1); }
     for (int s = 0; s < NBUF; ++s) { mbar_init(&S.tmem_full[s], 1); mbar_init(&S.tmem_empty[s], both * (N_EPI / 32)); }
 #ifdef MONO_PROFILE
     for (int i = 0; i < 48; ++i) (&S.whist[0][0])[i] = 0ull;
@@ -992,7 +1451,9 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   const uint32_t tmem_base = S.tmem_base;
   const int n_my = alive ? S.n_my_tiles : 0;
 
-  if (warp < 4) {
+  if constexpr (SPLIT) {
+    split_phase(p, S, wc, a_ring, b_ring, tmem_base);
+  } else if (warp < 4) {
     reg_dec<REGS_PRODUCER>();
     if (warp == WARP_TMA) {
       // ---------------------------------------------------------- weight producer
@@ -1981,10 +2442,32 @@ int cached_map(CUtensorMap* dst, int kind, const void* base, uint64_t rows, uint
   return 0;
 }
 
+// Whether the split form is expected to be faster, from the batch size alone (the tiles are only known on the device; a
+// wrong guess costs time, not results). Units are estimated for even routing: the experts that T tokens reach, half a
+// tile of padding once experts fill more than one. Then the slab steps of the busiest CTA are compared. A split step
+// costs about 1.4 whole ones (1.0 against 0.75 us with all SMs loading weights: the down passes fetch their rows again,
+// and every pass starts its pipeline anew). Measured, whole -> split, expert phase in us: H=2048 I=512, 256 experts: 1
+// token 65 -> 30, 8 70 -> 58, 32 144 -> 121; 16 tokens 81 -> 86, 256 155 -> 163 (these stay whole); 64 of 256 experts:
+// 8192 tokens 145 -> 122; H=7168, 8 units a token: 1 token 109 -> 57.
+bool split_pays(int num_tokens, int sh_units) {
+  const double rows = static_cast<double>(num_tokens) * TOP_K / E;  // of an expert
+  const double reached = 1.0 - pow(1.0 - static_cast<double>(TOP_K) / E, num_tokens);
+  const double tiles = fmax(reached, rows < 0.75 * TILE_M ? 0.0 : rows / TILE_M + 0.5);
+  const long long units = static_cast<long long>(ceil(E_LOCAL * tiles)) * NCH + sh_units;
+  auto per_cta = [](long long n) { return (n + kGrid - 1) / kGrid; };
+  const long long whole = per_cta(units) * (NP * NK + NHB * NP);
+  const long long split = per_cta(units * NP) * NK + per_cta(units * NHB) * NP;
+  return split * 10 < whole * 7;
+}
+
 cudaError_t ensure_kernel_attribute(int dev) {
   std::lock_guard<std::mutex> lock(g_plan_mutex);
   if (dev >= 0 && dev < 64 && g_attr_set[dev]) return cudaSuccess;
-  const cudaError_t err = cudaFuncSetAttribute(moe_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM);
+  cudaError_t err = cudaFuncSetAttribute(moe_prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM);
+  if constexpr (SPLIT_BUILD) {
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(moe_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_DYN_SMEM);
+  }
   if (err == cudaSuccess && dev >= 0 && dev < 64) g_attr_set[dev] = true;
   return err;
 }
@@ -1996,7 +2479,10 @@ using namespace mono;
 
 extern "C" {
 
-size_t prefill_wgmma_workspace_bytes() { return sizeof(Workspace); }
+// What every launch needs (sizeof(Workspace)) and, behind it, the intermediate rows of the split form. A workspace that
+// holds only the needed part is accepted: its launches compute whole units.
+constexpr size_t kSplitOffset = (sizeof(Workspace) + 255) / 256 * 256;
+size_t prefill_wgmma_workspace_bytes() { return kSplitOffset + SPLIT_ROWS * SPLIT_ROW_BYTES; }
 int prefill_wgmma_num_experts() { return E; }
 int prefill_wgmma_num_experts_local() { return E_LOCAL; }
 int prefill_wgmma_ep_capable() { return EP_BUILD ? 1 : 0; }
@@ -2174,6 +2660,21 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
   p.dbg_acc = g_dbg_acc;
   p.dbg_inter = g_dbg_inter;
   p.dbg_inter_scale = g_dbg_inter_scale;
+  bool split = false;
+  if constexpr (SPLIT_BUILD) {
+    // rows in 16-byte pieces; the debug dumps are written by whole units only
+    if (workspace_bytes > kSplitOffset && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 && p.dbg_acc == nullptr &&
+        p.dbg_inter == nullptr && p.dbg_inter_scale == nullptr) {
+      const int sh_parts = (sh != nullptr) ? sh->parts : 1;
+      const size_t rows = (workspace_bytes - kSplitOffset) / SPLIT_ROW_BYTES;
+      p.sp_rows = static_cast<int>(rows < SPLIT_ROWS ? rows : SPLIT_ROWS);
+      p.sp_inter = static_cast<uint8_t*>(workspace) + kSplitOffset;
+      p.sp_scale = reinterpret_cast<float*>(p.sp_inter + static_cast<size_t>(p.sp_rows) * N_HALF);
+      // all rows at once, or waves of units, which a smaller intermediate would leave too short
+      const bool fits = p.sp_rows == SPLIT_ROWS || numel + sh_tiles * TILE_M <= p.sp_rows;
+      split = fits && split_pays(num_tokens, static_cast<int>(sh_tiles / sh_parts) * NCH);
+    }
+  }
 
   int rc = cached_map(&p.tm_up, 0, up_w_fp8, static_cast<uint64_t>(E_LOCAL) * N_UP, K_DIM, HCB);
   if (rc != 0) {
@@ -2235,21 +2736,24 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
     static int clusters_fit = -1;   // every cluster has to be resident at once (grid barriers)
     if (clusters_fit < 0) {
       int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, moe_prefill_kernel, &cfg) != cudaSuccess) n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, moe_prefill_kernel<false>, &cfg) != cudaSuccess) n = 0;
       clusters_fit = n;
     }
     if (clusters_fit < kGrid / 2) {
       fprintf(stderr, "only %d of %d two-CTA clusters can be resident\n", clusters_fit, kGrid / 2);
       return -107;
     }
-    err = cudaLaunchKernelEx(&cfg, moe_prefill_kernel, p);
+    err = cudaLaunchKernelEx(&cfg, moe_prefill_kernel<false>, p);
     if (err != cudaSuccess) {
       fprintf(stderr, "kernel launch failed: %s\n", cudaGetErrorString(err));
       return static_cast<int>(err);
     }
     return 0;
   }
-  moe_prefill_kernel<<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
+  if constexpr (SPLIT_BUILD) {
+    if (split) moe_prefill_kernel<true><<<kGrid, BLOCK, SPLIT_DYN_SMEM, stream>>>(p);
+  }
+  if (!split) moe_prefill_kernel<false><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
   err = cudaGetLastError();
   if (err != cudaSuccess) {
     fprintf(stderr, "kernel launch failed: %s\n", cudaGetErrorString(err));
@@ -2431,7 +2935,9 @@ int launch_prefill_moe_wgmma_q1_ep(const float* logits, int num_tokens, int bloc
 constexpr int kNoAllocMaxTokens = (H_DIM <= 2048) ? 256 : (NCH > 1 ? 32 : 64);
 constexpr size_t na_align(size_t x) { return (x + 255) / 256 * 256; }
 constexpr size_t kNaWorkspace = 0;
-constexpr size_t kNaActFp8 = kNaWorkspace + na_align(sizeof(Workspace));
+constexpr size_t kNaWorkspaceBytes =   // the intermediate of every routed row of the largest batch
+    kSplitOffset + (SPLIT_BUILD ? static_cast<size_t>(kNoAllocMaxTokens) * TOP_K * SPLIT_ROW_BYTES : 0);
+constexpr size_t kNaActFp8 = kNaWorkspace + na_align(kNaWorkspaceBytes);
 constexpr size_t kNaActScales = kNaActFp8 + na_align(static_cast<size_t>(kNoAllocMaxTokens) * K_DIM);
 constexpr size_t kNaTopkIds = kNaActScales + na_align(static_cast<size_t>(kNoAllocMaxTokens) * NK * 4);
 constexpr size_t kNaTopkW = kNaTopkIds + na_align(static_cast<size_t>(kNoAllocMaxTokens) * TOP_K * 4);
@@ -2498,7 +3004,7 @@ int launch_prefill_moe_noalloc(const float* logits, int num_tokens, const void* 
   const int rc = noalloc_base(&b, true);
   if (rc != 0) return rc;
   return launch_prefill_moe_wgmma_q1_ep2(
-      logits, num_tokens, TILE_M, b + kNaWorkspace, sizeof(Workspace), act_bf16, b + kNaActFp8,
+      logits, num_tokens, TILE_M, b + kNaWorkspace, kNaWorkspaceBytes, act_bf16, b + kNaActFp8,
       reinterpret_cast<float*>(b + kNaActScales), up_w_fp8, up_w_scales, down_w_fp8, down_w_scales,
       reinterpret_cast<float*>(b + kNaPartial), reinterpret_cast<int32_t*>(b + kNaTopkIds),
       reinterpret_cast<float*>(b + kNaTopkW), reinterpret_cast<int32_t*>(b + kNaSorted), bf16_output, router_bias,
