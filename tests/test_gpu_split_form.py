@@ -4,7 +4,7 @@ because every row sees the same operations in the same order."""
 import pytest
 import torch
 
-from unimonomoe_b200 import MonoKernel, synth, variant_path
+from unimonomoe_b200 import MonoKernel, build as kbuild, synth, variant_path
 from unimonomoe_b200.loader import prepare_shared_expert
 
 pytestmark = pytest.mark.gpu
@@ -18,6 +18,9 @@ CASES += [(("qwen_ep4", synth.QWEN, 512, 64, False), T) for T in (9, 257)]
 CASES += [(("qwen_w1", synth.QWEN, 512, 256, True), T) for T in (3, 32)]
 CASES += [(("ds_tp8", synth.DEEPSEEK, 256, 256, False), T) for T in (1, 4)]
 CASES += [(("ds_ep8", synth.DEEPSEEK, 2048, 32, True), T) for T in (8, 20)]
+# more than 64 K slabs: a lane holds the weight scales of three of them
+WIDE = synth.LayerSpec("wide", hidden=9216, inter=256)
+CASES += [(("wide_ep8", WIDE, 256, 32, False), T) for T in (3, 16)]
 # every token on this rank's experts: 65536 rows, several waves of units through the intermediate
 CASES += [(("qwen_ep4", synth.QWEN, 512, 64, False), 8192)]
 _layers = {}
@@ -36,7 +39,8 @@ def _layer(build):
 @pytest.mark.parametrize("build,T", CASES, ids=[f"{b[0]}{'-shared' if b[4] else ''}-{T}" for b, T in CASES])
 def test_split_units_give_the_bits_of_whole_units(build, T):
     variant, spec, width, local, shared = build
-    layer, mk = _layer(build), MonoKernel(variant_path(variant))
+    path = kbuild.build_variant(variant) if variant in kbuild.DEV_VARIANTS else variant_path(variant)
+    layer, mk = _layer(build), MonoKernel(path)
     batch = synth.make_batch(spec, layer, T, seed=T, device=DEV, skew=0.5)
     emap = synth.expert_map(spec, 0, 256 // local, device=DEV) if local != 256 else None
     if T == 8192:

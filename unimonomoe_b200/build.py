@@ -46,10 +46,12 @@ VARIANTS = {
     "qwen_w1_pair": dict(QWEN, N_HALF=512, E_LOCAL=256, PAIR=1),
 }
 
-# development variants (not built by default): the stall-counter build and the builds that leave a piece of the
+# development variants (not built by default): the stall-counter build, a geometry for tests, and the builds that leave a piece of the
 # expert phase out (wrong results by design; their run-time differences split the phase)
 DEV_VARIANTS = {
     "qwen_w1_prof": dict(QWEN, N_HALF=512, E_LOCAL=256, PROFILE=1),
+    # more K slabs (72) than the shipped geometries have: for tests of code that spreads per-slab values over lanes
+    "wide_ep8": dict(K=9216, H=9216, MODE=0, N_HALF=256, E_LOCAL=32),
     "qwen_w1_trace": dict(QWEN, N_HALF=512, E_LOCAL=256, PROFILE=1, DEFS=("MONO_TRACE",)),
     **{f"qwen_w1_abl{m}": dict(QWEN, N_HALF=512, E_LOCAL=256, ABLATE=m) for m in (1, 4, 7, 15, 23, 31, 39, 71, 199, 256)},
 }

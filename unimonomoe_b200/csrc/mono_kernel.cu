@@ -969,8 +969,12 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
           const float a_s = a_n1;
           a_n1 = a_n2;
           if (ks + 2 < NK && fi >= 0) a_n2 = __ldcg(as_row + ks + 2);
-          const float s_g = __fmul_rn(__shfl_sync(0xFFFFFFFFu, (WR > 1 && ks >= 32) ? wg[WR - 1] : wg[0], ks & 31), a_s);
-          const float s_u = __fmul_rn(__shfl_sync(0xFFFFFFFFu, (WR > 1 && ks >= 32) ? wu[WR - 1] : wu[0], ks & 31), a_s);
+          float w_g = wg[0], w_u = wu[0];
+#pragma unroll
+          for (int j = 1; j < WR; ++j)
+            if (ks >= 32 * j) { w_g = wg[j]; w_u = wu[j]; }
+          const float s_g = __fmul_rn(__shfl_sync(0xFFFFFFFFu, w_g, ks & 31), a_s);
+          const float s_u = __fmul_rn(__shfl_sync(0xFFFFFFFFu, w_u, ks & 31), a_s);
           promote(acc, s_g, s_u, up_col);
         }
         // the row's amax over the pass's 128 columns: the two warps of these rows hold half of them each
