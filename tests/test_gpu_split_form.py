@@ -1,6 +1,7 @@
 """The split form of the expert phase (units cut into passes, dealt over all SMs in two halves) against whole units (the
 same launch with a workspace that has no room for the split intermediate): the outputs have to be the same bits,
-because every row sees the same operations in the same order."""
+because every row sees the same operations in the same order. And which of the two a batch gets: the units decide that
+there are, not those that even routing of as many tokens would give."""
 import pytest
 import torch
 
@@ -9,20 +10,26 @@ from unimonomoe_b200.loader import prepare_shared_expert
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
-
-# (build, layer, intermediate columns, local experts, shared expert), tokens: fewer passes than SMs, about one and two
-# rounds of units, one column pass per unit, ragged and full tiles, the shared expert's tiles, units in chunks
-CASES = [(("qwen_w1", synth.QWEN, 512, 256, False), T) for T in (1, 2, 9, 32)]
-CASES += [(("qwen_tp2", synth.QWEN, 256, 256, False), T) for T in (1, 3)]
-CASES += [(("qwen_ep4", synth.QWEN, 512, 64, False), T) for T in (9, 257)]
-CASES += [(("qwen_w1", synth.QWEN, 512, 256, True), T) for T in (3, 32)]
-CASES += [(("ds_tp8", synth.DEEPSEEK, 256, 256, False), T) for T in (1, 4)]
-CASES += [(("ds_ep8", synth.DEEPSEEK, 2048, 32, True), T) for T in (8, 20)]
 # more than 64 K slabs: a lane holds the weight scales of three of them
 WIDE = synth.LayerSpec("wide", hidden=9216, inter=256)
-CASES += [(("wide_ep8", WIDE, 256, 32, False), T) for T in (3, 16)]
-# every token on this rank's experts: 65536 rows, several waves of units through the intermediate
-CASES += [(("qwen_ep4", synth.QWEN, 512, 64, False), 8192)]
+
+# build: (binary, layer, intermediate columns, local experts, shared expert). A case: build, tokens, skew, where the
+# tokens go (None: as the router says; otherwise (n, the experts of the first n tokens, the experts of the others)).
+# Fewer passes than SMs, about one round of units and (even routing) somewhat more than one, ragged and full tiles, the
+# shared expert's tiles, units in chunks
+W1, SHARED = ("qwen_w1", synth.QWEN, 512, 256, False), ("qwen_w1", synth.QWEN, 512, 256, True)
+CASES = [(W1, T, 0.5, None) for T in (1, 2, 9)] + [(W1, 32, 0.0, None)]
+CASES += [(("qwen_tp2", synth.QWEN, 256, 256, False), T, 0.5, None) for T in (1, 3)]
+CASES += [(("qwen_ep4", synth.QWEN, 512, 64, False), T, 0.5, None) for T in (9, 257)]
+CASES += [(SHARED, 3, 0.5, None), (SHARED, 32, 0.0, None)]
+CASES += [(("ds_tp8", synth.DEEPSEEK, 256, 256, False), T, 0.5, None) for T in (1, 4)]
+CASES += [(("ds_ep8", synth.DEEPSEEK, 2048, 32, True), T, 0.5, None) for T in (8, 20)]
+CASES += [(("wide_ep8", WIDE, 256, 32, False), T, 0.5, None) for T in (3, 16)]
+# two waves of units through the intermediate: more rows than it holds; the shared expert's units in the second wave, and
+# units in chunks (2600 of the tokens on two local experts: 42 tiles)
+CASES += [(("qwen_ep8", synth.QWEN, 512, 32, True), 18000, 0.0, None)]
+CASES += [(("ds_ep8", synth.DEEPSEEK, 2048, 32, False), 3200, 0.0,
+           (2600, (3, 17, 40, 41, 77, 78, 100, 101), (40, 41, 77, 78, 100, 101, 130, 131)))]
 _layers = {}
 
 
@@ -36,15 +43,18 @@ def _layer(build):
     return _layers[build]
 
 
-@pytest.mark.parametrize("build,T", CASES, ids=[f"{b[0]}{'-shared' if b[4] else ''}-{T}" for b, T in CASES])
-def test_split_units_give_the_bits_of_whole_units(build, T):
+def _run(build, T, skew, experts=None):
+    """One launch with the intermediate and one without room for it: (output bits, split?, units) each."""
     variant, spec, width, local, shared = build
     path = kbuild.build_variant(variant) if variant in kbuild.DEV_VARIANTS else variant_path(variant)
     layer, mk = _layer(build), MonoKernel(path)
-    batch = synth.make_batch(spec, layer, T, seed=T, device=DEV, skew=0.5)
+    batch = synth.make_batch(spec, layer, T, seed=T, device=DEV, skew=skew)
+    if experts is not None:
+        n, first, others = experts
+        batch["logits"] -= 50.0
+        batch["logits"][:n, list(first)] += 100.0
+        batch["logits"][n:, list(others)] += 100.0
     emap = synth.expert_map(spec, 0, 256 // local, device=DEV) if local != 256 else None
-    if T == 8192:
-        batch["logits"][:, :local] += 50.0
     kw = {}
     if shared:
         sh = layer["shared"]
@@ -52,7 +62,7 @@ def test_split_units_give_the_bits_of_whole_units(build, T):
               "shared_part": (0, 256 // local), "out_scale": spec.routed_scaling}
     needed = mk._int_symbol("prof_offset") + 148 * 64 * 8
     ns = mk._int_symbol("phase_ns_offset") + 6 * 8        # time stamp between the halves of the split form
-    outs, ran = [], []
+    got = []
     for small in (False, True):
         sc = mk._allocate_scratch(T, DEV)
         sc["partial"].fill_(float("nan"))
@@ -61,8 +71,29 @@ def test_split_units_give_the_bits_of_whole_units(build, T):
         out = torch.full((T, spec.hidden), float("nan"), dtype=torch.bfloat16, device=DEV)
         mk.prefill_impl(batch["hs"], batch["logits"], layer["w13"], layer["w13_scale"], layer["w2"], layer["w2_scale"], 8,
                         True, layer["bias"], out, expert_map=emap, scratch=sc, check=True, **kw)
-        outs.append(out.view(torch.int16))
-        ran.append(int(sc["workspace"][ns:ns + 8].view(torch.int64)[0]) != 0)
-    assert ran == [True, False]
-    assert torch.equal(outs[0], outs[1])
-    assert bool(torch.isfinite(outs[0].view(torch.bfloat16).float()).all())
+        got.append((out.view(torch.int16), int(sc["workspace"][ns:ns + 8].view(torch.int64)[0]) != 0,
+                    mk.workspace_view(sc["workspace"])["total_tiles"]))
+    return got
+
+
+@pytest.mark.parametrize("build,T,skew,experts", CASES, ids=[f"{b[0]}{'-shared' if b[4] else ''}-{T}" for b, T, _, _ in CASES])
+def test_split_units_give_the_bits_of_whole_units(build, T, skew, experts):
+    (a, a_split, _), (b, b_split, _) = _run(build, T, skew, experts)
+    assert (a_split, b_split) == (True, False)
+    assert torch.equal(a, b)
+    assert bool(torch.isfinite(a.view(torch.bfloat16).float()).all())
+
+
+# 148 units fill one round of whole units, in which splitting does not pay from about 75 on: up to there, and from 149
+# to about 185, the split form. 32 tokens reach 169 experts at even routing, 124 at skew 0.5, 69 at skew 1.0.
+EP4 = ("qwen_ep4", synth.QWEN, 512, 64, False)
+CHOICES = [(W1, 32, 0.0, (149, 185), True), (W1, 32, 0.5, (76, 148), False), (W1, 32, 1.0, (1, 74), True),
+           (W1, 16, 0.0, (76, 148), False), (EP4, 7500, 0.0, (76, 148), False), (EP4, 8192, 0.0, (149, 185), True)]
+
+
+@pytest.mark.parametrize("build,T,skew,between,splits", CHOICES, ids=[f"{b[0]}-{T}-{s}" for b, T, s, _, _ in CHOICES])
+def test_the_units_of_the_batch_decide(build, T, skew, between, splits):
+    (a, a_split, units), (b, b_split, _) = _run(build, T, skew)
+    assert between[0] <= units <= between[1]
+    assert (a_split, b_split) == (splits, False)
+    assert torch.equal(a, b)

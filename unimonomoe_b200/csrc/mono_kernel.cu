@@ -206,9 +206,11 @@ constexpr int MAX_TILES = MAX_MY_TILES * kGrid;
 // 128-column pass of the up projection), whose e4m3 result and scales go to global memory; then, behind a grid-wide
 // counter, every (unit, 256-column pass of the down projection). The intermediate leaves shared memory, and the weight
 // ring takes its place. The operations on a row and their order are those of the whole unit: the same bits come out.
-constexpr bool SPLIT_BUILD = ONE_BOX && MONO_ABLATE == 0;
+// (With one pass of the up projection per unit there is too little to cut: no number of units makes it pay.)
+constexpr bool SPLIT_BUILD = ONE_BOX && NP > 1 && MONO_ABLATE == 0;
 constexpr size_t SPLIT_ROW_BYTES = N_HALF + NPT * sizeof(float);  // e4m3 intermediate and its scales, one row
-constexpr int SPLIT_ROWS = SPLIT_BUILD ? kGrid * TILE_M : 0;      // rows of the global intermediate
+constexpr int SPLIT_ROWS = SPLIT_BUILD ? kGrid / NCH * TILE_M : 0;  // rows of the global intermediate: kGrid full units
+static_assert(kGrid % NCH == 0, "a wave of kGrid units holds whole tiles");
 
 // ------------------------------------------------------------------ shared memory plan
 constexpr int A_STAGE_BYTES = TILE_M * 128;  // 128 rows x 128 B
@@ -238,11 +240,11 @@ static_assert(NWARPS * E * 4 <= SA * A_STAGE_BYTES, "phase-0 histograms live in 
 // split form: no intermediate and no scale staging in shared memory, so the weight ring is deeper
 constexpr int SPLIT_SA = 3;
 constexpr int SPLIT_SB = (SMEM_CAP - SMEM_STATIC_RESERVE - 1024 - SPLIT_SA * A_STAGE_BYTES) / B_STAGE_BYTES;
-constexpr int SPLIT_DYN_SMEM = 1024 + SPLIT_SA * A_STAGE_BYTES + SPLIT_SB * B_STAGE_BYTES;
+constexpr int SPLIT_SMEM = 1024 + SPLIT_SA * A_STAGE_BYTES + SPLIT_SB * B_STAGE_BYTES;
+constexpr int SHORT_DYN_SMEM = (SPLIT_BUILD && SPLIT_SMEM > DYN_SMEM) ? SPLIT_SMEM : DYN_SMEM;  // either form
 constexpr int A_STAGE_CAP = SPLIT_SA > STAGE_CAP ? SPLIT_SA : STAGE_CAP;
 constexpr int B_STAGE_CAP = SPLIT_SB > STAGE_CAP ? SPLIT_SB : STAGE_CAP;
-static_assert(!SPLIT_BUILD || (NWARPS * E * 4 <= SPLIT_SA * A_STAGE_BYTES && SPLIT_SB >= 3),
-              "phases R to 1 use the rings of the split form as they use the others");
+static_assert(!SPLIT_BUILD || SPLIT_SB >= 3, "the split form needs a weight ring of at least three stages");
 
 // Register budget (setmaxnreg). The kernel launches with REGS_LAUNCH registers per thread; the
 // producer warpgroup gives registers back and the epilogue warpgroups take them. The
@@ -606,7 +608,7 @@ struct __align__(16) SharedState {
   uint32_t flag;          // grid_sync result broadcast
   int n_my_tiles;
   int total_tiles;
-  int sp_units, sp_wave_units;   // split form: units in all, and units whose intermediate fits at a time
+  int sp_units, sp_waves;        // split form: units, and waves of them through the intermediate (0: whole units)
   uint32_t sp_flag, sp_gflag;    // split form: counter reached (epilogue, gather warps)
   TileInfo tiles[MAX_MY_TILES];
   int sp_row0[MAX_MY_TILES];     // split form: the tile's first row in the global intermediate
@@ -693,23 +695,48 @@ __device__ __forceinline__ void store_rows(const Params& p, const float2 (&acc)[
 }
 
 // ------------------------------------------------------------------ the split form
-// What CTA `bid` takes of wave w: the units [lo, hi) of the wave its passes belong to (kept from slot0 of its list),
-// the passes [a0, a1) of the up and [b0, b1) of the down projection, counted over the wave's units. Contiguous shares
-// that differ by at most one pass: the passes of one unit mostly follow one another on one CTA.
+// The units of a batch go through the intermediate in one wave where their rows fit, otherwise in waves of kGrid units.
+// What CTA `bid` takes of a wave of n units: the units [lo, hi) its passes belong to, the passes [a0, a1) of the up and
+// [b0, b1) of the down projection, counted over the wave's units. Contiguous shares that differ by at most one pass: the
+// passes of one unit mostly follow one another on one CTA. A full wave of kGrid units is one unit for every CTA, so the
+// units of wave w stand in its list from slot w on.
 struct SplitShare {
-  int lo, hi, slot0, a0, a1, b0, b1;
+  int lo, hi, a0, a1, b0, b1;
 };
-__device__ __forceinline__ SplitShare split_share(int w, int wave_units, int units, int bid) {
-  const int n = min(wave_units, units - w * wave_units);
+__device__ __forceinline__ SplitShare split_share(int n, int bid) {
   SplitShare s;
   s.lo = bid * n / kGrid;
   s.hi = ((bid + 1) * n + kGrid - 1) / kGrid;
-  s.slot0 = w * (((bid + 1) * wave_units + kGrid - 1) / kGrid - bid * wave_units / kGrid);  // the waves before w are full
   s.a0 = bid * (n * NP) / kGrid;
   s.a1 = (bid + 1) * (n * NP) / kGrid;
   s.b0 = bid * (n * NHB) / kGrid;
   s.b1 = (bid + 1) * (n * NHB) / kGrid;
   return s;
+}
+
+// Which batches the split form is faster for: those with at most SPLIT_MOST[r] units in the last of r + 1 rounds of whole
+// units. Every CTA looks that up in phase 1, where the units are known: how many experts a batch reaches depends on how
+// uneven its routing is, and a rule on the number of tokens alone loses a quarter of the expert phase where one round of
+// whole units suffices. The bounds come from the slab steps of the busiest CTA. A split step costs 1.3 to 1.4 whole ones
+// in the builds with H = 2048 (with all SMs loading weights; the down passes fetch their rows again, and every pass starts
+// its pipeline anew) and 1.05 to 1.25 with H = 7168. Measured, expert phase in us with weights from memory, whole -> split,
+// and what the rule takes: H=2048 I=512: 8 units 63 -> 29, 58 70 -> 62, 71 71 -> 67 (split); 76 72 -> 79, 106 79 -> 86,
+// 135 88 -> 104 (whole); 151 143 -> 118, 169 144 -> 122, 183 142 -> 132 (split); 189 142 -> 147, 256 153 -> 160 (whole).
+// I=256: 69 units 46 -> 40 (split), 79 46 -> 53 (whole). H=7168 I=256: 66 units 122 -> 90 (split), 85 124 -> 135 (whole),
+// 156 242 -> 203 (split).
+constexpr int split_steps(int n) { return (n * NP + kGrid - 1) / kGrid * NK + (n * NHB + kGrid - 1) / kGrid * NP; }
+constexpr int split_most(int round, bool one_wave) {   // of the units beyond the full rounds of whole units
+  int most = 0;
+  for (int n = 1; n <= kGrid; ++n) {
+    const int steps = one_wave ? split_steps(round * kGrid + n) : round * split_steps(kGrid) + split_steps(n);
+    if (steps * 10 < (round + 1) * (NP * NK + NHB * NP) * 7) most = n;
+  }
+  return most;
+}
+constexpr int SPLIT_MOST_1 = split_most(0, true), SPLIT_MOST_2 = split_most(1, true), SPLIT_MOST_2W = split_most(1, false);
+static_assert(split_most(2, true) == 0, "the split form is looked up for one and two rounds of units");
+__device__ __forceinline__ bool split_pays(int units, bool one_wave) {
+  return units <= kGrid ? units <= SPLIT_MOST_1 : units <= kGrid + (one_wave ? SPLIT_MOST_2 : SPLIT_MOST_2W);
 }
 
 // Phase 2 in the split form, with the roles of the whole-unit form. Both halves are the same slab step (weights
@@ -718,8 +745,8 @@ __device__ __forceinline__ SplitShare split_share(int w, int wave_units, int uni
 __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, const WaitCtx& wc, uint8_t* a_ring, uint8_t* b_ring,
                                             uint32_t tmem_base) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, bid = blockIdx.x;
-  const int units = S.sp_units, wave_units = S.sp_wave_units;
-  const int waves = (units + wave_units - 1) / wave_units;
+  const int units = S.sp_units, waves = S.sp_waves;
+  auto share = [&](int w) { return split_share(waves == 1 ? units : min(kGrid, units - w * kGrid), bid); };
   const int numel = p.num_tokens * TOP_K;
   Workspace* ws = p.ws;
   const uint32_t a_ring_u32 = smem_u32(a_ring), b_ring_u32 = smem_u32(b_ring);
@@ -738,9 +765,9 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
         };
         bool ok = true;
         for (int w = 0; w < waves && ok; ++w) {
-          const SplitShare my = split_share(w, wave_units, units, bid);
+          const SplitShare my = share(w);
           for (int u = my.a0; u < my.a1 && ok; ++u) {
-            const TileInfo ti = S.tiles[my.slot0 + u / NP - my.lo];
+            const TileInfo ti = S.tiles[w + u / NP - my.lo];
             const bool sh = ti.e == SHARED_E;
             for (int ks = 0; ks < NK; ++ks, ++nb) {
               uint8_t* dst = stage();
@@ -750,7 +777,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
             }
           }
           for (int u = my.b0; u < my.b1 && ok; ++u) {
-            const TileInfo ti = S.tiles[my.slot0 + u / NHB - my.lo];
+            const TileInfo ti = S.tiles[w + u / NHB - my.lo];
             const bool sh = ti.e == SHARED_E;
             for (int dk = 0; dk < NP; ++dk, ++nb) {
               uint8_t* dst = stage();
@@ -764,7 +791,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
     } else if (warp == WARP_MMA) {
       int steps = 0;
       for (int w = 0; w < waves; ++w) {
-        const SplitShare my = split_share(w, wave_units, units, bid);
+        const SplitShare my = share(w);
         steps += (my.a1 - my.a0) * NK + (my.b1 - my.b0) * NP;
       }
       for (uint32_t n = 0; n < static_cast<uint32_t>(steps); ++n) {
@@ -796,10 +823,10 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
       int fills = 0;
       bool dead = false;  // after an abort: the named barriers stay matched, the work is skipped
       for (int w = 0; w < waves; ++w) {
-        const SplitShare my = split_share(w, wave_units, units, bid);
+        const SplitShare my = share(w);
         int cur = -1;
         for (int u = my.a0; u < my.a1; ++u) {
-          const int slot = my.slot0 + u / NP - my.lo;
+          const int slot = w + u / NP - my.lo;
           if (slot != cur) {   // the passes of one unit follow one another: its tokens are looked up once
             cur = slot;
             ++fills;
@@ -845,8 +872,8 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
         named_bar_sync(2, N_GATHER);
         if (S.sp_gflag == 0u) dead = true;
         for (int u = my.b0; u < my.b1; ++u) {
-          const TileInfo ti = S.tiles[my.slot0 + u / NHB - my.lo];
-          const uint8_t* g0 = p.sp_inter + static_cast<size_t>(S.sp_row0[my.slot0 + u / NHB - my.lo]) * N_HALF + ti.chunk * CHUNK_COLS + gc * 16;
+          const TileInfo ti = S.tiles[w + u / NHB - my.lo];
+          const uint8_t* g0 = p.sp_inter + static_cast<size_t>(S.sp_row0[w + u / NHB - my.lo]) * N_HALF + ti.chunk * CHUNK_COLS + gc * 16;
           for (int dk = 0; dk < NP; ++dk) {
             const uint32_t sa = na % SPLIT_SA;
             if (!dead && !mbar_wait(&S.emptyA[sa], ((na / SPLIT_SA) & 1u) ^ 1u, wc, kSiteEmptyA)) dead = true;
@@ -940,11 +967,11 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
       if (S.sp_flag == 0u) dead = true;
     };
     for (int w = 0; w < waves; ++w) {
-      const SplitShare my = split_share(w, wave_units, units, bid);
+      const SplitShare my = share(w);
       // ---------------- up projection + SiLU*mul + requantisation
       int cur = -1, fi = -1, tok = 0;
       for (int u = my.a0; u < my.a1; ++u) {
-        const int ps = u % NP, slot = my.slot0 + u / NP - my.lo;
+        const int ps = u % NP, slot = w + u / NP - my.lo;
         const TileInfo ti = S.tiles[slot];
         if (q * 32 >= ti.rows) { pass_on(NK); continue; }
         if (slot != cur) { cur = slot; take_row(ti, fi, tok); }
@@ -998,7 +1025,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
       cur = -1;
       float rw = 0.f, isc[NP];
       for (int u = my.b0; u < my.b1; ++u) {
-        const int hb = u % NHB, slot = my.slot0 + u / NHB - my.lo;
+        const int hb = u % NHB, slot = w + u / NHB - my.lo;
         const TileInfo ti = S.tiles[slot];
         if (q * 32 >= ti.rows) { pass_on(NP); continue; }
         const bool sh = ti.e == SHARED_E;
@@ -1033,7 +1060,10 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
 }
 
 // ------------------------------------------------------------------ the kernel
-template <bool SPLIT>
+// SHORT: the instance for batches that are expected to be short. It holds both forms of the expert phase and takes one of
+// them by the units that phase 1 counts. The other instance computes whole units only, and computes them faster: inside
+// the first one they take 2 to 4 us more a launch (16 tokens 85 -> 88 us, 64 of 256 experts at 7500 tokens 153 -> 157).
+template <bool SHORT>
 __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t dyn_raw[];
   __shared__ SharedState S;
@@ -1045,13 +1075,14 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   const int T = p.num_tokens;
   const int numel = T * TOP_K;
 
-  constexpr int RS = SPLIT ? 3 : (SA < SB) ? SA : SB;  // stages of the router linear's ring
+  constexpr bool CAN_SPLIT = SHORT && SPLIT_BUILD;
+  constexpr int RS = (SA < SB) ? SA : SB;  // stages of the router linear's ring
   // 1024-byte aligned base of the operand buffers
   const uint32_t dyn_u32 = (smem_u32(dyn_raw) + 1023u) & ~1023u;
   uint8_t* dyn = dyn_raw + (dyn_u32 - smem_u32(dyn_raw));
   uint8_t* inter = dyn;
-  uint8_t* a_ring = SPLIT ? dyn : dyn + INTER_BYTES;
-  uint8_t* b_ring = a_ring + (SPLIT ? SPLIT_SA : SA) * A_STAGE_BYTES;
+  uint8_t* a_ring = dyn + INTER_BYTES;
+  uint8_t* b_ring = a_ring + SA * A_STAGE_BYTES;
   float* as_sm = reinterpret_cast<float*>(b_ring + SB * B_STAGE_BYTES);  // [NK][128]
   float* wsu_sm = as_sm + NK * TILE_M;                                    // [2][WSU_N]
   float* wsd_sm = wsu_sm + 2 * WSU_N;                                     // [2][WSD_N]
@@ -1330,20 +1361,28 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       sh_units = ((tok_tiles > p.sh_part) ? (tok_tiles - p.sh_part + p.sh_parts - 1) / p.sh_parts : 0) * NCH;
     }
     const int tt_routed = scan_tile[E - 1], rows_routed = scan_cnt[E - 1];
-    // Split form: every row of the batch in the intermediate at once where they fit (a row's place is its sorted
-    // position), otherwise waves of as many units as fit (its place is the unit's place in the wave).
-    const bool one_wave = !SPLIT || rows_routed + sh_units / NCH * TILE_M <= p.sp_rows;
-    const int wave_units = one_wave ? max(1, tt_routed + sh_units) : max(1, p.sp_rows / TILE_M * NCH);
+    // Split form: in one wave every row of the batch has its place in the intermediate (its sorted position); in waves of
+    // kGrid units the place is that of the unit in its wave.
+    const int units = tt_routed + sh_units;
+    const bool one_wave = rows_routed + sh_units / NCH * TILE_M <= p.sp_rows;
+    bool split = false;
+    int lo = 0, hi = 0;       // this CTA's units of the last wave
+    if constexpr (CAN_SPLIT) {
+      split = units > 0 && split_pays(units, one_wave);
+      const SplitShare mine = split_share(one_wave ? units : units - kGrid, bid);
+      lo = mine.lo;
+      hi = mine.hi;
+    }
     // place of unit g in this CTA's list, or -1; whole units are dealt round-robin
     auto slot_of = [&](int g) -> int {
-      if constexpr (SPLIT) {
-        const SplitShare mine = split_share(g / wave_units, wave_units, tt_routed + sh_units, bid);
-        const int l = g % wave_units;
-        return (l >= mine.lo && l < mine.hi) ? mine.slot0 + l - mine.lo : -1;
-      } else {
-        return (g % SCHED_UNITS == sched_me) ? g / SCHED_UNITS : -1;
+      if (CAN_SPLIT && split) {
+        if (!one_wave && g < kGrid) return g == bid ? 0 : -1;
+        const int l = one_wave ? g : g - kGrid;
+        return (l >= lo && l < hi) ? l - lo + (one_wave ? 0 : 1) : -1;
       }
+      return (g % SCHED_UNITS == sched_me) ? g / SCHED_UNITS : -1;
     };
+    auto split_row = [&](int g, int sorted_row) -> int { return one_wave ? sorted_row : g % kGrid / NCH * TILE_M; };
     if (tid < E) {
       const int off_e = scan_cnt[tid] - cnt;
       const int tbase = scan_tile[tid] - tiles_e;
@@ -1368,7 +1407,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             ti.rows = max(0, min(TILE_M, off_e + cnt - ti.row0));
             ti.chunk = i % NCH;
             S.tiles[slot] = ti;
-            if constexpr (SPLIT) S.sp_row0[slot] = one_wave ? ti.row0 : g % wave_units / NCH * TILE_M;
+            if (CAN_SPLIT && split) S.sp_row0[slot] = split_row(g, ti.row0);
           } else {
             report_error(ws, kErrBounds, 1, static_cast<uint32_t>(g), static_cast<uint32_t>(slot));
           }
@@ -1396,7 +1435,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             ti.rows = max(0, min(TILE_M, T - ti.row0));
             ti.chunk = i % NCH;
             S.tiles[slot] = ti;
-            if constexpr (SPLIT) S.sp_row0[slot] = one_wave ? rows_routed + i / NCH * TILE_M : g % wave_units / NCH * TILE_M;
+            if (CAN_SPLIT && split) S.sp_row0[slot] = split_row(g, rows_routed + i / NCH * TILE_M);
           } else {
             report_error(ws, kErrBounds, 3, static_cast<uint32_t>(g), static_cast<uint32_t>(slot));
           }
@@ -1404,10 +1443,9 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       }
     }
     if (tid == 0) {
-      const int tt = tt_routed + sh_units;
-      S.sp_units = tt;
-      S.sp_wave_units = wave_units;
-      S.n_my_tiles = (tt > sched_me) ? min(MAX_MY_TILES, (tt - sched_me + SCHED_UNITS - 1) / SCHED_UNITS) : 0;
+      S.sp_units = units;
+      S.sp_waves = split ? (one_wave ? 1 : 2) : 0;
+      S.n_my_tiles = (units > sched_me) ? min(MAX_MY_TILES, (units - sched_me + SCHED_UNITS - 1) / SCHED_UNITS) : 0;
     }
     // stable scatter: each warp re-walks its own tokens in ascending order
     for (int t = t_begin; t < t_end; ++t) {
@@ -1435,14 +1473,14 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   // inter_ready barriers collect the epilogue warps of both CTAs.
   const uint32_t crank = PAIR ? cluster_ctarank() : 0u;
   const bool leader = crank == 0u;
+  const bool split = CAN_SPLIT && alive && S.sp_waves != 0;
   if (tid == 0) {
-    if (SPLIT && !alive) { S.sp_units = 0; S.sp_wave_units = 1; }
     const uint32_t both = PAIR ? 2u : 1u;
-    for (int s = 0; s < (SPLIT ? SPLIT_SA : SA); ++s) {
+    for (int s = 0; s < (split ? SPLIT_SA : SA); ++s) {
       mbar_init(&S.fullA[s], N_GATHER + ((PAIR && leader) ? 1u : 0u));
       mbar_init(&S.emptyA[s], 1);
     }
-    for (int s = 0; s < (SPLIT ? SPLIT_SB : SB); ++s) { mbar_init(&S.fullB[s], 1); mbar_init(&S.emptyB[s], 1); }
+    for (int s = 0; s < (split ? SPLIT_SB : SB); ++s) { mbar_init(&S.fullB[s], 1); mbar_init(&S.emptyB[s], 1); }
     for (int s = 0; s < NBUF; ++s) { mbar_init(&S.tmem_full[s], 1); mbar_init(&S.tmem_empty[s], both * (N_EPI / 32)); }
 #ifdef MONO_PROFILE
     for (int i = 0; i < 48; ++i) (&S.whist[0][0])[i] = 0ull;
@@ -1470,8 +1508,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   const uint32_t tmem_base = S.tmem_base;
   const int n_my = alive ? S.n_my_tiles : 0;
 
-  if constexpr (SPLIT) {
-    split_phase(p, S, wc, a_ring, b_ring, tmem_base);
+  if (split) {
+    if constexpr (CAN_SPLIT) split_phase(p, S, wc, dyn, dyn + SPLIT_SA * A_STAGE_BYTES, tmem_base);
   } else if (warp < 4) {
     reg_dec<REGS_PRODUCER>();
     if (warp == WARP_TMA) {
@@ -2461,22 +2499,17 @@ int cached_map(CUtensorMap* dst, int kind, const void* base, uint64_t rows, uint
   return 0;
 }
 
-// Whether the split form is expected to be faster, from the batch size alone (the tiles are only known on the device; a
-// wrong guess costs time, not results). Units are estimated for even routing: the experts that T tokens reach, half a
-// tile of padding once experts fill more than one. Then the slab steps of the busiest CTA are compared. A split step
-// costs about 1.4 whole ones (1.0 against 0.75 us with all SMs loading weights: the down passes fetch their rows again,
-// and every pass starts its pipeline anew). Measured, whole -> split, expert phase in us: H=2048 I=512, 256 experts: 1
-// token 65 -> 30, 8 70 -> 58, 32 144 -> 121; 16 tokens 81 -> 86, 256 155 -> 163 (these stay whole); 64 of 256 experts:
-// 8192 tokens 145 -> 122; H=7168, 8 units a token: 1 token 109 -> 57.
-bool split_pays(int num_tokens, int sh_units) {
+// Whether a batch gets the instance that can compute the split form, from its size alone (the units are only known on the
+// device, which then chooses between the forms). Units are estimated for even routing: the experts that T tokens reach,
+// half a tile of padding once experts fill more than one. Where fewer units come out, the device stays with whole units:
+// 32 tokens of uneven routing with 124 units take 91 us (105 in the split form, 87 in the instance without it), 64 of 256
+// experts at 7500 tokens with 135 units 157 (182, 153).
+bool short_expected(int num_tokens, int sh_units) {
   const double rows = static_cast<double>(num_tokens) * TOP_K / E;  // of an expert
   const double reached = 1.0 - pow(1.0 - static_cast<double>(TOP_K) / E, num_tokens);
   const double tiles = fmax(reached, rows < 0.75 * TILE_M ? 0.0 : rows / TILE_M + 0.5);
-  const long long units = static_cast<long long>(ceil(E_LOCAL * tiles)) * NCH + sh_units;
-  auto per_cta = [](long long n) { return (n + kGrid - 1) / kGrid; };
-  const long long whole = per_cta(units) * (NP * NK + NHB * NP);
-  const long long split = per_cta(units * NP) * NK + per_cta(units * NHB) * NP;
-  return split * 10 < whole * 7;
+  const double units = ceil(E_LOCAL * tiles) * NCH + sh_units;
+  return units <= SPLIT_MOST_1 || (units > kGrid && units <= kGrid + SPLIT_MOST_2);
 }
 
 cudaError_t ensure_kernel_attribute(int dev) {
@@ -2485,7 +2518,7 @@ cudaError_t ensure_kernel_attribute(int dev) {
   cudaError_t err = cudaFuncSetAttribute(moe_prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM);
   if constexpr (SPLIT_BUILD) {
     if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(moe_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_DYN_SMEM);
+      err = cudaFuncSetAttribute(moe_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SHORT_DYN_SMEM);
   }
   if (err == cudaSuccess && dev >= 0 && dev < 64) g_attr_set[dev] = true;
   return err;
@@ -2679,7 +2712,7 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
   p.dbg_acc = g_dbg_acc;
   p.dbg_inter = g_dbg_inter;
   p.dbg_inter_scale = g_dbg_inter_scale;
-  bool split = false;
+  bool short_batch = false;
   if constexpr (SPLIT_BUILD) {
     // rows in 16-byte pieces; the debug dumps are written by whole units only
     if (workspace_bytes > kSplitOffset && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 && p.dbg_acc == nullptr &&
@@ -2689,9 +2722,9 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
       p.sp_rows = static_cast<int>(rows < SPLIT_ROWS ? rows : SPLIT_ROWS);
       p.sp_inter = static_cast<uint8_t*>(workspace) + kSplitOffset;
       p.sp_scale = reinterpret_cast<float*>(p.sp_inter + static_cast<size_t>(p.sp_rows) * N_HALF);
-      // all rows at once, or waves of units, which a smaller intermediate would leave too short
-      const bool fits = p.sp_rows == SPLIT_ROWS || numel + sh_tiles * TILE_M <= p.sp_rows;
-      split = fits && split_pays(num_tokens, static_cast<int>(sh_tiles / sh_parts) * NCH);
+      // all rows at once, or waves of kGrid units, which need all of the intermediate
+      short_batch = (p.sp_rows == SPLIT_ROWS || numel + sh_tiles * TILE_M <= p.sp_rows) &&
+                    short_expected(num_tokens, static_cast<int>(sh_tiles / sh_parts) * NCH);
     }
   }
 
@@ -2770,9 +2803,9 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
     return 0;
   }
   if constexpr (SPLIT_BUILD) {
-    if (split) moe_prefill_kernel<true><<<kGrid, BLOCK, SPLIT_DYN_SMEM, stream>>>(p);
+    if (short_batch) moe_prefill_kernel<true><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
   }
-  if (!split) moe_prefill_kernel<false><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
+  if (!short_batch) moe_prefill_kernel<false><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
   err = cudaGetLastError();
   if (err != cudaSuccess) {
     fprintf(stderr, "kernel launch failed: %s\n", cudaGetErrorString(err));
