@@ -15,7 +15,7 @@
  *
  * Return codes of the launch entry points (Q:1569-1599, Q:1621-1638, EP:1658-1659):
  *     0      launched
- *  -100      workspace null or smaller than every launch needs (230 KB)
+ *  -100      workspace null or smaller than prefill_wgmma_workspace_min_bytes()
  *  -101      num_tokens <= 0
  *  -102      num_tokens*top_k/128 + local experts exceeds prefill_wgmma_max_tiles()
  *  -103      device has fewer SMs than prefill_wgmma_grid_size()
@@ -32,10 +32,10 @@
  *
  * Buffers (T = num_tokens, k = top_k = 8, E = 256 routed experts, El = local experts):
  *   logits            fp32 [T, E]                      in
- *   workspace         prefill_wgmma_workspace_bytes(); zeroed by the launch itself as far as it has to be. The part
- *                     behind the first 230 KB holds the intermediate of the split form (short batches); a smaller
- *                     workspace, or one that is not 16-byte aligned, is accepted and does without that form: the same
- *                     bits, later
+ *   workspace         prefill_wgmma_workspace_bytes(); zeroed by the launch itself as far as it has to be. What lies
+ *                     behind prefill_wgmma_workspace_min_bytes() holds the intermediate of the split form (short
+ *                     batches); a smaller workspace, or one that is not 16-byte aligned, is accepted and does without
+ *                     that form: the same bits, later
  *   act_bf16          bf16 [T, K]                      in
  *   act_fp8           u8   [T, K]                      scratch/out: e4m3 activations
  *   act_scales        fp32 [T, K/128]                  scratch/out
@@ -239,6 +239,9 @@ int prefill_wgmma_cta_pair(void);
 int prefill_wgmma_partial_chunks(void);
 int prefill_wgmma_block_threads(void);        /* threads per CTA */
 int prefill_wgmma_stable_sort(void);          /* 1 = sorted_token_ids is deterministic (stable) */
+/* The workspace that every launch accepts (230 KB); the rest of prefill_wgmma_workspace_bytes() is the intermediate of
+ * the split form: 10 MB, 5 MB at N_HALF = 256, none at 128 and in the two-CTA build, which have no split form. */
+size_t prefill_wgmma_workspace_min_bytes(void);
 /* Bounded waits: every device-side wait gives up after the time limit, records
  * (code << 24 | site << 16 | block) in the 32-bit status word of the workspace and the
  * launch returns normally. Read the word after synchronising; 0 = success. */

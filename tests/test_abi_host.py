@@ -43,6 +43,26 @@ def test_geometry_readback(built_libs, variant):
     assert geo["workspace_bytes"] >= 148 * 256 * 4
 
 
+@pytest.mark.parametrize("variant", ["qwen_w1", "qwen_tp4", "ds_ep8", "qwen_w1_pair"])
+def test_workspace_sizes_and_what_of_it_is_cleared(built_libs, variant, monkeypatch):
+    """The intermediate of the split form is behind the part that every launch needs: at most 148 tiles of rows, in builds
+    that can use it; only the needed part is cleared when scratch is made (a captured call repeats that at every replay)."""
+    mk = MonoKernel(built_libs[variant])
+    geo, least = mk.geometry(), mk._int_symbol("workspace_min_bytes")
+    assert 148 * 256 * 4 <= least <= 1 << 18
+    rows = {"qwen_w1": 148 * 128, "ds_ep8": 37 * 128}.get(variant, 0)
+    assert geo["workspace_bytes"] == -(-least // 256) * 256 + rows * (geo["n_half"] + geo["n_half"] // 128 * 4)
+    cleared = []
+    zeros, zero_ = torch.zeros, torch.Tensor.zero_
+    monkeypatch.setattr(torch, "zeros", lambda *a, **k: (lambda t: (cleared.append(t.numel() * t.element_size()), t)[1])(zeros(*a, **k)))
+    monkeypatch.setattr(torch.Tensor, "zero_", lambda t: (cleared.append(t.numel() * t.element_size()), zero_(t))[1])
+    sc = mk._allocate_scratch(2, "cpu")
+    assert sc["workspace"].numel() == geo["workspace_bytes"] and not sc["workspace"][:least].any()
+    assert sum(cleared) == least
+    small, keep = _args(ws_bytes=least - 1)
+    assert mk.lib.launch_prefill_moe_wgmma_q1(*small) == -100
+
+
 def _args(n_tokens=16, ws_bytes=None, null=None, extra=()):
     """Argument list with small dummy host buffers: every call below must be declined before
     the library touches CUDA, so the pointers are never dereferenced."""

@@ -60,7 +60,7 @@ def _run(build, T, skew, experts=None):
         sh = layer["shared"]
         kw = {"shared": prepare_shared_expert(sh["w13"], sh["w13_scale"], sh["w2"], sh["w2_scale"], sh["gate"]),
               "shared_part": (0, 256 // local), "out_scale": spec.routed_scaling}
-    needed = mk._int_symbol("prof_offset") + 148 * 64 * 8
+    needed = mk._int_symbol("workspace_min_bytes")
     ns = mk._int_symbol("phase_ns_offset") + 6 * 8        # time stamp between the halves of the split form
     got = []
     for small in (False, True):

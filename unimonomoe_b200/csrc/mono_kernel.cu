@@ -2535,6 +2535,7 @@ extern "C" {
 // holds only the needed part is accepted: its launches compute whole units.
 constexpr size_t kSplitOffset = (sizeof(Workspace) + 255) / 256 * 256;
 size_t prefill_wgmma_workspace_bytes() { return kSplitOffset + SPLIT_ROWS * SPLIT_ROW_BYTES; }
+size_t prefill_wgmma_workspace_min_bytes() { return sizeof(Workspace); }
 int prefill_wgmma_num_experts() { return E; }
 int prefill_wgmma_num_experts_local() { return E_LOCAL; }
 int prefill_wgmma_ep_capable() { return EP_BUILD ? 1 : 0; }

@@ -209,8 +209,12 @@ class MonoKernel:
         geo = self.geometry()
         K, H, k = geo["k_dim"], geo["h_dim"], geo["top_k"]
         chunks = self._int_symbol("partial_chunks") or 1
+        # zeros for whoever reads the counters back before a first launch; the intermediate rows behind them are written
+        # before they are read, and clearing them too would put 10 MB of memset into every replay of a captured call
+        workspace = torch.empty(geo["workspace_bytes"], dtype=torch.uint8, device=device)
+        workspace[:self._int_symbol("workspace_min_bytes")].zero_()
         return {
-            "workspace": torch.zeros(geo["workspace_bytes"], dtype=torch.uint8, device=device),
+            "workspace": workspace,
             "act_fp8": torch.empty(tokens, K, dtype=torch.uint8, device=device),
             "act_scales": torch.empty(tokens, K // 128, dtype=torch.float32, device=device),
             "topk_ids": torch.empty(tokens, k, dtype=torch.int32, device=device),
