@@ -91,6 +91,20 @@ CHOICES = [(W1, 32, 0.0, (149, 185), True), (W1, 32, 0.5, (76, 148), False), (W1
            (W1, 16, 0.0, (76, 148), False), (EP4, 7500, 0.0, (76, 148), False), (EP4, 8192, 0.0, (149, 185), True)]
 
 
+def test_the_time_stamp_tells_which_form_ran():
+    """Two launches on one workspace: the second computes whole units and must not keep the first one's time stamp."""
+    layer, mk = _layer(W1), MonoKernel(variant_path("qwen_w1"))
+    sc = mk._allocate_scratch(16, DEV)
+    seen = []
+    for T in (1, 16, 1):
+        batch = synth.make_batch(synth.QWEN, layer, T, seed=T, device=DEV)
+        out = torch.empty(T, 2048, dtype=torch.bfloat16, device=DEV)
+        mk.prefill_impl(batch["hs"], batch["logits"], layer["w13"], layer["w13_scale"], layer["w2"], layer["w2_scale"], 8,
+                        True, None, out, scratch=sc, check=True)
+        seen.append(int(mk.workspace_view(sc["workspace"])["phase_ns"][6]) != 0)
+    assert seen == [True, False, True]
+
+
 @pytest.mark.parametrize("build,T,skew,between,splits", CHOICES, ids=[f"{b[0]}-{T}-{s}" for b, T, s, _, _ in CHOICES])
 def test_the_units_of_the_batch_decide(build, T, skew, between, splits):
     (a, a_split, units), (b, b_split, _) = _run(build, T, skew)

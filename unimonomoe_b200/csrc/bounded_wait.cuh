@@ -50,7 +50,8 @@ struct Workspace {
   int32_t expert_offsets[kNumExperts + 1];  // exclusive prefix sum of expert_counts
   int32_t reserved1[3];
   int32_t cta_hist[kGrid][kNumExperts];     // per-CTA histograms (basis of the stable scatter)
-  uint64_t phase_ns[8];                     // %globaltimer at phase boundaries, written by block 0
+  uint64_t phase_ns[8];                     // %globaltimer at phase boundaries, written by block 0; [6]: between the halves of
+                                            // the split form, 0 if this launch computed whole units
   uint64_t prof[kGrid][64];                 // per-CTA stall counters (cycles), filled only by MONO_PROFILE builds
 };
 constexpr size_t kWorkspaceZeroBytes = offsetof(Workspace, total_tiles);

@@ -1092,7 +1092,10 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   int* ph1_tot = scan_tile + E;
   int* ph1_pre = ph1_tot + E;
 
-  if (bid == 0 && tid == 0) ws->phase_ns[0] = globaltimer_ns();
+  if (bid == 0 && tid == 0) {
+    ws->phase_ns[0] = globaltimer_ns();
+    ws->phase_ns[6] = 0;   // written again by a launch that takes the split form
+  }
 
   // launch sequence of the tensor-parallel epilogue: a device counter outside the
   // workspace (which is zeroed every launch) so that CUDA-graph replays advance it
