@@ -518,33 +518,40 @@ def test_router_linear_inside_the_launch(gu, oracle, qwen_full, T):
     assert torch.equal(res["out"].view(torch.int16), out.view(torch.int16))
 
 
-def test_tiny_batches_repeated(gu, qwen_full):
-    """At one or a few tokens almost every CTA has no tile and runs straight through the expert phase:
-    the hand-back of registers between producer and epilogue warps must not depend on who asks first.
-    150 launches each of 1 and 7 tokens, through both entries, with a host-side deadline instead of a
-    blocking synchronise so that a stall fails the test."""
+# tokens, skew, workspace without room for the split form, which form the logits-in launches take
+@pytest.mark.parametrize("T,skew,small,splits", [(1, 0.0, False, True), (7, 0.0, False, True), (1, 0.0, True, False),
+                                                 (16, 0.0, False, False), (32, 0.5, False, False)])
+def test_tiny_batches_repeated(gu, qwen_full, T, skew, small, splits):
+    """At one or a few tokens many CTAs have no tile. In the whole-unit form (no room for the split form; 16 tokens, 106
+    units on 148 SMs; 32 uneven tokens, 124 units in the instance that holds both forms) such a CTA runs straight through
+    the expert phase: the hand-back of registers between producer and epilogue warps must not depend on who asks first. In
+    the split form it waits at the counter between the halves. 150 launches each, through both entries, with a host-side
+    deadline instead of a blocking synchronise so that a stall fails the test."""
     import time
     mk = gu.kernel("qwen_w1")
     from unimonomoe_b200.loader import prepare_router_weight
     rw16 = prepare_router_weight(qwen_full["router_w"].to(torch.bfloat16))
-    for T in (1, 7):
-        batch = synth.make_batch(synth.QWEN, qwen_full, T, seed=11, device=gu.DEV)
-        out = torch.empty(T, 2048, dtype=torch.bfloat16, device=gu.DEV)
-        first = None
-        for i in range(150):
-            ev = torch.cuda.Event()
-            mk.prefill_impl(batch["hs"], batch["logits"], qwen_full["w13"], qwen_full["w13_scale"], qwen_full["w2"],
-                            qwen_full["w2_scale"], 8, True, None, out, router_weight=rw16 if i % 2 else None)
-            ev.record()
-            t0 = time.time()
-            while not ev.query():
-                assert time.time() - t0 < 10.0, f"launch {i} at T={T} did not finish within 10 s"
-                time.sleep(0.001)
-            if i % 2 == 0:
-                if first is None:
-                    first = out.clone()
-                assert torch.equal(out.view(torch.int16), first.view(torch.int16))
-        mk.check_status(mk.scratch(T, gu.DEV)["workspace"])
+    batch = synth.make_batch(synth.QWEN, qwen_full, T, seed=T if skew else 11, device=gu.DEV, skew=skew)
+    out = torch.empty(T, 2048, dtype=torch.bfloat16, device=gu.DEV)
+    sc = dict(mk.scratch(T, gu.DEV))
+    if small:
+        sc["workspace"] = sc["workspace"][:mk._int_symbol("workspace_min_bytes")]
+    first = None
+    for i in range(151):
+        ev = torch.cuda.Event()
+        mk.prefill_impl(batch["hs"], batch["logits"], qwen_full["w13"], qwen_full["w13_scale"], qwen_full["w2"],
+                        qwen_full["w2_scale"], 8, True, None, out, router_weight=rw16 if i % 2 else None, scratch=sc)
+        ev.record()
+        t0 = time.time()
+        while not ev.query():
+            assert time.time() - t0 < 10.0, f"launch {i} at T={T} did not finish within 10 s"
+            time.sleep(0.001)
+        if i % 2 == 0:
+            if first is None:
+                first = out.clone()
+            assert torch.equal(out.view(torch.int16), first.view(torch.int16))
+    mk.check_status(sc["workspace"])
+    assert (int(mk.workspace_view(sc["workspace"])["phase_ns"][6]) != 0) == splits
 
 
 def test_descriptors_are_made_once_per_weight_tensor(gu, qwen_full):
