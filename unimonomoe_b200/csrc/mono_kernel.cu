@@ -149,9 +149,9 @@ static_assert(ROUTER_MODE != 2 || N_GROUP * 32 == E, "grouped routing assumes 32
 // ------------------------------------------------------------------ launch shape
 // Warps 0-3 are the producer warpgroup (weight TMA, MMA issue, two gather warps); the epilogue is
 // EPI_WGS warpgroups of 128 threads. Thread i of an epilogue warpgroup owns row i of the tile
-// (TMEM lane i); warpgroup h owns columns [h*WC, (h+1)*WC) of every accumulator buffer: HCB gate
-// columns followed by the HCB matching up columns in the up projection, WC output columns in
-// the down projection.
+// (TMEM lane i); warpgroup h owns WC columns of every accumulator buffer: HCB gate columns and the HCB
+// matching up columns in the up projection (side by side, or BC / 2 apart where a stage comes in one box:
+// ONE_BOX below), output columns [h*WC, (h+1)*WC) in the down projection.
 #ifndef MONO_EPI_WGS
 #define MONO_EPI_WGS 2
 #endif
@@ -182,9 +182,9 @@ constexpr int PASS_STRIDE = 128 / NSPLIT;  // intermediate columns covered by on
 constexpr int LDW = (WC <= 64) ? WC : HCB;  // TMEM columns per tcgen05.ld
 constexpr int NLD = WC / LDW;
 // One TMA request per weight stage where a stage is one MMA operand: for one SM alone the copy engine takes 861 cycles for
-// 32 KB as one box of 256 rows of 128 bytes and 1142 as four boxes of 64 rows. (The layer gains 0.5 % from it at every
-// batch size: with three stages a step is otherwise bound by what an SM takes in from L2, 48 KB of weights and rows.) A
-// box cannot interleave gate and up rows, so a stage of the up projection holds the pass's 128 gate rows and then its 128
+// 32 KB as one box of 256 rows of 128 bytes and 1142 as four boxes of 64 rows. Whole units gain nothing measurable from it
+// (four-way shard at 8192 tokens 237 -> 238 us, H=7168 at 16384 1968 -> 1966, each within the runs' spread): a step is bound
+// by what an SM takes in from L2, 48 KB of weights and rows. The split form is written for it. A box cannot interleave gate and up rows, so a stage of the up projection holds the pass's 128 gate rows and then its 128
 // up rows, and a warpgroup's columns of such a buffer are two pieces BC / 2 apart.
 constexpr bool ONE_BOX = !PAIR && NSPLIT == 1 && EPI_WGS == 2;
 constexpr int DOWN_BOX = ONE_BOX ? 256 : HCB;  // rows of a box of the down projection's weights
@@ -207,7 +207,13 @@ constexpr int MAX_TILES = MAX_MY_TILES * kGrid;
 // counter, every (unit, 256-column pass of the down projection). The intermediate leaves shared memory, and the weight
 // ring takes its place. The operations on a row and their order are those of the whole unit: the same bits come out.
 // (With one pass of the up projection per unit there is too little to cut: no number of units makes it pay.)
-constexpr bool SPLIT_BUILD = ONE_BOX && NP > 1 && MONO_ABLATE == 0;
+// Profiling and ablation builds compute whole units: the stall counters and the switches are in that loop only.
+#ifdef MONO_PROFILE
+constexpr bool PROFILE_BUILD = true;
+#else
+constexpr bool PROFILE_BUILD = false;
+#endif
+constexpr bool SPLIT_BUILD = ONE_BOX && NP > 1 && MONO_ABLATE == 0 && !PROFILE_BUILD;
 constexpr size_t SPLIT_ROW_BYTES = N_HALF + NPT * sizeof(float);  // e4m3 intermediate and its scales, one row
 constexpr int SPLIT_ROWS = SPLIT_BUILD ? kGrid / NCH * TILE_M : 0;  // rows of the global intermediate: kGrid full units
 static_assert(kGrid % NCH == 0, "a wave of kGrid units holds whole tiles");
@@ -266,7 +272,9 @@ constexpr uint32_t IDESC = umma_idesc_e4m3_f32(PAIR ? 256 : 128, BC);
 constexpr uint32_t IDESC_ROUTER = umma_idesc_bf16_f32(128, E);
 constexpr int RK = K_DIM / 64;
 
-// Largest batch whose expert ids every CTA counts itself: the scan takes 3.6 us instead of 5.9 at 1 to 256 tokens.
+// Largest batch whose expert ids every CTA counts itself. Scan phase in us, histograms -> own count: 1 token 5.5 -> 3.1, 256
+// 5.8 -> 4.1, 512 6.0 -> 4.4, 1024 6.1 -> 5.7, 2048 6.6 -> 7.7, 4096 6.6 -> 12.1 (H=7168: 256 7.7 -> 5.6, 1024 8.3 -> 7.6,
+// 2048 8.0 -> 9.7). The two meet between 1024 and 2048 tokens; beyond 256 what is saved is below 1 % of the launch.
 constexpr int kDirectTokens = 256;
 constexpr uint32_t kSplitCounter = 3;  // workspace counter between the halves of the split form (0-2: grid barriers)
 
@@ -329,7 +337,7 @@ struct Params {
 
 // e == SHARED_E marks a tile of the shared expert: its rows are the tokens row0 .. row0 + rows - 1 themselves
 // (no sort indirection), its weights the shared expert's.
-struct TileInfo {
+struct alignas(16) TileInfo {   // read as one 16-byte word
   int e, row0, rows, chunk;
 };
 constexpr int SHARED_E = E_LOCAL;
@@ -607,7 +615,6 @@ struct __align__(16) SharedState {
   uint32_t tmem_base;
   uint32_t flag;          // grid_sync result broadcast
   int n_my_tiles;
-  int total_tiles;
   int sp_units, sp_waves;        // split form: units, and waves of them through the intermediate (0: whole units)
   uint32_t sp_flag, sp_gflag;    // split form: counter reached (epilogue, gather warps)
   TileInfo tiles[MAX_MY_TILES];
@@ -625,23 +632,17 @@ static_assert(sizeof(SharedState) <= SMEM_STATIC_RESERVE, "static shared state e
 // ------------------------------------------------------------------ pieces of the split form's epilogue
 // (The whole-unit loop has the same sections in line: with these functions called there the expert phase of the H = 7168
 // build took 3 % longer at 16384 tokens, its loop has no register to spare.)
-// SiLU(gate) * up (kernel/qwen_tp/src/prefill_mono_final_nb.cu:678), written over the gate columns; returns the amax
-// of this thread's columns.
+// SiLU(gate) * up as in the whole-unit loop (there the reason for this form of it), written over the gate columns; returns
+// the amax of this thread's columns.
 __device__ __forceinline__ float silu_mul(float2 (&acc)[TCOLS / 2]) {
   float mx = 0.f;
 #pragma unroll
-  for (int j = 0; j < ((MONO_ABLATE & 2) ? 0 : NSPLIT); ++j) {
-#pragma unroll
-    for (int i = 0; i < HCB / 2; ++i) {
-      const float2 g = acc[j * (WC / 2) + i], u = acc[j * (WC / 2) + HCB / 2 + i];
-      // the reference's form (exp and division on the special-function unit). A tanh.approx form needs one
-      // special-function operation instead of two and is 15 us faster per layer, but its 2^-11 relative error
-      // moves enough e4m3 codes of the intermediate to push about one output in 10^5 beyond 2e-2 rms
-      const float v0 = __fdividef(u.x * g.x, 1.0f + __expf(-g.x));
-      const float v1 = __fdividef(u.y * g.y, 1.0f + __expf(-g.y));
-      acc[j * (WC / 2) + i] = make_float2(v0, v1);
-      mx = fmaxf(mx, fmaxf(fabsf(v0), fabsf(v1)));
-    }
+  for (int i = 0; i < HCB / 2; ++i) {
+    const float2 g = acc[i], u = acc[HCB / 2 + i];
+    const float v0 = __fdividef(u.x * g.x, 1.0f + __expf(-g.x));
+    const float v1 = __fdividef(u.y * g.y, 1.0f + __expf(-g.y));
+    acc[i] = make_float2(v0, v1);
+    mx = fmaxf(mx, fmaxf(fabsf(v0), fabsf(v1)));
   }
   return mx;
 }
@@ -659,37 +660,31 @@ __device__ __forceinline__ void store_rows(const Params& p, const float2 (&acc)[
   // Neighbouring lanes swap half of their 32-byte pieces first, so that in every store instruction
   // lanes 2i and 2i+1 write 64 contiguous bytes of ONE row: 16 lines per instruction instead of 32.
   // (the guard is made warp-uniform: the shuffles below need every lane of the warp)
-  if (__all_sync(0xFFFFFFFFu, ok) && (MONO_ABLATE & 4) == 0) {
+  if (__all_sync(0xFFFFFFFFu, ok)) {
     const bool odd = (lane & 1) != 0;
     const int fi_even = __shfl_sync(0xFFFFFFFFu, fi, lane & ~1), fi_odd = __shfl_sync(0xFFFFFFFFu, fi, lane | 1);
     __nv_bfloat16* row_even = p.partial + (static_cast<size_t>(fi_even < 0 ? 0 : fi_even) * NCH + chunk) * H_DIM + col0;
     __nv_bfloat16* row_odd = p.partial + (static_cast<size_t>(fi_odd < 0 ? 0 : fi_odd) * NCH + chunk) * H_DIM + col0;
 #pragma unroll
-    for (int j = 0; j < NSPLIT; ++j) {
-      __nv_bfloat16* dst_even = row_even + j * BC;
-      __nv_bfloat16* dst_odd = row_odd + j * BC;
+    for (int k2 = 0; k2 < WC / 32; ++k2) {   // pieces 2*k2 and 2*k2+1 of this thread's WC columns
+      uint32_t lo[8], hi[8], mine[8], theirs[8];
 #pragma unroll
-      for (int k2 = 0; k2 < WC / 32; ++k2) {   // pieces 2*k2 and 2*k2+1 of this thread's WC columns of buffer j
-        uint32_t lo[8], hi[8], mine[8], theirs[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float2 a = __fmul2_rn(acc[j * (WC / 2) + (2 * k2) * 8 + i], rw2);
-          const float2 b = __fmul2_rn(acc[j * (WC / 2) + (2 * k2 + 1) * 8 + i], rw2);
-          lo[i] = cvt_bf16x2_satfinite(a.x, a.y);
-          hi[i] = cvt_bf16x2_satfinite(b.x, b.y);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          // an even lane keeps its piece 2*k2 and gives away 2*k2+1; an odd lane the other way round
-          const uint32_t send = odd ? lo[i] : hi[i];
-          theirs[i] = (MONO_ABLATE & 256) ? send : __shfl_xor_sync(0xFFFFFFFFu, send, 1);
-          mine[i] = odd ? hi[i] : lo[i];
-        }
-        const int piece = 2 * k2 + (odd ? 1 : 0);
-        // row of the even lane: its own piece from the even lane, the received one from the odd lane
-        if (fi_even >= 0) st_global_256_stream(dst_even + piece * 16, odd ? theirs : mine);
-        if (fi_odd >= 0) st_global_256_stream(dst_odd + piece * 16, odd ? mine : theirs);
+      for (int i = 0; i < 8; ++i) {
+        const float2 a = __fmul2_rn(acc[(2 * k2) * 8 + i], rw2);
+        const float2 b = __fmul2_rn(acc[(2 * k2 + 1) * 8 + i], rw2);
+        lo[i] = cvt_bf16x2_satfinite(a.x, a.y);
+        hi[i] = cvt_bf16x2_satfinite(b.x, b.y);
       }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        // an even lane keeps its piece 2*k2 and gives away 2*k2+1; an odd lane the other way round
+        theirs[i] = __shfl_xor_sync(0xFFFFFFFFu, odd ? lo[i] : hi[i], 1);
+        mine[i] = odd ? hi[i] : lo[i];
+      }
+      const int piece = 2 * k2 + (odd ? 1 : 0);
+      // row of the even lane: its own piece from the even lane, the received one from the odd lane
+      if (fi_even >= 0) st_global_256_stream(row_even + piece * 16, odd ? theirs : mine);
+      if (fi_odd >= 0) st_global_256_stream(row_odd + piece * 16, odd ? mine : theirs);
     }
   }
 }
@@ -1094,7 +1089,6 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
 
   if (bid == 0 && tid == 0) {
     ws->phase_ns[0] = globaltimer_ns();
-    ws->phase_ns[6] = 0;   // written again by a launch that takes the split form
   }
 
   // launch sequence of the tensor-parallel epilogue: a device counter outside the
@@ -1389,7 +1383,6 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     if (tid < E) {
       const int off_e = scan_cnt[tid] - cnt;
       const int tbase = scan_tile[tid] - tiles_e;
-      if (tid == E - 1) S.total_tiles = tbase + tiles_e;
       if (bid == 0) {
         ws->expert_counts[tid] = cnt;
         ws->expert_offsets[tid] = off_e;
@@ -1465,7 +1458,10 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   }
 
   alive = grid_sync(wc, 1, &S.flag) && alive;
-  if (bid == 0 && tid == 0) ws->phase_ns[2] = globaltimer_ns();
+  if (bid == 0 && tid == 0) {
+    ws->phase_ns[2] = globaltimer_ns();
+    ws->phase_ns[6] = 0;   // written again by a launch that takes the split form
+  }
   // phase 1 wrote the operand rings with ordinary stores (histograms, scan arrays); phase 2 fills them through
   // the async proxy (TMA), so order the two proxies once here
   fence_proxy_async_smem();
@@ -2564,7 +2560,7 @@ int prefill_wgmma_tp_pad_words(int nchunk, int ncomm, int world) { return (nchun
 int prefill_wgmma_up_pipe() { return SB; }
 int prefill_wgmma_dn_pipe() { return SB; }
 int prefill_wgmma_a_stages() { return SA; }
-int prefill_wgmma_shm_total() { return DYN_SMEM + static_cast<int>(sizeof(SharedState)); }
+int prefill_wgmma_shm_total() { return SHORT_DYN_SMEM + static_cast<int>(sizeof(SharedState)); }
 
 // ---- additions of this build (new capability = new symbol)
 int prefill_wgmma_arch() { return 100; }
