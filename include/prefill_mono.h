@@ -255,7 +255,7 @@ int prefill_wgmma_total_tiles_offset(void);   /* i32 */
 /* u64 [8] %globaltimer: [0] start, [1] routed and quantised, [2] sorted, [3] experts computed, [4] summed; [6] between
  * the two halves of the split form's expert phase, 0 when the launch computed whole units */
 int prefill_wgmma_phase_ns_offset(void);
-int prefill_wgmma_prof_offset(void);          /* u64 [148][16] stall counters, filled only by profiling builds */
+int prefill_wgmma_prof_offset(void);          /* u64 [148][64] stall counters, filled only by profiling builds */
 /* Debug dump targets for later launches (device pointers or null): raw gate|up sums
  * fp32 [T*k, 2*N_HALF], e4m3 intermediate [T*k, N_HALF], its scales fp32 [T*k, N_HALF/128],
  * indexed by sorted row. */

@@ -184,8 +184,9 @@ constexpr int NLD = WC / LDW;
 // One TMA request per weight stage where a stage is one MMA operand: for one SM alone the copy engine takes 861 cycles for
 // 32 KB as one box of 256 rows of 128 bytes and 1142 as four boxes of 64 rows. Whole units gain nothing measurable from it
 // (four-way shard at 8192 tokens 237 -> 238 us, H=7168 at 16384 1968 -> 1966, each within the runs' spread): a step is bound
-// by what an SM takes in from L2, 48 KB of weights and rows. The split form is written for it. A box cannot interleave gate and up rows, so a stage of the up projection holds the pass's 128 gate rows and then its 128
-// up rows, and a warpgroup's columns of such a buffer are two pieces BC / 2 apart.
+// by what an SM takes in from L2, 48 KB of weights and rows. The split form is written for it. A box cannot interleave gate
+// and up rows, so a stage of the up projection holds the pass's 128 gate rows and then its 128 up rows, and a warpgroup's
+// columns of such a buffer are two pieces BC / 2 apart.
 constexpr bool ONE_BOX = !PAIR && NSPLIT == 1 && EPI_WGS == 2;
 constexpr int DOWN_BOX = ONE_BOX ? 256 : HCB;  // rows of a box of the down projection's weights
 static_assert(HCB == 32 || HCB == 64, "unsupported split of the accumulator between warpgroups");
