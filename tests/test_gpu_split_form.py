@@ -14,7 +14,8 @@ DEV = "cuda:0"
 WIDE = synth.LayerSpec("wide", hidden=9216, inter=256)
 
 # build: (binary, layer, intermediate columns, local experts, shared expert). A case: build, tokens, skew, where the
-# tokens go (None: as the router says; otherwise (n, the experts of the first n tokens, the experts of the others)).
+# tokens go (None: as the router says; "apart": each to eight experts of its own; otherwise
+# (n, the experts of the first n tokens, the experts of the others)).
 # Fewer passes than SMs, about one round of units and (even routing) somewhat more than one, ragged and full tiles, the
 # shared expert's tiles, units in chunks
 W1, SHARED = ("qwen_w1", synth.QWEN, 512, 256, False), ("qwen_w1", synth.QWEN, 512, 256, True)
@@ -50,8 +51,12 @@ def _run(build, T, skew, experts=None):
     layer, mk = _layer(build), MonoKernel(path)
     batch = synth.make_batch(spec, layer, T, seed=T, device=DEV, skew=skew)
     if experts is not None:
-        n, first, others = experts
         batch["logits"] -= 50.0
+        if experts == "apart":
+            for t in range(T):
+                batch["logits"][t, 8 * t:8 * t + 8] += 100.0
+    if isinstance(experts, tuple):
+        n, first, others = experts
         batch["logits"][:n, list(first)] += 100.0
         batch["logits"][n:, list(others)] += 100.0
     emap = synth.expert_map(spec, 0, 256 // local, device=DEV) if local != 256 else None
@@ -84,13 +89,6 @@ def test_split_units_give_the_bits_of_whole_units(build, T, skew, experts):
     assert bool(torch.isfinite(a.view(torch.bfloat16).float()).all())
 
 
-# 148 units fill one round of whole units, in which splitting does not pay from about 75 on: up to there, and from 149
-# to about 185, the split form. 32 tokens reach 169 experts at even routing, 124 at skew 0.5, 69 at skew 1.0.
-EP4 = ("qwen_ep4", synth.QWEN, 512, 64, False)
-CHOICES = [(W1, 32, 0.0, (149, 185), True), (W1, 32, 0.5, (76, 148), False), (W1, 32, 1.0, (1, 74), True),
-           (W1, 16, 0.0, (76, 148), False), (EP4, 7500, 0.0, (76, 148), False), (EP4, 8192, 0.0, (149, 185), True)]
-
-
 def test_the_time_stamp_tells_which_form_ran():
     """Two launches on one workspace: the second computes whole units and must not keep the first one's time stamp."""
     layer, mk = _layer(W1), MonoKernel(variant_path("qwen_w1"))
@@ -105,9 +103,19 @@ def test_the_time_stamp_tells_which_form_ran():
     assert seen == [True, False, True]
 
 
-@pytest.mark.parametrize("build,T,skew,between,splits", CHOICES, ids=[f"{b[0]}-{T}-{s}" for b, T, s, _, _ in CHOICES])
-def test_the_units_of_the_batch_decide(build, T, skew, between, splits):
-    (a, a_split, units), (b, b_split, _) = _run(build, T, skew)
+# 148 units fill one round of whole units, in which splitting does not pay from about 75 on (where a unit is long, H =
+# 7168 and 512 columns, from 112 on, and with a few rows a tile it pays throughout): up to there, and from 149 to about 203, the split form. 32 tokens reach 169 experts at even routing,
+# 124 at skew 0.5, 69 at skew 1.0.
+EP4, TP4 = ("qwen_ep4", synth.QWEN, 512, 64, False), ("ds_tp4", synth.DEEPSEEK, 512, 256, False)
+CHOICES = [(W1, 32, 0.0, None, (149, 203), True), (W1, 32, 0.5, None, (76, 148), False), (W1, 32, 1.0, None, (1, 74), True),
+           (W1, 16, 0.0, None, (76, 148), False), (EP4, 7500, 0.0, None, (76, 148), False),
+           (EP4, 8192, 0.0, None, (149, 203), True), (TP4, 12, 0.0, "apart", (96, 96), True),
+           (TP4, 28, 0.5, None, (112, 148), True), (W1, 9, 0.0, "apart", (72, 72), True)]
+
+
+@pytest.mark.parametrize("build,T,skew,experts,between,splits", CHOICES, ids=[f"{c[0][0]}-{c[1]}-{c[3] or c[2]}" for c in CHOICES])
+def test_the_units_of_the_batch_decide(build, T, skew, experts, between, splits):
+    (a, a_split, units), (b, b_split, _) = _run(build, T, skew, experts)
     assert between[0] <= units <= between[1]
     assert (a_split, b_split) == (splits, False)
     assert torch.equal(a, b)

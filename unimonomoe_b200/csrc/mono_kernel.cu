@@ -710,29 +710,36 @@ __device__ __forceinline__ SplitShare split_share(int n, int bid) {
   return s;
 }
 
-// Which batches the split form is faster for: those with at most SPLIT_MOST[r] units in the last of r + 1 rounds of whole
-// units. Every CTA looks that up in phase 1, where the units are known: how many experts a batch reaches depends on how
-// uneven its routing is, and a rule on the number of tokens alone loses a quarter of the expert phase where one round of
-// whole units suffices. The bounds come from the slab steps of the busiest CTA. A split step costs 1.3 to 1.4 whole ones
-// in the builds with H = 2048 (with all SMs loading weights; the down passes fetch their rows again, and every pass starts
-// its pipeline anew) and 1.05 to 1.25 with H = 7168. Measured, expert phase in us with weights from memory, whole -> split,
-// and what the rule takes: H=2048 I=512: 8 units 63 -> 29, 58 70 -> 62, 71 71 -> 67 (split); 76 72 -> 79, 106 79 -> 86,
-// 135 88 -> 104 (whole); 151 143 -> 118, 169 144 -> 122, 183 142 -> 132 (split); 189 142 -> 147, 256 153 -> 160 (whole).
-// I=256: 69 units 46 -> 40 (split), 79 46 -> 53 (whole). H=7168 I=256: 66 units 122 -> 90 (split), 85 124 -> 135 (whole),
-// 156 242 -> 203 (split).
+// Which batches the split form is faster for: those whose units do not exceed SPLIT_MOST_1 (one round of whole units) or
+// lie in the second round up to SPLIT_MOST_2. Every CTA looks that up in phase 1, where the units are known: how many
+// experts a batch reaches depends on how uneven its routing is, and a rule on the number of tokens alone loses a quarter of
+// the expert phase where one round of whole units suffices. The bounds compare the slab steps of the busiest CTA. A split
+// step costs 1.3 to 1.4 whole ones at H = 2048 (with all SMs loading weights; the down passes fetch their rows again, and
+// every pass starts its pipeline anew), less where a pass has more slabs or the batch is bound by memory in either form.
+// Measured, expert phase in us with weights from memory, whole -> split. H=2048 I=512, taken split: 8 units 63 -> 29, 58
+// 70 -> 62, 71 71 -> 67, 151 143 -> 118, 169 144 -> 122, 183 142 -> 132, 190 144 -> 136 (with full tiles 142 -> 147); taken
+// whole: 76 72 -> 79, 106 79 -> 86, 135 88 -> 104, 256 153 -> 160. I=256: 69 46 -> 40, 169 84 -> 79 (split), 79 46 -> 53
+// (whole). H=7168 I=256: 66 122 -> 90, 156 242 -> 203, 195 249 -> 216 (split), 85 124 -> 135 (whole). H=7168 I=512: 85
+// 270 -> 200, 95 275 -> 203, 156 541 -> 321 (split). There units of a few rows pay in the whole first round, the weights'
+// 11 MB a unit bound both forms and the split one deals them more evenly: 113 286 -> 251, a launch with 148 units 374 -> 329;
+// with full tiles they don't, 132 328 -> 345.
 constexpr int split_steps(int n) { return (n * NP + kGrid - 1) / kGrid * NK + (n * NHB + kGrid - 1) / kGrid * NP; }
-constexpr int split_most(int round, bool one_wave) {   // of the units beyond the full rounds of whole units
+// units beyond the full rounds of whole units, up to which the split form has less than `percent` of the whole units' steps
+constexpr int split_most(int round, bool one_wave, int percent) {
   int most = 0;
   for (int n = 1; n <= kGrid; ++n) {
     const int steps = one_wave ? split_steps(round * kGrid + n) : round * split_steps(kGrid) + split_steps(n);
-    if (steps * 10 < (round + 1) * (NP * NK + NHB * NP) * 7) most = n;
+    if (steps * 100 < (round + 1) * (NP * NK + NHB * NP) * percent) most = n;
   }
   return most;
 }
-constexpr int SPLIT_MOST_1 = split_most(0, true), SPLIT_MOST_2 = split_most(1, true), SPLIT_MOST_2W = split_most(1, false);
-static_assert(split_most(2, true) == 0, "the split form is looked up for one and two rounds of units");
-__device__ __forceinline__ bool split_pays(int units, bool one_wave) {
-  return units <= kGrid ? units <= SPLIT_MOST_1 : units <= kGrid + (one_wave ? SPLIT_MOST_2 : SPLIT_MOST_2W);
+constexpr int SPLIT_MOST_1 = split_most(0, true, K_DIM > 4096 ? 76 : 70);
+constexpr int SPLIT_MOST_2 = split_most(1, true, K_DIM > 4096 ? 80 : 75), SPLIT_MOST_2W = split_most(1, false, K_DIM > 4096 ? 80 : 75);
+constexpr bool LONG_UNITS = K_DIM > 4096 && NP > 2;
+constexpr int FEW_ROWS = 16;   // of a tile, on average
+__device__ __forceinline__ bool split_pays(int units, bool few_rows, bool one_wave) {
+  return units <= kGrid ? units <= SPLIT_MOST_1 || (LONG_UNITS && few_rows)
+                        : units <= kGrid + (one_wave ? SPLIT_MOST_2 : SPLIT_MOST_2W);
 }
 
 // Phase 2 in the split form, with the roles of the whole-unit form. Both halves are the same slab step (weights
@@ -1366,7 +1373,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     bool split = false;
     int lo = 0, hi = 0;       // this CTA's units of the last wave
     if constexpr (CAN_SPLIT) {
-      split = units > 0 && split_pays(units, one_wave);
+      split = units > 0 && split_pays(units, rows_routed * NCH <= FEW_ROWS * tt_routed, one_wave);
       const SplitShare mine = split_share(one_wave ? units : units - kGrid, bid);
       lo = mine.lo;
       hi = mine.hi;
@@ -2509,7 +2516,10 @@ bool short_expected(int num_tokens, int sh_units) {
   const double reached = 1.0 - pow(1.0 - static_cast<double>(TOP_K) / E, num_tokens);
   const double tiles = fmax(reached, rows < 0.75 * TILE_M ? 0.0 : rows / TILE_M + 0.5);
   const double units = ceil(E_LOCAL * tiles) * NCH + sh_units;
-  return units <= SPLIT_MOST_1 || (units > kGrid && units <= kGrid + SPLIT_MOST_2);
+  // 70 % of the steps, not the device's bounds: near those a few units decide, and a batch that then stays with whole units
+  // has paid for the instance
+  constexpr int most1 = split_most(0, true, 70), most2 = split_most(1, true, 70);
+  return units <= most1 || (units > kGrid && units <= kGrid + most2);
 }
 
 cudaError_t ensure_kernel_attribute(int dev) {
