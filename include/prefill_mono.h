@@ -34,8 +34,9 @@
  *   logits            fp32 [T, E]                      in
  *   workspace         prefill_wgmma_workspace_bytes(); zeroed by the launch itself as far as it has to be. What lies
  *                     behind prefill_wgmma_workspace_min_bytes() holds the intermediate of the split form (short
- *                     batches); a smaller workspace, or one that is not 16-byte aligned, is accepted and does without
- *                     that form: the same bits, later
+ *                     batches) or the positions of the slots in the sort (large ones, whose partial rows are then in
+ *                     sorted order); a smaller workspace, or one that is not 16-byte aligned, is accepted and does
+ *                     without either: the same bits, later
  *   act_bf16          bf16 [T, K]                      in
  *   act_fp8           u8   [T, K]                      scratch/out: e4m3 activations
  *   act_scales        fp32 [T, K/128]                  scratch/out

@@ -43,6 +43,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 #include "bounded_wait.cuh"
@@ -267,6 +268,25 @@ static_assert(128 * REGS_PRODUCER + N_EPI * REGS_EPILOGUE <= BLOCK * REGS_LAUNCH
               "setmaxnreg.inc would wait forever: the epilogue asks for more registers than the producers release");
 static_assert(REGS_LAUNCH * BLOCK <= 65536, "launch register count exceeds the register file");
 
+// ------------------------------------------------------------------ partial rows in sorted order
+// An SM pushes at most 32 B/clk towards L2, so the 64 KB of a down pass take 2.1 k cycles however they are stored; stored
+// by the epilogue itself they hold it up that long (2.7 k with packing and the lane exchange), and with it the tensor
+// core, which runs only two slabs ahead. With the rows in the order of the sort instead of the slots' a tile's rows are
+// neighbours in memory: a warp puts its 32 rows x 128 columns of a pass into the activation stages, which are idle during
+// the down projection (as many of its four blocks of 32 columns as they hold), and one copy-engine request takes them from
+// there while the next pass runs. The slot sum finds a token's rows through their positions, kept in the workspace.
+// Warps whose 32 rows are not all there store directly. Expert phase in us, slot order -> sorted order: H=2048 I=512, 16384
+// tokens 612 -> 584, 8192 378 -> 362, 5000 300 -> 287; H=7168 I=256, 16384 tokens 1265 -> 1076, 4096 439 -> 426. The slot
+// sum reads single rows instead of eight neighbours: 115 -> 117, H=7168 378 -> 397. Per-row requests in slot order
+// (scatter4) take 7 cycles a row: 18 B/clk with 128-byte rows. With 128 columns of intermediate a pass is one slab step
+// and has nothing to hide the stores behind (131 -> 131): those builds keep the slots' order.
+constexpr bool SORTED_BUILD = ONE_BOX && NP > 1;
+constexpr int ROW_BOX = 32;                  // rows, and columns of a block of a box
+constexpr int ROW_BLOCKS = SA < 4 ? SA : 4;  // blocks of a box: of the four of a pass, those that find room
+constexpr int ROW_SLOT_BYTES = ROW_BLOCKS * ROW_BOX * ROW_BOX * 2;
+constexpr bool LAST_IN_INTER = ROW_SLOT_BYTES * (N_EPI / 32) <= INTER_BYTES;
+static_assert(!SORTED_BUILD || ROW_SLOT_BYTES * (N_EPI / 32) <= SA * A_STAGE_BYTES, "one slot per epilogue warp in the activation stages");
+
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t IDESC = umma_idesc_e4m3_f32(PAIR ? 256 : 128, BC);
 // router GEMV: one [128 tokens x 256 experts] accumulator, K slabs of 64 bf16 (128 bytes)
@@ -277,12 +297,16 @@ constexpr int RK = K_DIM / 64;
 // 5.8 -> 4.1, 512 6.0 -> 4.4, 1024 6.1 -> 5.7, 2048 6.6 -> 7.7, 4096 6.6 -> 12.1 (H=7168: 256 7.7 -> 5.6, 1024 8.3 -> 7.6,
 // 2048 8.0 -> 9.7). The two meet between 1024 and 2048 tokens; beyond 256 what is saved is below 1 % of the launch.
 constexpr int kDirectTokens = 256;
+// Smallest batch whose partial rows are in sorted order: an expert then has a full tile on average. Launch in us, slot order ->
+// sorted, H=2048 I=512: 2048 tokens 193 -> 198, 3000 215 -> 221, 4096 298 -> 298, 5000 371 -> 361; H=7168 I=256: 2500 503 -> 508,
+// 4096 614 -> 609, 6000 824 -> 813; 128 of 256 experts: 4096 tokens 197 -> 191.
+constexpr int kSortedTokens = 4096;
 constexpr uint32_t kSplitCounter = 3;  // workspace counter between the halves of the split form (0-2: grid barriers)
 
 // wait sites reported in the status word
 enum Site : uint32_t {
   kSiteEmptyB = 1, kSiteFullB, kSiteFullA, kSiteEmptyA, kSiteTmemEmpty, kSiteTmemFull, kSiteInterReady,
-  kSiteRouterEmpty, kSiteRouterFull, kSiteRouterAccEmpty, kSiteRouterAccFull,
+  kSiteRouterEmpty, kSiteRouterFull, kSiteRouterAccEmpty, kSiteRouterAccFull, kSiteRowsRead,
 };
 
 struct Params {
@@ -326,6 +350,9 @@ struct Params {
   const __nv_bfloat16* sh_gate;   // [K] gate vector (sigmoid(x . g) scales the row), or null: weight 1
   float* sh_gate_w;               // [T] fp32, written by phase 0 when sh_gate is given
   int sh_on, sh_part, sh_parts;
+  // Partial rows in the order of the sort instead of the slots' (row = sorted position): a tile's rows are then
+  // neighbours and leave through the copy engine. [T*8] position of every slot (-1: no row here); null: in slot order
+  int32_t* slot_pos;
   // router GEMV (null: the caller supplied the logits)
   float* logits_out;        // [T, E] fp32, written by phase R and read back by phase 0
   alignas(64) CUtensorMap tm_up;
@@ -334,6 +361,7 @@ struct Params {
   alignas(64) CUtensorMap tm_rw;   // bf16 router weight [E, K]
   alignas(64) CUtensorMap tm_sh_up;    // shared expert [2 * N_HALF, K]
   alignas(64) CUtensorMap tm_sh_down;  // shared expert [H, N_HALF]
+  alignas(64) CUtensorMap tm_rows;     // sorted partial rows [rows, H], boxes of 32 rows
 };
 
 // e == SHARED_E marks a tile of the shared expert: its rows are the tokens row0 .. row0 + rows - 1 themselves
@@ -342,6 +370,8 @@ struct alignas(16) TileInfo {   // read as one 16-byte word
   int e, row0, rows, chunk;
 };
 constexpr int SHARED_E = E_LOCAL;
+
+enum Form { FORM_WHOLE, FORM_SHORT, FORM_SORTED };   // instances of the kernel
 
 // ------------------------------------------------------------------ small helpers
 __device__ __forceinline__ uint32_t float_key(float f) {
@@ -612,6 +642,7 @@ struct __align__(16) SharedState {
   uint64_t fullA[A_STAGE_CAP], emptyA[A_STAGE_CAP], fullB[B_STAGE_CAP], emptyB[B_STAGE_CAP];
   uint64_t tmem_full[NBUF], tmem_empty[NBUF];
   uint64_t inter_ready[4];  // one per 128-column pass of the intermediate (NP <= 4)
+  uint64_t rows_read;       // sorted partial rows: the copy engine has read the tile's rows out of the activation stages
   uint64_t rfull[4], rempty[4], racc_full, racc_empty;  // phase R only
   uint32_t tmem_base;
   uint32_t flag;          // grid_sync result broadcast
@@ -1063,10 +1094,12 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
 }
 
 // ------------------------------------------------------------------ the kernel
-// SHORT: the instance for batches that are expected to be short. It holds both forms of the expert phase and takes one of
-// them by the units that phase 1 counts. The other instance computes whole units only, and computes them faster: inside
+// FORM_SORTED: whole units with the partial rows in sorted order, an instance of its own because its store section changes
+// the registers of the slab loop (the others take 2 to 5 % longer with both in one).
+// FORM_SHORT: the instance for batches that are expected to be short. It holds both forms of the expert phase and takes one of
+// them by the units that phase 1 counts. FORM_WHOLE computes whole units only, and computes them faster: inside
 // the first one they take 2 to 4 us more a launch (16 tokens 85 -> 88 us, 64 of 256 experts at 7500 tokens 153 -> 157).
-template <bool SHORT>
+template <int FORM>
 __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t dyn_raw[];
   __shared__ SharedState S;
@@ -1078,7 +1111,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   const int T = p.num_tokens;
   const int numel = T * TOP_K;
 
-  constexpr bool CAN_SPLIT = SHORT && SPLIT_BUILD;
+  constexpr bool CAN_SPLIT = FORM == FORM_SHORT && SPLIT_BUILD;
+  constexpr bool SORTED = FORM == FORM_SORTED && SORTED_BUILD;
   constexpr int RS = (SA < SB) ? SA : SB;  // stages of the router linear's ring
   // 1024-byte aligned base of the operand buffers
   const uint32_t dyn_u32 = (smem_u32(dyn_raw) + 1023u) & ~1023u;
@@ -1455,11 +1489,13 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     for (int t = t_begin; t < t_end; ++t) {
       if (lane < TOP_K) {
         const int lid = p.topk_ids[t * TOP_K + lane];
+        int pos = -1;
         if (lid >= 0) {
-          const int pos = hist[warp * E + lid]++;
+          pos = hist[warp * E + lid]++;
           if (pos >= 0 && pos < numel) p.sorted_ids[pos] = t * TOP_K + lane;
           else report_error(ws, kErrBounds, 2, static_cast<uint32_t>(pos), static_cast<uint32_t>(t));
         }
+        if constexpr (SORTED) p.slot_pos[t * TOP_K + lane] = pos;
       }
       __syncwarp();
     }
@@ -1493,6 +1529,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     for (int i = 0; i < 48; ++i) (&S.whist[0][0])[i] = 0ull;
 #endif
     for (int s = 0; s < NP; ++s) mbar_init(&S.inter_ready[s], both * (N_EPI / 32));
+    mbar_init(&S.rows_read, N_EPI / 32);
     mbar_init_fence();
   }
   if (warp == WARP_MMA && !gemv) {  // phase R already holds the allocation
@@ -1784,6 +1821,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
           S.gather_tok[it & 1][r & 7][r >> 3] = t;
         }
         named_bar_sync(2, N_GATHER);
+        // the previous tile's partial rows pass through the activation stages
+        if (SORTED && it > 0 && !dead && !mbar_wait(&S.rows_read, static_cast<uint32_t>(it - 1) & 1u, wc, kSiteRowsRead)) dead = true;
         for (int s = 0; s < NP * NK; ++s) {
           const int ks = s % NK;
           const uint32_t sa = na % SA;
@@ -1931,6 +1970,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
           d[0] = as_v.x; d[TILE_M] = as_v.y; d[2 * TILE_M] = as_v.z; d[3 * TILE_M] = as_v.w;
         }
       };
+      // sorted partial rows: this warp's slot in the activation stages and in the intermediate
+      const uint32_t ring_slot = smem_u32(a_ring) + (warp - 4) * ROW_SLOT_BYTES, inter_slot = smem_u32(inter) + (warp - 4) * ROW_SLOT_BYTES;
       if (n_my > 0) {
         stage_ids(0);
         stage_weight_store(0);
@@ -1945,6 +1986,10 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
         const float* wsu_t = wsu_sm + (it & 1) * WSU_N;
         const float* wsd_t = wsd_sm + (it & 1) * WSD_N;
         const bool has_next = it + 1 < n_my;
+        // sorted rows of a tile follow one another from tile_row on; this thread's (-1: none)
+        const int tile_row = SORTED ? ti.chunk * (numel + (p.sh_on ? T : 0)) + (ti.e == SHARED_E ? numel : 0) + ti.row0 : 0;
+        const int prow = fi < 0 ? -1 : tile_row + r;
+        const bool box_full = SORTED && __all_sync(0xFFFFFFFFu, fi >= 0);
         float iscale[NP];
         { PROF_T0();
         named_bar_sync(1, N_EPI);  // this tile's staged scales are visible to all epilogue threads
@@ -2007,6 +2052,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
           }
           // the row's amax over the pass's 128 columns: every warpgroup holds NSPLIT*HCB of them
           S.rowmax[ps & 1][h][r] = mx;
+          if (SORTED && LAST_IN_INTER && ps == 0 && lane == 0) bulk_wait_read<0>();   // the previous tile's last rows have left the intermediate
           named_bar_sync(1, N_EPI);
 #pragma unroll
           for (int hh = 0; hh < EPI_WGS; ++hh) mx = fmaxf(mx, S.rowmax[ps & 1][hh][r]);
@@ -2073,20 +2119,22 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             }
           }
           PROF_T0();
+          const bool alive_w = !__any_sync(0xFFFFFFFFu, dead);
           // Neighbouring lanes swap half of their 32-byte pieces first, so that in every store instruction
           // lanes 2i and 2i+1 write 64 contiguous bytes of ONE row: 16 lines per instruction instead of 32.
-          // (the guard is made warp-uniform: the shuffles below need every lane of the warp)
-          if (!__any_sync(0xFFFFFFFFu, dead) && (MONO_ABLATE & 4) == 0) {
+          // (only in warp-uniform branches: the shuffles need every lane of the warp.) `row`: this thread's partial row, or
+          // -1; pieces 2*k2 and 2*k2+1 of its WC columns of a buffer, k2 from `first` on
+          auto store_direct = [&](auto first, int row, int step, int chunk) {
             const bool odd = (lane & 1) != 0;
-            const int fi_even = __shfl_sync(0xFFFFFFFFu, fi, lane & ~1), fi_odd = __shfl_sync(0xFFFFFFFFu, fi, lane | 1);
-            __nv_bfloat16* row_even = p.partial + (static_cast<size_t>(fi_even < 0 ? 0 : fi_even) * NCH + ti.chunk) * H_DIM + hb * 256 + h * WC;
-            __nv_bfloat16* row_odd = p.partial + (static_cast<size_t>(fi_odd < 0 ? 0 : fi_odd) * NCH + ti.chunk) * H_DIM + hb * 256 + h * WC;
+            const int row_e = __shfl_sync(0xFFFFFFFFu, row, lane & ~1), row_o = __shfl_sync(0xFFFFFFFFu, row, lane | 1);
+            __nv_bfloat16* row_even = p.partial + (static_cast<size_t>(row_e < 0 ? 0 : row_e) * step + chunk) * H_DIM + hb * 256 + h * WC;
+            __nv_bfloat16* row_odd = p.partial + (static_cast<size_t>(row_o < 0 ? 0 : row_o) * step + chunk) * H_DIM + hb * 256 + h * WC;
 #pragma unroll
             for (int j = 0; j < NSPLIT; ++j) {
               __nv_bfloat16* dst_even = row_even + j * BC;
               __nv_bfloat16* dst_odd = row_odd + j * BC;
 #pragma unroll
-              for (int k2 = 0; k2 < WC / 32; ++k2) {   // pieces 2*k2 and 2*k2+1 of this thread's WC columns of buffer j
+              for (int k2 = decltype(first)::value; k2 < WC / 32; ++k2) {
                 uint32_t lo[8], hi[8], mine[8], theirs[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -2104,14 +2152,56 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
                 }
                 const int piece = 2 * k2 + (odd ? 1 : 0);
                 // row of the even lane: its own piece from the even lane, the received one from the odd lane
-                if (fi_even >= 0) st_global_256_stream(dst_even + piece * 16, odd ? theirs : mine);
-                if (fi_odd >= 0) st_global_256_stream(dst_odd + piece * 16, odd ? mine : theirs);
+                if (row_e >= 0) st_global_256_stream(dst_even + piece * 16, odd ? theirs : mine);
+                if (row_o >= 0) st_global_256_stream(dst_odd + piece * 16, odd ? mine : theirs);
               }
             }
+          };
+          if constexpr (SORTED) {
+            // The last passes leave the activation stages to the gather warps, which refill them: the last one goes through
+            // the intermediate, which nothing reads any more, or where that is too small the last two are stored directly.
+            constexpr int RING_PASSES = LAST_IN_INTER ? NHB - 1 : NHB - 2;
+            const bool staged = box_full && alive_w && (hb < RING_PASSES || LAST_IN_INTER);
+            const uint32_t slot = hb < RING_PASSES ? ring_slot : inter_slot;
+            if (lane == 0) {
+              bulk_wait_read<0>();   // the previous pass's box has left its slot
+              if (hb == RING_PASSES) mbar_arrive(&S.rows_read);
+            }
+            __syncwarp();
+            if (staged) {
+              if constexpr (ROW_BLOCKS < WC / 32) store_direct(std::integral_constant<int, ROW_BLOCKS>(), prow, 1, 0);
+#pragma unroll
+              for (int c = 0; c < ROW_BLOCKS; ++c) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                  uint32_t w[4];
+#pragma unroll
+                  for (int i = 0; i < 4; ++i) {
+                    const float2 a = __fmul2_rn(acc[c * (ROW_BOX / 2) + k * 4 + i], rw2);
+                    w[i] = cvt_bf16x2_satfinite(a.x, a.y);
+                  }
+                  st_shared_128(slot + c * (ROW_BOX * ROW_BOX * 2) + lane * (ROW_BOX * 2) + ((k ^ ((lane >> 1) & 3)) << 4), w);   // the box's 64-byte swizzle
+                }
+              }
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                tma_store_3d_stream(&p.tm_rows, 0, static_cast<uint32_t>(tile_row + q * 32), static_cast<uint32_t>((hb * 256 + h * WC) / ROW_BOX), slot);
+                bulk_commit();
+              }
+            } else if (alive_w) {
+              store_direct(std::integral_constant<int, 0>(), prow, 1, 0);
+            }
+          } else if (alive_w && (MONO_ABLATE & 4) == 0) {
+            store_direct(std::integral_constant<int, 0>(), fi, NCH, ti.chunk);
           }
           if (has_next && hb >= 1 && hb - 1 < AS_PIECES) as_piece_store(hb - 1);
           PROF_ADD(pe_store);
         }
+      }
+      if (SORTED && lane == 0) {   // the rows are in memory, and visible to ordinary loads behind the grid barrier
+        bulk_wait_all();
+        fence_proxy_async();
       }
       if (et == 0) {
         PROF_STORE(8, pe_wait); PROF_STORE(9, pe_up); PROF_STORE(10, pe_silu); PROF_STORE(11, pe_down);
@@ -2274,19 +2364,36 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       return true;
     };
 
+    // per slot of a token: its position in the sort (sorted rows) or its expert id (EP), -1 where this rank has no row
+    constexpr bool BY_SLOTS = SORTED || EP_BUILD;
+    const int32_t* const slots = SORTED ? p.slot_pos : p.topk_ids;
+    auto slots_of = [&](uint32_t tok, int (&w)[TOP_K]) {
+      const int4* o = reinterpret_cast<const int4*>(slots + static_cast<size_t>(tok) * TOP_K);
+      const int4 o0 = o[0], o1 = o[1];   // (kept in L1: the threads of a token read the same 32 bytes)
+      w[0] = o0.x; w[1] = o0.y; w[2] = o0.z; w[3] = o0.w;
+      w[4] = o1.x; w[5] = o1.y; w[6] = o1.z; w[7] = o1.w;
+    };
+    // the chunks of a slot are neighbours in slot order and whole blocks of sorted rows apart
+    const uint32_t chunk_step = SORTED ? static_cast<uint32_t>(numel + (p.sh_on ? T : 0)) : 1u;
+
     if (!tp_on || bid < ncomp) {
-      const size_t stride = static_cast<size_t>(ncomp) * BLOCK;
+      const uint32_t stride = static_cast<uint32_t>(ncomp) * BLOCK;
       for (int c = 0; c < nchunk; ++c) {
-        const size_t c_lo = out_vec * c / nchunk, c_hi = out_vec * (c + 1) / nchunk;
-        for (size_t iv = c_lo + static_cast<size_t>(bid) * BLOCK + tid; iv < c_hi; iv += stride) {
-          const size_t tok = iv / HV;
+        const uint32_t c_lo = static_cast<uint32_t>(out_vec * c / nchunk), c_hi = static_cast<uint32_t>(out_vec * (c + 1) / nchunk);
+        int next[TOP_K];
+        uint32_t iv = c_lo + static_cast<uint32_t>(bid) * BLOCK + tid;
+        if (BY_SLOTS && iv < c_hi) slots_of(iv / HV, next);
+        for (; iv < c_hi; iv += stride) {
+          const uint32_t tok = iv / HV;
           const int hv = static_cast<int>(iv % HV);
-          int own[TOP_K];
-          if constexpr (EP_BUILD) {
-            const int4* o = reinterpret_cast<const int4*>(p.topk_ids + tok * TOP_K);
-            const int4 o0 = o[0], o1 = o[1];
-            own[0] = o0.x; own[1] = o0.y; own[2] = o0.z; own[3] = o0.w;
-            own[4] = o1.x; own[5] = o1.y; own[6] = o1.z; own[7] = o1.w;
+          int row[TOP_K];   // first partial row of every slot, -1: none
+          if constexpr (BY_SLOTS) {
+#pragma unroll
+            for (int k = 0; k < TOP_K; ++k) row[k] = SORTED || next[k] < 0 ? next[k] : static_cast<int>(tok * TOP_K + k) * NCH;
+            if (iv + stride < c_hi) slots_of((iv + stride) / HV, next);   // on their way while this vector is summed
+          } else {
+#pragma unroll
+            for (int k = 0; k < TOP_K; ++k) row[k] = static_cast<int>(tok * TOP_K + k) * NCH;
           }
           float s[W];
 #pragma unroll
@@ -2295,11 +2402,9 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
           uint4 raw[TOP_K * NCH];
 #pragma unroll
           for (int k = 0; k < TOP_K * NCH; ++k) {
-            bool mine = true;
-            if constexpr (EP_BUILD) mine = own[k / NCH] >= 0;
             raw[k] = make_uint4(0u, 0u, 0u, 0u);
-            if (mine)
-              raw[k] = __ldcg(reinterpret_cast<const uint4*>(p.partial + (tok * (TOP_K * NCH) + k) * H_DIM + hv * W));
+            if (row[k / NCH] >= 0)
+              raw[k] = __ldcg(reinterpret_cast<const uint4*>(p.partial + (static_cast<size_t>(row[k / NCH]) + (k % NCH) * chunk_step) * H_DIM + hv * W));
           }
 #pragma unroll
           for (int k = 0; k < TOP_K * NCH; ++k) {
@@ -2316,15 +2421,16 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             if (static_cast<int>(tok / TILE_M) % p.sh_parts == p.sh_part) {   // rows this launch computed
 #pragma unroll
               for (int c = 0; c < NCH; ++c) {
+                const size_t srow = static_cast<size_t>(numel) + tok;
                 const uint4 sr = __ldcg(reinterpret_cast<const uint4*>(
-                    p.partial + ((static_cast<size_t>(numel) + tok) * NCH + c) * H_DIM + hv * W));
+                    p.partial + (SORTED ? static_cast<size_t>(c) * chunk_step + srow : srow * NCH + c) * H_DIM + hv * W));
                 const __nv_bfloat16* sb = reinterpret_cast<const __nv_bfloat16*>(&sr);
 #pragma unroll
                 for (int i = 0; i < W; ++i) base[i] += __bfloat162float(sb[i]);
               }
             }
             if (p.residual != nullptr) {
-              const uint4 rr = *reinterpret_cast<const uint4*>(p.residual + iv * W);
+              const uint4 rr = *reinterpret_cast<const uint4*>(p.residual + static_cast<size_t>(iv) * W);
               const __nv_bfloat16* rb = reinterpret_cast<const __nv_bfloat16*>(&rr);
 #pragma unroll
               for (int i = 0; i < W; ++i) base[i] += __bfloat162float(rb[i]);
@@ -2332,7 +2438,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
 #pragma unroll
             for (int i = 0; i < W; ++i) o[i] = __float2bfloat16(__fmaf_rn(s[i], p.out_scale, base[i]));
           } else if (p.residual != nullptr) {
-            const uint4 rr = *reinterpret_cast<const uint4*>(p.residual + iv * W);
+            const uint4 rr = *reinterpret_cast<const uint4*>(p.residual + static_cast<size_t>(iv) * W);
             const __nv_bfloat16* rb = reinterpret_cast<const __nv_bfloat16*>(&rr);
 #pragma unroll
             for (int i = 0; i < W; ++i) o[i] = __float2bfloat16(__fmaf_rn(s[i], p.out_scale, __bfloat162float(rb[i])));
@@ -2340,7 +2446,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
 #pragma unroll
             for (int i = 0; i < W; ++i) o[i] = __float2bfloat16(__fmul_rn(s[i], p.out_scale));
           }
-          *reinterpret_cast<uint4*>(p.out + iv * W) = *reinterpret_cast<const uint4*>(o);
+          *reinterpret_cast<uint4*>(p.out + static_cast<size_t>(iv) * W) = *reinterpret_cast<const uint4*>(o);
         }
         if (!tp_on) continue;
         __threadfence_system();  // a peer's communication block reads these bytes through the multicast alias
@@ -2462,6 +2568,19 @@ int make_bf16_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
+// Sorted partial rows [rows, H] bf16 as blocks of 32 columns: a box is 32 rows of ROW_BLOCKS neighbouring blocks.
+int make_rows_map(CUtensorMap* m, void* base, uint64_t rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return -1;
+  cuuint64_t gd[3] = {ROW_BOX, rows, H_DIM / ROW_BOX};
+  cuuint64_t gs[2] = {H_DIM * 2, ROW_BOX * 2};
+  cuuint32_t bx[3] = {ROW_BOX, ROW_BOX, ROW_BLOCKS};
+  cuuint32_t es[3] = {1u, 1u, 1u};
+  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, gd, gs, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
+}
+
 // Plan / run split. What a launch needs besides its arguments depends only on the device (the kernel's
 // shared-memory attribute) and on the weight tensors (their TMA descriptors: base address + the compiled
 // extents). Both are made once and kept: a descriptor per (kind, base address, rows) in a small table, the
@@ -2525,10 +2644,14 @@ bool short_expected(int num_tokens, int sh_units) {
 cudaError_t ensure_kernel_attribute(int dev) {
   std::lock_guard<std::mutex> lock(g_plan_mutex);
   if (dev >= 0 && dev < 64 && g_attr_set[dev]) return cudaSuccess;
-  cudaError_t err = cudaFuncSetAttribute(moe_prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM);
+  cudaError_t err = cudaFuncSetAttribute(moe_prefill_kernel<FORM_WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM);
+  if constexpr (SORTED_BUILD) {
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(moe_prefill_kernel<FORM_SORTED>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM);
+  }
   if constexpr (SPLIT_BUILD) {
     if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(moe_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SHORT_DYN_SMEM);
+      err = cudaFuncSetAttribute(moe_prefill_kernel<FORM_SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SHORT_DYN_SMEM);
   }
   if (err == cudaSuccess && dev >= 0 && dev < 64) g_attr_set[dev] = true;
   return err;
@@ -2766,6 +2889,13 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
   } else {
     p.sh_parts = 1;
   }
+  if constexpr (SORTED_BUILD) {
+    // the positions take the place of the split form's intermediate
+    if (!short_batch && num_tokens >= kSortedTokens && workspace_bytes >= kSplitOffset + numel * sizeof(int32_t) &&
+        reinterpret_cast<uintptr_t>(workspace) % 16 == 0 &&
+        make_rows_map(&p.tm_rows, p.partial, static_cast<uint64_t>(numel + (sh != nullptr ? num_tokens : 0)) * NCH) == 0)
+      p.slot_pos = reinterpret_cast<int32_t*>(static_cast<uint8_t*>(workspace) + kSplitOffset);
+  }
   if (router_w != nullptr) {
     p.logits_out = logits_buf;
     rc = cached_map(&p.tm_x, 2, act_bf16, static_cast<uint64_t>(num_tokens), K_DIM, TILE_M);
@@ -2799,14 +2929,14 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
     static int clusters_fit = -1;   // every cluster has to be resident at once (grid barriers)
     if (clusters_fit < 0) {
       int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, moe_prefill_kernel<false>, &cfg) != cudaSuccess) n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, moe_prefill_kernel<FORM_WHOLE>, &cfg) != cudaSuccess) n = 0;
       clusters_fit = n;
     }
     if (clusters_fit < kGrid / 2) {
       fprintf(stderr, "only %d of %d two-CTA clusters can be resident\n", clusters_fit, kGrid / 2);
       return -107;
     }
-    err = cudaLaunchKernelEx(&cfg, moe_prefill_kernel<false>, p);
+    err = cudaLaunchKernelEx(&cfg, moe_prefill_kernel<FORM_WHOLE>, p);
     if (err != cudaSuccess) {
       fprintf(stderr, "kernel launch failed: %s\n", cudaGetErrorString(err));
       return static_cast<int>(err);
@@ -2814,9 +2944,12 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
     return 0;
   }
   if constexpr (SPLIT_BUILD) {
-    if (short_batch) moe_prefill_kernel<true><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
+    if (short_batch) moe_prefill_kernel<FORM_SHORT><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
   }
-  if (!short_batch) moe_prefill_kernel<false><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
+  if constexpr (SORTED_BUILD) {
+    if (p.slot_pos != nullptr) moe_prefill_kernel<FORM_SORTED><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
+  }
+  if (!short_batch && p.slot_pos == nullptr) moe_prefill_kernel<FORM_WHOLE><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
   err = cudaGetLastError();
   if (err != cudaSuccess) {
     fprintf(stderr, "kernel launch failed: %s\n", cudaGetErrorString(err));

@@ -92,6 +92,27 @@ __device__ __forceinline__ void tma_load_3d(const CUtensorMap* m, uint32_t x, ui
       : "memory");
 }
 
+// 3-D tiled store of a box from this CTA's shared memory; completion through the thread's bulk groups. Evict-first in L2,
+// as in st_global_256_stream.
+__device__ __forceinline__ void tma_store_3d_stream(const CUtensorMap* m, uint32_t x, uint32_t y, uint32_t z, uint32_t src_smem) {
+  asm volatile("{\n\t.reg .b64 pol;\n\t"
+               "createpolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
+               "cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group.L2::cache_hint [%0, {%1, %2, %3}], [%4], pol;\n\t}"
+               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(z), "r"(src_smem)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// At most N of this thread's latest bulk groups still read shared memory.
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+__device__ __forceinline__ void st_shared_128(uint32_t addr, const uint32_t (&w)[4]) {
+  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+}
+
 // ---------------------------------------------------------------- cp.async (16 B, L2 only)
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
