@@ -626,30 +626,42 @@ struct __align__(16) SharedState {
 };
 static_assert(sizeof(SharedState) <= SMEM_STATIC_RESERVE, "static shared state exceeds its reserve");
 
+// SiLU(g) * u of a pair of columns, in the reference's form u * g / (1 + exp(-g)) (kernel/qwen_tp/src/prefill_mono_final_nb.cu:678)
+// with both special functions in their flush-to-zero variants: what exp(-g) loses below 2^-126 does not change 1 + exp(-g), and
+// a quotient that small is 0 behind any scale of the requantisation. The variants that keep subnormals cost a range check
+// and two multiplications each: H=2048 I=512, launch of 4096 tokens 298 -> 290 us, 8192 454 -> 448, 16384 755 -> 748
+// (the same bits in all of them).
+// (tanh.approx needs one special-function operation instead of two, but its 2^-11 relative error moves enough e4m3 codes of the
+// intermediate to push about one output in 10^5 beyond 2e-2 rms.)
+__device__ __forceinline__ float2 silu_mul2(float2 g, float2 u) {
+  const float2 t = __fmul2_rn(g, make_float2(-1.44269504f, -1.44269504f));
+  const float2 d = __fadd2_rn(make_float2(ex2_approx_ftz(t.x), ex2_approx_ftz(t.y)), make_float2(1.f, 1.f));
+  return __fmul2_rn(__fmul2_rn(g, u), make_float2(rcp_approx_ftz(d.x), rcp_approx_ftz(d.y)));
+}
+
 // ------------------------------------------------------------------ pieces of the split form's epilogue
 // (The whole-unit loop has the same sections in line: with these functions called there the expert phase of the H = 7168
 // build took 3 % longer at 16384 tokens, its loop has no register to spare.)
-// SiLU(gate) * up as in the whole-unit loop (there the reason for this form of it), written over the gate columns; returns
+// SiLU(gate) * up, written over the gate columns; returns
 // the amax of this thread's columns.
 __device__ __forceinline__ float silu_mul(float2 (&acc)[TCOLS / 2]) {
   float mx = 0.f;
 #pragma unroll
   for (int i = 0; i < HCB / 2; ++i) {
-    const float2 g = acc[i], u = acc[HCB / 2 + i];
-    const float v0 = __fdividef(u.x * g.x, 1.0f + __expf(-g.x));
-    const float v1 = __fdividef(u.y * g.y, 1.0f + __expf(-g.y));
-    acc[i] = make_float2(v0, v1);
-    mx = fmaxf(mx, fmaxf(fabsf(v0), fabsf(v1)));
+    acc[i] = silu_mul2(acc[i], acc[HCB / 2 + i]);
+    mx = fmaxf(mx, fmaxf(fabsf(acc[i].x), fabsf(acc[i].y)));
   }
   return mx;
 }
 __device__ __forceinline__ uint4 pack_e4m3x16(const float2* a, float inv) {
-  uint4 qv;
-  qv.x = pack_e4m3x4(a[0].x * inv, a[0].y * inv, a[1].x * inv, a[1].y * inv);
-  qv.y = pack_e4m3x4(a[2].x * inv, a[2].y * inv, a[3].x * inv, a[3].y * inv);
-  qv.z = pack_e4m3x4(a[4].x * inv, a[4].y * inv, a[5].x * inv, a[5].y * inv);
-  qv.w = pack_e4m3x4(a[6].x * inv, a[6].y * inv, a[7].x * inv, a[7].y * inv);
-  return qv;
+  const float2 inv2 = make_float2(inv, inv);
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 x = __fmul2_rn(a[2 * i], inv2), y = __fmul2_rn(a[2 * i + 1], inv2);
+    w[i] = pack_e4m3x4(x.x, x.y, y.x, y.y);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
 }
 // The accumulators of a down pass times the routing weight, as bf16 into columns col0 .. of the partial row.
 __device__ __forceinline__ void store_rows(const Params& p, const float2 (&acc)[TCOLS / 2], int fi, float2 rw2, int chunk, int col0, bool ok) {
@@ -1976,20 +1988,15 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
               }
             }
           }
-          // SiLU(gate) * up (kernel/qwen_tp/src/prefill_mono_final_nb.cu:678), written over the gate columns
+          // SiLU(gate) * up, written over the gate columns
           float mx = 0.f;
 #pragma unroll
           for (int j = 0; j < ((MONO_ABLATE & 2) ? 0 : NSPLIT); ++j) {
 #pragma unroll
             for (int i = 0; i < HCB / 2; ++i) {
-              const float2 g = acc[j * (WC / 2) + i], u = acc[j * (WC / 2) + HCB / 2 + i];
-              // the reference's form (exp and division on the special-function unit). A tanh.approx form needs one
-              // special-function operation instead of two and is 15 us faster per layer, but its 2^-11 relative error
-              // moves enough e4m3 codes of the intermediate to push about one output in 10^5 beyond 2e-2 rms
-              const float v0 = __fdividef(u.x * g.x, 1.0f + __expf(-g.x));
-              const float v1 = __fdividef(u.y * g.y, 1.0f + __expf(-g.y));
-              acc[j * (WC / 2) + i] = make_float2(v0, v1);
-              mx = fmaxf(mx, fmaxf(fabsf(v0), fabsf(v1)));
+              const float2 v = silu_mul2(acc[j * (WC / 2) + i], acc[j * (WC / 2) + HCB / 2 + i]);
+              acc[j * (WC / 2) + i] = v;
+              mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
             }
           }
           // the row's amax over the pass's 128 columns: every warpgroup holds NSPLIT*HCB of them
@@ -2009,12 +2016,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
           for (int j = 0; j < ((MONO_ABLATE & 2) ? 0 : NSPLIT); ++j) {
 #pragma unroll
             for (int c = 0; c < HCB / 16; ++c) {
-              const float2* a = &acc[j * (WC / 2) + c * 8];
-              uint4 qv;
-              qv.x = pack_e4m3x4(a[0].x * inv, a[0].y * inv, a[1].x * inv, a[1].y * inv);
-              qv.y = pack_e4m3x4(a[2].x * inv, a[2].y * inv, a[3].x * inv, a[3].y * inv);
-              qv.z = pack_e4m3x4(a[4].x * inv, a[4].y * inv, a[5].x * inv, a[5].y * inv);
-              qv.w = pack_e4m3x4(a[6].x * inv, a[6].y * inv, a[7].x * inv, a[7].y * inv);
+              const uint4 qv = pack_e4m3x16(&acc[j * (WC / 2) + c * 8], inv);
               const int col0 = j * PASS_STRIDE + h * HCB + c * 16;  // column inside the pass's 128
               *reinterpret_cast<uint4*>(irow + sw128(r, col0 / 16)) = qv;
               if (p.dbg_inter != nullptr && fi >= 0 && !dead && ti.e != SHARED_E)

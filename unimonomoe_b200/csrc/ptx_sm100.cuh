@@ -282,6 +282,18 @@ __device__ __forceinline__ uint32_t cvt_bf16x2_satfinite(float lo, float hi) {
   return r;
 }
 
+// 2^x and 1/x of the special-function unit, subnormal operands and results flushed to zero.
+__device__ __forceinline__ float ex2_approx_ftz(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rcp_approx_ftz(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // 32-byte (256-bit) global store; the address must be 32-byte aligned.
 __device__ __forceinline__ void st_global_256(void* p, const uint32_t (&w)[8]) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
