@@ -1,5 +1,6 @@
 """Partial rows in sorted order (large batches) against slot order (the same launch with a workspace that has no room for the
-slots' positions): the outputs have to be the same bits, and the positions the inverse of the sort."""
+slots' positions): the outputs have to be the same bits, and the positions the inverse of the sort. And the units that are
+left behind the full rounds: split where every CTA gets one pass of the up projection at most."""
 import pytest
 import torch
 
@@ -15,6 +16,12 @@ CASES = [(("qwen_w1", synth.QWEN, 512, 256, False), T, skew, False) for T, skew 
 CASES += [(("qwen_w1", synth.QWEN, 512, 256, True), 4157, 0.5, True), (("qwen_tp2", synth.QWEN, 256, 256, False), 4111, 0.5, False),
           (("qwen_ep4", synth.QWEN, 512, 64, False), 11003, 1.0, False), (("ds_tp8", synth.DEEPSEEK, 256, 256, False), 4099, 0.5, False),
           (("ds_tp4", synth.DEEPSEEK, 512, 256, False), 4096, 1.0, False), (("ds_ep8", synth.DEEPSEEK, 2048, 32, True), 4133, 0.5, False)]
+# a few units left behind one round or several, the shared expert's among them, chunks, more than are split, none, less than one round
+CASES += [(("qwen_ep4", synth.QWEN, 512, 64, False), 8192, 0.5, False), (("qwen_ep4", synth.QWEN, 512, 64, False), 7500, 0.0, False),
+          (("qwen_ep8", synth.QWEN, 512, 32, True), 18000, 0.0, False), (("qwen_ep8", synth.QWEN, 512, 32, False), 6000, 0.0, False),
+          (("qwen_w1", synth.QWEN, 512, 256, False), 10000, 0.0, False), (("ds_tp8", synth.DEEPSEEK, 256, 256, False), 8192, 0.0, False),
+          (("ds_ep8", synth.DEEPSEEK, 2048, 32, False), 8000, 0.0, False)]
+PASSES = {"qwen_w1": 4, "qwen_ep4": 4, "qwen_ep8": 4, "ds_tp8": 2, "ds_tp4": 4, "ds_ep8": 4}   # of a unit's up projection, where units are long
 
 
 @pytest.mark.parametrize("build,T,skew,residual", CASES, ids=[f"{b[0]}{'-shared' if b[4] else ''}-{T}" for b, T, _, _ in CASES])
@@ -46,7 +53,7 @@ def test_sorted_rows_give_the_bits_of_slot_order(build, T, skew, residual):
         mk.prefill_impl(batch["hs"], batch["logits"], layer["w13"], layer["w13_scale"], layer["w2"], layer["w2_scale"], 8,
                         True, layer["bias"], out, scratch=sc, check=True, **kw)
         got.append((out.view(torch.int16), sc))
-    (a, sc), (b, _) = got
+    (a, sc), (b, flat) = got
     assert torch.equal(a, b)
     assert bool(torch.isfinite(a.view(torch.bfloat16).float()).all())
     pos = sc["workspace"][behind:behind + T * 32].view(torch.int32)
@@ -58,3 +65,11 @@ def test_sorted_rows_give_the_bits_of_slot_order(build, T, skew, residual):
     assert bool((pos[~here] == -1).all())
     assert torch.equal(sc["sorted_ids"][pos[here].long()], here.nonzero()[:, 0].int())
     assert int(pos.max()) == rows - 1
+    # units behind the full rounds: split or not
+    view, chunks = mk.workspace_view(sc["workspace"]), max(width // 512, 1)
+    units = view["total_tiles"] + (-(-(-(-T // 128)) // (256 // local)) * chunks if shared else 0)
+    left = units % 148 if units > 148 else 0
+    split = int(view["phase_ns"][6]) != 0
+    if units > 148:
+        assert split == (variant in PASSES and 0 < left <= 148 // PASSES[variant] // chunks * chunks)
+    assert int(mk.workspace_view(flat["workspace"])["phase_ns"][6]) == 0

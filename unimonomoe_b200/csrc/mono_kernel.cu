@@ -603,16 +603,21 @@ __device__ __forceinline__ size_t wsd_index(int e, int chunk, int i) {
 }
 
 // ------------------------------------------------------------------ shared state
+struct SplitBars {   // split form; its own, since the last arrivals of whole units before it may still be on their way
+  uint64_t fullA[SPLIT_SA], emptyA[SPLIT_SA], fullB[SPLIT_SB], emptyB[SPLIT_SB], tmem_full[NBUF], tmem_empty[NBUF];
+};
 struct __align__(16) SharedState {
   uint64_t fullA[A_STAGE_CAP], emptyA[A_STAGE_CAP], fullB[B_STAGE_CAP], emptyB[B_STAGE_CAP];
   uint64_t tmem_full[NBUF], tmem_empty[NBUF];
   uint64_t inter_ready[4];  // one per 128-column pass of the intermediate (NP <= 4)
   uint64_t rows_read;       // sorted partial rows: the copy engine has read the tile's rows out of the activation stages
   uint64_t rfull[4], rempty[4], racc_full, racc_empty;  // phase R only
+  SplitBars sp;
   uint32_t tmem_base;
   uint32_t flag;          // grid_sync result broadcast
   int n_my_tiles;
   int sp_units, sp_waves;        // split form: units, and waves of them through the intermediate (0: whole units)
+  int sp_slot0;                  // place of its first unit in the CTA's list (behind the whole units)
   uint32_t sp_flag, sp_gflag;    // split form: counter reached (epilogue, gather warps)
   TileInfo tiles[MAX_MY_TILES];
   int sp_row0[MAX_MY_TILES];     // split form: the tile's first row in the global intermediate
@@ -664,16 +669,16 @@ __device__ __forceinline__ uint4 pack_e4m3x16(const float2* a, float inv) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 // The accumulators of a down pass times the routing weight, as bf16 into columns col0 .. of the partial row.
-__device__ __forceinline__ void store_rows(const Params& p, const float2 (&acc)[TCOLS / 2], int fi, float2 rw2, int chunk, int col0, bool ok) {
+__device__ __forceinline__ void store_rows(const Params& p, const float2 (&acc)[TCOLS / 2], int row, float2 rw2, int col0, bool ok) {
   const int lane = threadIdx.x & 31;
   // Neighbouring lanes swap half of their 32-byte pieces first, so that in every store instruction
   // lanes 2i and 2i+1 write 64 contiguous bytes of ONE row: 16 lines per instruction instead of 32.
   // (the guard is made warp-uniform: the shuffles below need every lane of the warp)
   if (__all_sync(0xFFFFFFFFu, ok)) {
     const bool odd = (lane & 1) != 0;
-    const int fi_even = __shfl_sync(0xFFFFFFFFu, fi, lane & ~1), fi_odd = __shfl_sync(0xFFFFFFFFu, fi, lane | 1);
-    __nv_bfloat16* row_even = p.partial + (static_cast<size_t>(fi_even < 0 ? 0 : fi_even) * NCH + chunk) * H_DIM + col0;
-    __nv_bfloat16* row_odd = p.partial + (static_cast<size_t>(fi_odd < 0 ? 0 : fi_odd) * NCH + chunk) * H_DIM + col0;
+    const int row_e = __shfl_sync(0xFFFFFFFFu, row, lane & ~1), row_o = __shfl_sync(0xFFFFFFFFu, row, lane | 1);
+    __nv_bfloat16* row_even = p.partial + static_cast<size_t>(row_e < 0 ? 0 : row_e) * H_DIM + col0;
+    __nv_bfloat16* row_odd = p.partial + static_cast<size_t>(row_o < 0 ? 0 : row_o) * H_DIM + col0;
 #pragma unroll
     for (int k2 = 0; k2 < WC / 32; ++k2) {   // pieces 2*k2 and 2*k2+1 of this thread's WC columns
       uint32_t lo[8], hi[8], mine[8], theirs[8];
@@ -692,8 +697,8 @@ __device__ __forceinline__ void store_rows(const Params& p, const float2 (&acc)[
       }
       const int piece = 2 * k2 + (odd ? 1 : 0);
       // row of the even lane: its own piece from the even lane, the received one from the odd lane
-      if (fi_even >= 0) st_global_256_stream(row_even + piece * 16, odd ? theirs : mine);
-      if (fi_odd >= 0) st_global_256_stream(row_odd + piece * 16, odd ? mine : theirs);
+      if (row_e >= 0) st_global_256_stream(row_even + piece * 16, odd ? theirs : mine);
+      if (row_o >= 0) st_global_256_stream(row_odd + piece * 16, odd ? mine : theirs);
     }
   }
 }
@@ -743,6 +748,15 @@ constexpr int split_most(int round, bool one_wave, int percent) {
 }
 constexpr int SPLIT_MOST_1 = split_most(0, true, K_DIM > 4096 ? 76 : 70);
 constexpr int SPLIT_MOST_2 = split_most(1, true, K_DIM > 4096 ? 80 : 75), SPLIT_MOST_2W = split_most(1, false, K_DIM > 4096 ? 80 : 75);
+// Large batches: whole units in full rounds, and what is left behind them in the split form, where that is at most one pass of
+// the up projection per CTA and a unit is long enough to pay for the change of form (25 us: the CTAs meet, and the pipelines
+// start twice). Launch in us without -> with: H=2048 I=512: 765 units (25 left) 532 -> 505, 64 of 256 experts 169 units 203 ->
+// 184, 32 of 256 with 173 282 -> 258; two passes per CTA: 634 units (42 left) 436 -> 438, 501 (57 left) 338 -> 338. H=7168 I=256: 641
+// units (49 left) 997 -> 954, 756 (16 left) 1197 -> 1124. I=256 at H=2048, 48 slab steps a unit: 634 units (42 left) 287 -> 293.
+// (The weights of the left units into L2 beforehand: 184 -> 187, 338 -> 343.) Batches of less than one round have the bound of the short ones.
+constexpr bool REST_BUILD = SPLIT_BUILD && NP * NK + NHB * NP >= 96;
+constexpr int REST_MOST = kGrid / NP / NCH * NCH;
+constexpr int REST_ROWS = (REST_MOST > SPLIT_MOST_1 ? REST_MOST : SPLIT_MOST_1) / NCH * TILE_M;   // of the global intermediate
 constexpr bool LONG_UNITS = K_DIM > 4096 && NP > 2;
 constexpr int FEW_ROWS = 16;   // of a tile, on average
 __device__ __forceinline__ bool split_pays(int units, bool few_rows, bool one_wave) {
@@ -753,10 +767,12 @@ __device__ __forceinline__ bool split_pays(int units, bool few_rows, bool one_wa
 // Phase 2 in the split form, with the roles of the whole-unit form. Both halves are the same slab step (weights
 // through one ring, rows through the other). The weights of the down passes do not depend on the up passes, so the
 // TMA and the MMA warp run through the counter between the halves; the gather warps and the epilogue wait at it.
+// SORTED: the partial rows are in sorted order.
+template <bool SORTED>
 __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, const WaitCtx& wc, uint8_t* a_ring, uint8_t* b_ring,
                                             uint32_t tmem_base) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, bid = blockIdx.x;
-  const int units = S.sp_units, waves = S.sp_waves;
+  const int units = S.sp_units, waves = S.sp_waves, slot0 = S.sp_slot0;
   auto share = [&](int w) { return split_share(waves == 1 ? units : min(kGrid, units - w * kGrid), bid); };
   const int numel = p.num_tokens * TOP_K;
   Workspace* ws = p.ws;
@@ -770,31 +786,31 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
         uint32_t nb = 0;
         auto stage = [&]() -> uint8_t* {   // the next free stage, its bytes announced; null on abort
           const uint32_t st = nb % SPLIT_SB;
-          if (!mbar_wait(&S.emptyB[st], ((nb / SPLIT_SB) & 1u) ^ 1u, wc, kSiteEmptyB)) return nullptr;
-          mbar_arrive_expect_tx(&S.fullB[st], B_STAGE_BYTES);
+          if (!mbar_wait(&S.sp.emptyB[st], ((nb / SPLIT_SB) & 1u) ^ 1u, wc, kSiteEmptyB)) return nullptr;
+          mbar_arrive_expect_tx(&S.sp.fullB[st], B_STAGE_BYTES);
           return b_ring + st * B_STAGE_BYTES;
         };
         bool ok = true;
         for (int w = 0; w < waves && ok; ++w) {
           const SplitShare my = share(w);
           for (int u = my.a0; u < my.a1 && ok; ++u) {
-            const TileInfo ti = S.tiles[w + u / NP - my.lo];
+            const TileInfo ti = S.tiles[slot0 + w + u / NP - my.lo];
             const bool sh = ti.e == SHARED_E;
             for (int ks = 0; ks < NK; ++ks, ++nb) {
               uint8_t* dst = stage();
               if (dst == nullptr) { ok = false; break; }
               tma_load_3d(sh ? &p.tm_sh_up : &p.tm_up, ks * 128, ti.chunk * CHUNK_COLS + u % NP * 128, sh ? 0 : 2 * ti.e, dst,
-                          &S.fullB[nb % SPLIT_SB]);
+                          &S.sp.fullB[nb % SPLIT_SB]);
             }
           }
           for (int u = my.b0; u < my.b1 && ok; ++u) {
-            const TileInfo ti = S.tiles[w + u / NHB - my.lo];
+            const TileInfo ti = S.tiles[slot0 + w + u / NHB - my.lo];
             const bool sh = ti.e == SHARED_E;
             for (int dk = 0; dk < NP; ++dk, ++nb) {
               uint8_t* dst = stage();
               if (dst == nullptr) { ok = false; break; }
               tma_load_2d(sh ? &p.tm_sh_down : &p.tm_down, (ti.chunk * NP + dk) * 128, (sh ? 0 : ti.e) * H_DIM + u % NHB * 256,
-                          dst, &S.fullB[nb % SPLIT_SB]);
+                          dst, &S.sp.fullB[nb % SPLIT_SB]);
             }
           }
         }
@@ -807,9 +823,9 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
       }
       for (uint32_t n = 0; n < static_cast<uint32_t>(steps); ++n) {
         const uint32_t sb = n % SPLIT_SB, sa = n % SPLIT_SA, buf = n % NBUF;
-        if (!mbar_wait_warp(&S.fullB[sb], (n / SPLIT_SB) & 1u, wc, kSiteFullB) ||
-            !mbar_wait_warp(&S.fullA[sa], (n / SPLIT_SA) & 1u, wc, kSiteFullA) ||
-            !mbar_wait_warp(&S.tmem_empty[buf], ((n / NBUF) & 1u) ^ 1u, wc, kSiteTmemEmpty))
+        if (!mbar_wait_warp(&S.sp.fullB[sb], (n / SPLIT_SB) & 1u, wc, kSiteFullB) ||
+            !mbar_wait_warp(&S.sp.fullA[sa], (n / SPLIT_SA) & 1u, wc, kSiteFullA) ||
+            !mbar_wait_warp(&S.sp.tmem_empty[buf], ((n / NBUF) & 1u) ^ 1u, wc, kSiteTmemEmpty))
           break;
         // the gathered rows were written by cp.async (generic proxy); the tensor core reads them through the async proxy
         fence_proxy_async_smem();
@@ -819,9 +835,9 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
         if (elect_one_sync()) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) umma_f8(tmem_base + buf * BC, da + 2u * k, db + 2u * k, IDESC, k > 0 ? 1u : 0u);
-          umma_commit(&S.tmem_full[buf]);
-          umma_commit(&S.emptyA[sa]);
-          umma_commit(&S.emptyB[sb]);
+          umma_commit(&S.sp.tmem_full[buf]);
+          umma_commit(&S.sp.emptyA[sa]);
+          umma_commit(&S.sp.emptyB[sb]);
         }
         __syncwarp();
       }
@@ -837,7 +853,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
         const SplitShare my = share(w);
         int cur = -1;
         for (int u = my.a0; u < my.a1; ++u) {
-          const int slot = w + u / NP - my.lo;
+          const int slot = slot0 + w + u / NP - my.lo;
           if (slot != cur) {   // the passes of one unit follow one another: its tokens are looked up once
             cur = slot;
             ++fills;
@@ -860,7 +876,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
           }
           for (int ks = 0; ks < NK; ++ks) {
             const uint32_t sa = na % SPLIT_SA;
-            if (!dead && !mbar_wait(&S.emptyA[sa], ((na / SPLIT_SA) & 1u) ^ 1u, wc, kSiteEmptyA)) dead = true;
+            if (!dead && !mbar_wait(&S.sp.emptyA[sa], ((na / SPLIT_SA) & 1u) ^ 1u, wc, kSiteEmptyA)) dead = true;
             if (dead) continue;
             const uint8_t* g0 = p.act_fp8 + ks * 128 + gc * 16;
 #pragma unroll
@@ -871,7 +887,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
               for (int i = 0; i < 4; ++i)
                 if (tok[i] >= 0) cp_async16(dst0 + sa * A_STAGE_BYTES + (4 * i4 + i) * 1024, g0 + static_cast<size_t>(tok[i]) * K_DIM);
             }
-            cp_async_arrive_noinc(&S.fullA[sa]);
+            cp_async_arrive_noinc(&S.sp.fullA[sa]);
             ++na;
           }
         }
@@ -883,18 +899,18 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
         named_bar_sync(2, N_GATHER);
         if (S.sp_gflag == 0u) dead = true;
         for (int u = my.b0; u < my.b1; ++u) {
-          const TileInfo ti = S.tiles[w + u / NHB - my.lo];
-          const uint8_t* g0 = p.sp_inter + static_cast<size_t>(S.sp_row0[w + u / NHB - my.lo]) * N_HALF + ti.chunk * CHUNK_COLS + gc * 16;
+          const TileInfo ti = S.tiles[slot0 + w + u / NHB - my.lo];
+          const uint8_t* g0 = p.sp_inter + static_cast<size_t>(S.sp_row0[slot0 + w + u / NHB - my.lo]) * N_HALF + ti.chunk * CHUNK_COLS + gc * 16;
           for (int dk = 0; dk < NP; ++dk) {
             const uint32_t sa = na % SPLIT_SA;
-            if (!dead && !mbar_wait(&S.emptyA[sa], ((na / SPLIT_SA) & 1u) ^ 1u, wc, kSiteEmptyA)) dead = true;
+            if (!dead && !mbar_wait(&S.sp.emptyA[sa], ((na / SPLIT_SA) & 1u) ^ 1u, wc, kSiteEmptyA)) dead = true;
             if (dead) continue;
 #pragma unroll
             for (int i = 0; i < ROWS_PER_THREAD; ++i) {
               const int r = gr + 8 * i;
               if (r < ti.rows) cp_async16(dst0 + sa * A_STAGE_BYTES + i * 1024, g0 + static_cast<size_t>(r) * N_HALF + dk * 128);
             }
-            cp_async_arrive_noinc(&S.fullA[sa]);
+            cp_async_arrive_noinc(&S.sp.fullA[sa]);
             ++na;
           }
         }
@@ -914,7 +930,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
     bool dead = false;
     auto full = [&]() -> uint32_t {   // the next accumulator buffer, once it is full
       const uint32_t buf = nt % NBUF;
-      if (!dead && !mbar_wait(&S.tmem_full[buf], (nt / NBUF) & 1u, wc, kSiteTmemFull)) dead = true;
+      if (!dead && !mbar_wait(&S.sp.tmem_full[buf], (nt / NBUF) & 1u, wc, kSiteTmemFull)) dead = true;
       ++nt;
       dead = __any_sync(0xFFFFFFFFu, dead);
       return buf;
@@ -932,7 +948,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
         if (c == 1) {
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&S.tmem_empty[buf]);
+          if (lane == 0) mbar_arrive(&S.sp.tmem_empty[buf]);
         }
         const float sc = (c == 0) ? s_lo : s_hi;
 #pragma unroll
@@ -947,7 +963,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
 #pragma unroll 1
       for (int i = 0; i < n; ++i) {
         const uint32_t buf = full();
-        if (lane == 0 && !dead) mbar_arrive(&S.tmem_empty[buf]);
+        if (lane == 0 && !dead) mbar_arrive(&S.sp.tmem_empty[buf]);
       }
     };
     // index of this thread's partial row in tile ti (-1: no row) and its token
@@ -982,7 +998,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
       // ---------------- up projection + SiLU*mul + requantisation
       int cur = -1, fi = -1, tok = 0;
       for (int u = my.a0; u < my.a1; ++u) {
-        const int ps = u % NP, slot = w + u / NP - my.lo;
+        const int ps = u % NP, slot = slot0 + w + u / NP - my.lo;
         const TileInfo ti = S.tiles[slot];
         if (q * 32 >= ti.rows) { pass_on(NK); continue; }
         if (slot != cur) { cur = slot; take_row(ti, fi, tok); }
@@ -1036,7 +1052,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
       cur = -1;
       float rw = 0.f, isc[NP];
       for (int u = my.b0; u < my.b1; ++u) {
-        const int hb = u % NHB, slot = w + u / NHB - my.lo;
+        const int hb = u % NHB, slot = slot0 + w + u / NHB - my.lo;
         const TileInfo ti = S.tiles[slot];
         if (q * 32 >= ti.rows) { pass_on(NP); continue; }
         const bool sh = ti.e == SHARED_E;
@@ -1063,7 +1079,8 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
         for (int i = 0; i < TCOLS / 2; ++i) acc[i] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int dk = 0; dk < NP; ++dk) promote(acc, sc[dk], sc[dk], down_col);
-        store_rows(p, acc, fi, make_float2(rw, rw), ti.chunk, hb * 256 + h * WC, !dead);
+        const int prow = fi < 0 ? -1 : SORTED ? ti.chunk * (numel + (p.sh_on ? p.num_tokens : 0)) + (sh ? numel : 0) + ti.row0 + r : fi * NCH + ti.chunk;
+        store_rows(p, acc, prow, make_float2(rw, rw), hb * 256 + h * WC, !dead);
       }
       if (w + 1 < waves) meet(static_cast<uint32_t>((2 * w + 2) * kGrid));  // the intermediate may be overwritten
     }
@@ -1071,7 +1088,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
 }
 
 // ------------------------------------------------------------------ the kernel
-// FORM_SORTED: whole units with the partial rows in sorted order, an instance of its own because its store section changes
+// FORM_SORTED: whole units with the partial rows in sorted order (and the split form for those behind the full rounds), an instance of its own because its store section changes
 // the registers of the slab loop (the others take 2 to 5 % longer with both in one).
 // FORM_SHORT: the instance for batches that are expected to be short. It holds both forms of the expert phase and takes one of
 // them by the units that phase 1 counts. FORM_WHOLE computes whole units only, and computes them faster: inside
@@ -1090,6 +1107,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
 
   constexpr bool CAN_SPLIT = FORM == FORM_SHORT && SPLIT_BUILD;
   constexpr bool SORTED = FORM == FORM_SORTED && SORTED_BUILD;
+  constexpr bool REST = SORTED && REST_BUILD;   // what is left behind the full rounds of units can be split
   constexpr int RS = (SA < SB) ? SA : SB;  // stages of the router linear's ring
   // 1024-byte aligned base of the operand buffers
   const uint32_t dyn_u32 = (smem_u32(dyn_raw) + 1023u) & ~1023u;
@@ -1366,8 +1384,22 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       lo = mine.lo;
       hi = mine.hi;
     }
+    // Units behind the last full round of whole units, where they are worth splitting.
+    int rest0 = units, rest = 0;
+    if constexpr (REST) {
+      rest = units % kGrid;
+      if (rest > (units < kGrid ? SPLIT_MOST_1 : REST_MOST) || p.sp_rows < REST_ROWS) rest = 0;
+      rest0 = units - rest;
+      const SplitShare mine = split_share(rest, bid);
+      lo = mine.lo;
+      hi = mine.hi;
+    }
     // place of unit g in this CTA's list, or -1; whole units are dealt round-robin
     auto slot_of = [&](int g) -> int {
+      if (REST && g >= rest0) {
+        const int l = g - rest0;
+        return (l >= lo && l < hi) ? rest0 / kGrid + l - lo : -1;
+      }
       if (CAN_SPLIT && split) {
         if (!one_wave && g < kGrid) return g == bid ? 0 : -1;
         const int l = one_wave ? g : g - kGrid;
@@ -1375,7 +1407,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       }
       return (g % SCHED_UNITS == sched_me) ? g / SCHED_UNITS : -1;
     };
-    auto split_row = [&](int g, int sorted_row) -> int { return one_wave ? sorted_row : g % kGrid / NCH * TILE_M; };
+    auto split_row = [&](int g, int sorted_row) -> int { return one_wave && !REST ? sorted_row : g % kGrid / NCH * TILE_M; };
     if (tid < E) {
       const int off_e = scan_cnt[tid] - cnt;
       const int tbase = scan_tile[tid] - tiles_e;
@@ -1399,7 +1431,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             ti.rows = max(0, min(TILE_M, off_e + cnt - ti.row0));
             ti.chunk = i % NCH;
             S.tiles[slot] = ti;
-            if (CAN_SPLIT && split) S.sp_row0[slot] = split_row(g, ti.row0);
+            if ((CAN_SPLIT && split) || (REST && g >= rest0)) S.sp_row0[slot] = split_row(g, ti.row0);
           } else {
             report_error(ws, kErrBounds, 1, static_cast<uint32_t>(g), static_cast<uint32_t>(slot));
           }
@@ -1427,7 +1459,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             ti.rows = max(0, min(TILE_M, T - ti.row0));
             ti.chunk = i % NCH;
             S.tiles[slot] = ti;
-            if (CAN_SPLIT && split) S.sp_row0[slot] = split_row(g, rows_routed + i / NCH * TILE_M);
+            if ((CAN_SPLIT && split) || (REST && g >= rest0)) S.sp_row0[slot] = split_row(g, rows_routed + i / NCH * TILE_M);
           } else {
             report_error(ws, kErrBounds, 3, static_cast<uint32_t>(g), static_cast<uint32_t>(slot));
           }
@@ -1435,9 +1467,10 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       }
     }
     if (tid == 0) {
-      S.sp_units = units;
-      S.sp_waves = split ? (one_wave ? 1 : 2) : 0;
-      S.n_my_tiles = (units > sched_me) ? min(MAX_MY_TILES, (units - sched_me + SCHED_UNITS - 1) / SCHED_UNITS) : 0;
+      S.sp_units = REST ? rest : units;
+      S.sp_waves = split ? (one_wave ? 1 : 2) : rest > 0 ? 1 : 0;
+      S.sp_slot0 = rest > 0 ? rest0 / kGrid : 0;
+      S.n_my_tiles = (rest0 > sched_me) ? min(MAX_MY_TILES, (rest0 - sched_me + SCHED_UNITS - 1) / SCHED_UNITS) : 0;
     }
     // stable scatter: each warp re-walks its own tokens in ascending order
     for (int t = t_begin; t < t_end; ++t) {
@@ -1473,11 +1506,16 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   const bool split = CAN_SPLIT && alive && S.sp_waves != 0;
   if (tid == 0) {
     const uint32_t both = PAIR ? 2u : 1u;
-    for (int s = 0; s < (split ? SPLIT_SA : SA); ++s) {
+    for (int s = 0; s < SA; ++s) {
       mbar_init(&S.fullA[s], N_GATHER + ((PAIR && leader) ? 1u : 0u));
       mbar_init(&S.emptyA[s], 1);
     }
-    for (int s = 0; s < (split ? SPLIT_SB : SB); ++s) { mbar_init(&S.fullB[s], 1); mbar_init(&S.emptyB[s], 1); }
+    for (int s = 0; s < SB; ++s) { mbar_init(&S.fullB[s], 1); mbar_init(&S.emptyB[s], 1); }
+    if constexpr (CAN_SPLIT || REST) {
+      for (int s = 0; s < SPLIT_SA; ++s) { mbar_init(&S.sp.fullA[s], N_GATHER); mbar_init(&S.sp.emptyA[s], 1); }
+      for (int s = 0; s < SPLIT_SB; ++s) { mbar_init(&S.sp.fullB[s], 1); mbar_init(&S.sp.emptyB[s], 1); }
+      for (int s = 0; s < NBUF; ++s) { mbar_init(&S.sp.tmem_full[s], 1); mbar_init(&S.sp.tmem_empty[s], N_EPI / 32); }
+    }
     for (int s = 0; s < NBUF; ++s) { mbar_init(&S.tmem_full[s], 1); mbar_init(&S.tmem_empty[s], both * (N_EPI / 32)); }
 #ifdef MONO_PROFILE
     for (int i = 0; i < 48; ++i) (&S.whist[0][0])[i] = 0ull;
@@ -1507,7 +1545,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   const int n_my = alive ? S.n_my_tiles : 0;
 
   if (split) {
-    if constexpr (CAN_SPLIT) split_phase(p, S, wc, dyn, dyn + SPLIT_SA * A_STAGE_BYTES, tmem_base);
+    if constexpr (CAN_SPLIT) split_phase<false>(p, S, wc, dyn, dyn + SPLIT_SA * A_STAGE_BYTES, tmem_base);
   } else if (warp < 4) {
     reg_dec<REGS_PRODUCER>();
     if (warp == WARP_TMA) {
@@ -2158,6 +2196,22 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     }
   }
 
+  if constexpr (REST) {
+    // The units behind the full rounds, in the split form. Its rings take all of the shared memory: everything in it has been
+    // read (the epilogue has seen every MMA complete and waited for its boxes), and the fence orders the two proxies.
+    if (alive && S.sp_waves != 0) {
+      fence_proxy_async_smem();
+      tc_fence_before();
+      __syncthreads();
+      tc_fence_after();
+      // Back to the launch split, and behind another barrier: an epilogue warp that went on to its setmaxnreg.inc at once
+      // could take back what it had just released before the producers were served, who would then wait for ever.
+      if (warp < 4) reg_inc<REGS_LAUNCH>(); else reg_dec<REGS_LAUNCH>();
+      __syncthreads();
+      split_phase<true>(p, S, wc, dyn, dyn + SPLIT_SA * A_STAGE_BYTES, tmem_base);
+    }
+  }
+
   // teardown of phase 2: when aborting, give in-flight bulk copies and MMAs time to land
   if (aborted(ws)) __nanosleep(200000);
   tc_fence_before();
@@ -2591,7 +2645,7 @@ cudaError_t ensure_kernel_attribute(int dev) {
   cudaError_t err = cudaFuncSetAttribute(moe_prefill_kernel<FORM_WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM);
   if constexpr (SORTED_BUILD) {
     if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(moe_prefill_kernel<FORM_SORTED>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM);
+      err = cudaFuncSetAttribute(moe_prefill_kernel<FORM_SORTED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SHORT_DYN_SMEM);
   }
   if constexpr (SPLIT_BUILD) {
     if (err == cudaSuccess)
@@ -2834,11 +2888,22 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
     p.sh_parts = 1;
   }
   if constexpr (SORTED_BUILD) {
-    // the positions take the place of the split form's intermediate
-    if (!short_batch && num_tokens >= kSortedTokens && workspace_bytes >= kSplitOffset + numel * sizeof(int32_t) &&
-        reinterpret_cast<uintptr_t>(workspace) % 16 == 0 &&
-        make_rows_map(&p.tm_rows, p.partial, static_cast<uint64_t>(numel + (sh != nullptr ? num_tokens : 0)) * NCH) == 0)
+    // the positions take the place of the split form's intermediate, whose rows for the rest of the units come behind them
+    const size_t pos_bytes = (numel * sizeof(int32_t) + 255) / 256 * 256;
+    if (num_tokens >= kSortedTokens && workspace_bytes >= kSplitOffset + pos_bytes && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 &&
+        make_rows_map(&p.tm_rows, p.partial, static_cast<uint64_t>(numel + (sh != nullptr ? num_tokens : 0)) * NCH) == 0) {
+      short_batch = false;
       p.slot_pos = reinterpret_cast<int32_t*>(static_cast<uint8_t*>(workspace) + kSplitOffset);
+      p.sp_rows = 0;
+      if constexpr (REST_BUILD) {
+        if (workspace_bytes >= kSplitOffset + pos_bytes + REST_ROWS * SPLIT_ROW_BYTES && p.dbg_acc == nullptr && p.dbg_inter == nullptr &&
+            p.dbg_inter_scale == nullptr) {
+          p.sp_rows = REST_ROWS;
+          p.sp_inter = reinterpret_cast<uint8_t*>(p.slot_pos) + pos_bytes;
+          p.sp_scale = reinterpret_cast<float*>(p.sp_inter + static_cast<size_t>(REST_ROWS) * N_HALF);
+        }
+      }
+    }
   }
   if (router_w != nullptr) {
     p.logits_out = logits_buf;
@@ -2891,7 +2956,7 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
     if (short_batch) moe_prefill_kernel<FORM_SHORT><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
   }
   if constexpr (SORTED_BUILD) {
-    if (p.slot_pos != nullptr) moe_prefill_kernel<FORM_SORTED><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
+    if (p.slot_pos != nullptr) moe_prefill_kernel<FORM_SORTED><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
   }
   if (!short_batch && p.slot_pos == nullptr) moe_prefill_kernel<FORM_WHOLE><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
   err = cudaGetLastError();
