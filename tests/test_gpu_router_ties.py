@@ -1,4 +1,4 @@
-"""Routing where scores tie inside a lane's experts, between lanes and between groups, with zeros of both signs and masked experts,
+"""(Up to eight tokens every CTA routes and sorts the batch for itself.) Routing where scores tie inside a lane's experts, between lanes and between groups, with zeros of both signs and masked experts,
 and activation scales of tokens whose columns are zero, subnormal or huge: the same bits as the oracle, in every router mode."""
 import pytest
 import torch
@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("variant,spec,width,local,mode", [("qwen_ep8", synth.QWEN, 512, 32, 0), ("qwen_sig_w1", synth.QWEN, 512, 256, 1),
                                                            ("ds_tp8", synth.DEEPSEEK, 256, 256, 2)])
-@pytest.mark.parametrize("T", [1, 149, 300])
+@pytest.mark.parametrize("T", [1, 8, 9, 149, 300])
 def test_ties_and_extremes_are_exact(variant, spec, width, local, mode, T):
     from oracle import cpu_oracle as O
     from tests import gpu_util as gu

@@ -301,6 +301,10 @@ constexpr int kDirectTokens = 256;
 // sorted, H=2048 I=512: 2048 tokens 193 -> 198, 3000 215 -> 221, 4096 298 -> 298, 5000 371 -> 361; H=7168 I=256: 2500 503 -> 508,
 // 4096 614 -> 609, 6000 824 -> 813; 128 of 256 experts: 4096 tokens 197 -> 191.
 constexpr int kSortedTokens = 4096;
+// Largest batch that every CTA routes for itself. Launch in us, dealt over the CTAs -> by each: 1 token 35.2 -> 31.8, 4 39.0 -> 35.3,
+// 64 of 256 experts 9 35.6 -> 34.8, 12 tokens 74.1 -> 74.9 (a warp's token takes longer with all warps of the SM at it); H=7168
+// 1 token 61.6 -> 59.4, 8 90.4 -> 89.7. Not with the router linear inside: 5 tokens 57.7 -> 63.5.
+constexpr int kSoloTokens = 8;
 constexpr uint32_t kSplitCounter = 3;  // workspace counter between the halves of the split form (0-2: grid barriers)
 
 // wait sites reported in the status word
@@ -1140,7 +1144,11 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   // Every warp routes a contiguous range of tokens, so a CTA routes one contiguous range as well.
   // The ranges differ by one token at most: a few tokens to every SM finish before many to some
   // (routing and quantisation of 200 tokens 5.8 -> 5.2 us, of 777 at H = 7168 16.2 -> 14.5).
-  const int cta_t0 = static_cast<int>(static_cast<long long>(bid) * T / kGrid), cta_t1 = static_cast<int>(static_cast<long long>(bid + 1) * T / kGrid);
+  // A batch of a few tokens is routed and sorted by every CTA for itself: all of them write the same bytes, each reads what it
+  // wrote, and the two grid barriers in front of the expert phase are not needed.
+  const bool solo = !PAIR && T <= kSoloTokens && p.logits_out == nullptr;
+  const int cta_t0 = solo ? 0 : static_cast<int>(static_cast<long long>(bid) * T / kGrid);
+  const int cta_t1 = solo ? T : static_cast<int>(static_cast<long long>(bid + 1) * T / kGrid);
   const int t_begin = cta_t0 + warp * (cta_t1 - cta_t0) / NWARPS, t_end = cta_t0 + (warp + 1) * (cta_t1 - cta_t0) / NWARPS;
 
   // ================================================================ phase R (router GEMV)
@@ -1313,7 +1321,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     ws->cta_hist[bid][tid] = c;
   }
 
-  bool alive = grid_sync(wc, 0, &S.flag);
+  bool alive = solo || grid_sync(wc, 0, &S.flag);
   if (bid == 0 && tid == 0) ws->phase_ns[1] = globaltimer_ns();
 
   // ================================================================ phase 1
@@ -1324,7 +1332,14 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   if (alive) {
     if (tid < E) { ph1_tot[tid] = 0; ph1_pre[tid] = 0; }
     __syncthreads();
-    if (direct) {
+    if (solo) {
+      if (tid < E) {
+        int c = 0;
+#pragma unroll
+        for (int w = 0; w < NWARPS; ++w) c += hist[w * E + tid];
+        ph1_tot[tid] = c;
+      }
+    } else if (direct) {
       const int before = cta_t0 * TOP_K;  // slots of lower CTAs
 #pragma unroll 4
       for (int i = tid; i < numel; i += BLOCK) {
@@ -1488,7 +1503,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     }
   }
 
-  alive = grid_sync(wc, 1, &S.flag) && alive;
+  if (solo) __syncthreads();
+  else alive = grid_sync(wc, 1, &S.flag) && alive;
   if (bid == 0 && tid == 0) {
     ws->phase_ns[2] = globaltimer_ns();
     ws->phase_ns[6] = 0;   // written again by a launch that takes the split form
