@@ -216,6 +216,11 @@ constexpr bool PROFILE_BUILD = true;
 constexpr bool PROFILE_BUILD = false;
 #endif
 constexpr bool SPLIT_BUILD = ONE_BOX && NP > 1 && MONO_ABLATE == 0 && !PROFILE_BUILD;
+// With one pass of the up projection per unit there is nothing to deal in two halves. There a unit that is left behind the full
+// rounds (or one of a batch of few units) is given to several CTAs: each computes its up projection and a part of the output
+// columns. Launch in us, one CTA per unit -> several: 8192 tokens (634 units, 42 left) 225 -> 216, 5000 (444 or so) 166 -> 159,
+// 32 tokens 59.9 -> 54.4, 9 37.2 -> 34.3, 1 31.4 -> 28.6.
+constexpr bool SHARE_BUILD = ONE_BOX && NP == 1 && MONO_ABLATE == 0 && !PROFILE_BUILD;
 constexpr size_t SPLIT_ROW_BYTES = N_HALF + NPT * sizeof(float);  // e4m3 intermediate and its scales, one row
 constexpr int SPLIT_ROWS = SPLIT_BUILD ? kGrid / NCH * TILE_M : 0;  // rows of the global intermediate: kGrid full units
 static_assert(kGrid % NCH == 0, "a wave of kGrid units holds whole tiles");
@@ -621,6 +626,7 @@ struct __align__(16) SharedState {
   uint32_t flag;          // grid_sync result broadcast
   int n_my_tiles;
   int sp_units, sp_waves;        // split form: units, and waves of them through the intermediate (0: whole units)
+  int down[SHARE_BUILD ? MAX_MY_TILES : 1];   // passes of the down projection of each unit in the list: from | to << 16
   int sp_slot0;                  // place of its first unit in the CTA's list (behind the whole units)
   uint32_t sp_flag, sp_gflag;    // split form: counter reached (epilogue, gather warps)
   TileInfo tiles[MAX_MY_TILES];
@@ -1111,6 +1117,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
 
   constexpr bool CAN_SPLIT = FORM == FORM_SHORT && SPLIT_BUILD;
   constexpr bool SORTED = FORM == FORM_SORTED && SORTED_BUILD;
+  constexpr bool SHARE = FORM == FORM_WHOLE && SHARE_BUILD;   // units behind the full rounds are shared by several CTAs
   constexpr bool REST = SORTED && REST_BUILD;   // what is left behind the full rounds of units can be split
   constexpr int RS = (SA < SB) ? SA : SB;  // stages of the router linear's ring
   // 1024-byte aligned base of the operand buffers
@@ -1409,8 +1416,16 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       lo = mine.lo;
       hi = mine.hi;
     }
+    int sharers = 1;   // CTAs of a unit behind the last full round
+    if constexpr (SHARE) {
+      rest = units % kGrid;
+      if (2 * rest > kGrid) rest = 0;
+      rest0 = units - rest;
+      if (rest > 0) sharers = min(NHB, kGrid / rest);
+    }
     // place of unit g in this CTA's list, or -1; whole units are dealt round-robin
     auto slot_of = [&](int g) -> int {
+      if (SHARE && g >= rest0) return bid / sharers == g - rest0 ? rest0 / kGrid : -1;
       if (REST && g >= rest0) {
         const int l = g - rest0;
         return (l >= lo && l < hi) ? rest0 / kGrid + l - lo : -1;
@@ -1483,9 +1498,14 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     }
     if (tid == 0) {
       S.sp_units = REST ? rest : units;
-      S.sp_waves = split ? (one_wave ? 1 : 2) : rest > 0 ? 1 : 0;
+      S.sp_waves = split ? (one_wave ? 1 : 2) : REST && rest > 0 ? 1 : 0;
       S.sp_slot0 = rest > 0 ? rest0 / kGrid : 0;
       S.n_my_tiles = (rest0 > sched_me) ? min(MAX_MY_TILES, (rest0 - sched_me + SCHED_UNITS - 1) / SCHED_UNITS) : 0;
+      if (SHARE && bid < rest * sharers) S.n_my_tiles = min(MAX_MY_TILES, rest0 / kGrid + 1);
+    }
+    if (SHARE && tid < MAX_MY_TILES) {
+      const int part = bid % sharers;
+      S.down[tid] = rest > 0 && tid == rest0 / kGrid ? part * NHB / sharers | (part + 1) * NHB / sharers << 16 : NHB << 16;
     }
     // stable scatter: each warp re-walks its own tokens in ascending order
     for (int t = t_begin; t < t_end; ++t) {
@@ -1620,7 +1640,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
               ++nb;
             }
           }
-          for (int hb = 0; hb < NHB && ok; ++hb) {
+          const int hb_end = SHARE ? S.down[it] >> 16 : NHB;
+          for (int hb = SHARE ? S.down[it] & 0xFFFF : 0; hb < hb_end && ok; ++hb) {
             const uint32_t y = static_cast<uint32_t>(e * H_DIM + hb * 256);
             for (int dk = 0; dk < NP; ++dk) {
               const uint32_t st = nb % SB, ph = (nb / SB) & 1u;
@@ -1734,7 +1755,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             TRACE_M(4);
           }
           if (!ok) break;
-          for (int s = 0; s < NHB * NP; ++s) {
+          const int down_steps = SHARE ? ((S.down[it] >> 16) - (S.down[it] & 0xFFFF)) * NP : NHB * NP;
+          for (int s = 0; s < down_steps; ++s) {
             const int dk = s % NP;
             const uint32_t sb = nb % SB;
             if (s < NP) {
@@ -2089,8 +2111,10 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
         // ---------------- down projection, routing weight, bf16 partial rows.
         // Every epilogue thread is past the last pass's barrier, so nobody reads this tile's
         // activation scales any more: the next tile's are staged while the down slabs run.
+        // (A unit with a part of the passes is the last of its CTA: nothing is staged behind it.)
         if (has_next) stage_ids(it + 1);
-        for (int hb = 0; hb < NHB; ++hb) {
+        const int hb_end = SHARE ? S.down[it] >> 16 : NHB;
+        for (int hb = SHARE ? S.down[it] & 0xFFFF : 0; hb < hb_end; ++hb) {
 #pragma unroll
           for (int i = 0; i < TCOLS / 2; ++i) acc[i] = make_float2(0.f, 0.f);
           if (has_next) {
