@@ -2666,8 +2666,8 @@ int cached_map(CUtensorMap* dst, int kind, const void* base, uint64_t rows, uint
 // Whether a batch gets the instance that can compute the split form, from its size alone (the units are only known on the
 // device, which then chooses between the forms). Units are estimated for even routing: the experts that T tokens reach,
 // half a tile of padding once experts fill more than one. Where fewer units come out, the device stays with whole units:
-// 32 tokens of uneven routing with 124 units take 91 us (105 in the split form, 87 in the instance without it), 64 of 256
-// experts at 7500 tokens with 135 units 157 (182, 153).
+// 32 tokens of uneven routing with 124 units take 91 us (105 in the split form, 87 in the instance without it). Batches whose
+// partial rows are in sorted order have an instance of their own.
 bool short_expected(int num_tokens, int sh_units) {
   const double rows = static_cast<double>(num_tokens) * TOP_K / E;  // of an expert
   const double reached = 1.0 - pow(1.0 - static_cast<double>(TOP_K) / E, num_tokens);
