@@ -3,7 +3,8 @@
 // exp() is written out as a fixed sequence of IEEE fp32 operations (one multiply,
 // round-to-nearest-even, two fused multiply-adds for the range reduction, a degree-5
 // Horner polynomial in fused multiply-adds, one add, one multiply by an exact power of
-// two), so any implementation that performs the same sequence in IEEE fp32 reproduces
+// two; the method, the polynomial and the two parts of ln 2 are those of the Cephes
+// library by S. L. Moshier), so any implementation that performs the same sequence in IEEE fp32 reproduces
 // it exactly. The sigmoid router (modes 1 and 2) selects experts by comparing
 // sigmoid(logit) + bias; with a library expf the last-ulp differences between two
 // libraries flip selections at near-ties (the reference documents one such flip per
