@@ -4,7 +4,7 @@ left behind the full rounds: split where every CTA gets one pass of the up proje
 import pytest
 import torch
 
-from unimonomoe_b200 import MonoKernel, synth, variant_path
+from unimonomoe_b200 import MonoKernel, loader, synth, variant_path
 from unimonomoe_b200.loader import prepare_shared_expert
 
 pytestmark = pytest.mark.gpu
@@ -21,12 +21,16 @@ CASES += [(("qwen_ep4", synth.QWEN, 512, 64, False), 8192, 0.5, False), (("qwen_
           (("qwen_ep8", synth.QWEN, 512, 32, True), 18000, 0.0, False), (("qwen_ep8", synth.QWEN, 512, 32, False), 6000, 0.0, False),
           (("qwen_w1", synth.QWEN, 512, 256, False), 10000, 0.0, False), (("ds_tp8", synth.DEEPSEEK, 256, 256, False), 8192, 0.0, False),
           (("ds_ep8", synth.DEEPSEEK, 2048, 32, False), 8000, 0.0, False)]
+# the most tokens that the C entries take (the Python entries have a cap of their own): 31 full rounds, and no room in the
+# CTAs' lists for a part of the units behind them
+CASES += [(("qwen_w1", synth.QWEN, 512, 256, False), 71680, 0.0, False)]
 PASSES = {"qwen_w1": 4, "qwen_ep4": 4, "qwen_ep8": 4, "ds_tp8": 2, "ds_tp4": 4, "ds_ep8": 4}   # of a unit's up projection, where units are long
 
 
 @pytest.mark.parametrize("build,T,skew,residual", CASES, ids=[f"{b[0]}{'-shared' if b[4] else ''}-{T}" for b, T, _, _ in CASES])
-def test_sorted_rows_give_the_bits_of_slot_order(build, T, skew, residual):
+def test_sorted_rows_give_the_bits_of_slot_order(build, T, skew, residual, monkeypatch):
     variant, spec, width, local, shared = build
+    monkeypatch.setattr(loader, "MOE_MONOKERNEL_PREFILL_MAX_TOKENS", max(T, loader.MOE_MONOKERNEL_PREFILL_MAX_TOKENS))
     mk = MonoKernel(variant_path(variant))
     layer = synth.make_layer(spec, seed=5, device=DEV, inter_slice=(0, width) if width != spec.inter else None,
                              expert_slice=(0, local) if local != 256 else None, with_shared=shared)
@@ -71,5 +75,6 @@ def test_sorted_rows_give_the_bits_of_slot_order(build, T, skew, residual):
     left = units % 148 if units > 148 else 0
     split = int(view["phase_ns"][6]) != 0
     if units > 148:
-        assert split == (variant in PASSES and 0 < left <= 148 // PASSES[variant] // chunks * chunks)
+        room = units // 148 + 2 <= mk._int_symbol("max_tiles") // 148
+        assert split == (variant in PASSES and 0 < left <= 148 // PASSES[variant] // chunks * chunks and room)
     assert int(mk.workspace_view(flat["workspace"])["phase_ns"][6]) == 0

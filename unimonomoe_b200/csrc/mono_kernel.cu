@@ -722,8 +722,8 @@ __device__ __forceinline__ void store_rows(const Params& p, const float2 (&acc)[
 struct SplitShare {
   int lo, hi, a0, a1, b0, b1;
 };
-__device__ __forceinline__ SplitShare split_share(int n, int bid) {
-  SplitShare s;
+__host__ __device__ constexpr SplitShare split_share(int n, int bid) {
+  SplitShare s{};
   s.lo = bid * n / kGrid;
   s.hi = ((bid + 1) * n + kGrid - 1) / kGrid;
   s.a0 = bid * (n * NP) / kGrid;
@@ -767,6 +767,23 @@ constexpr int SPLIT_MOST_2 = split_most(1, true, K_DIM > 4096 ? 80 : 75), SPLIT_
 constexpr bool REST_BUILD = SPLIT_BUILD && NP * NK + NHB * NP >= 96;
 constexpr int REST_MOST = kGrid / NP / NCH * NCH;
 constexpr int REST_ROWS = (REST_MOST > SPLIT_MOST_1 ? REST_MOST : SPLIT_MOST_1) / NCH * TILE_M;   // of the global intermediate
+// How many of a batch's units that is. A CTA's share of them can touch two units, which stand in its list behind the whole
+// ones: where the list has no two places left, all units stay whole.
+static_assert(!REST_BUILD || (REST_MOST < kGrid && SPLIT_MOST_1 < kGrid), "a share of less than a round touches two units at most");
+__host__ __device__ constexpr int rest_units(int units) {
+  const int rest = units % kGrid;
+  return rest > (units < kGrid ? SPLIT_MOST_1 : REST_MOST) || units / kGrid + 2 > MAX_MY_TILES ? 0 : rest;
+}
+// Places that the longest list of a CTA takes up in a large batch: its whole units, and its share of those that are split.
+constexpr int list_places(int units) {
+  const int rest = REST_BUILD ? rest_units(units) : 0, whole = units - rest;
+  int most = (whole + kGrid - 1) / kGrid;
+  for (int cta = 0; cta < kGrid; ++cta) {
+    const SplitShare s = split_share(rest, cta);
+    if (s.hi > s.lo && whole / kGrid + s.hi - s.lo > most) most = whole / kGrid + s.hi - s.lo;
+  }
+  return most;
+}
 constexpr bool LONG_UNITS = K_DIM > 4096 && NP > 2;
 constexpr int FEW_ROWS = 16;   // of a tile, on average
 __device__ __forceinline__ bool split_pays(int units, bool few_rows, bool one_wave) {
@@ -1409,8 +1426,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     // Units behind the last full round of whole units, where they are worth splitting.
     int rest0 = units, rest = 0;
     if constexpr (REST) {
-      rest = units % kGrid;
-      if (rest > (units < kGrid ? SPLIT_MOST_1 : REST_MOST) || p.sp_rows < REST_ROWS) rest = 0;
+      rest = p.sp_rows < REST_ROWS ? 0 : rest_units(units);
       rest0 = units - rest;
       const SplitShare mine = split_share(rest, bid);
       lo = mine.lo;
@@ -2743,6 +2759,8 @@ int prefill_wgmma_cta_pair() { return PAIR ? 1 : 0; }
 // allocation is large enough, beyond that the caller sizes it from this accessor.
 int prefill_wgmma_partial_chunks() { return NCH; }
 int prefill_wgmma_block_threads() { return BLOCK; }
+// Places of the longest per-CTA unit list of a large batch of `units` units; a list has max_tiles / grid_size of them.
+int prefill_wgmma_list_places(int units) { return list_places(units); }
 int prefill_wgmma_stable_sort() { return 1; }
 // Byte offset of the 32-bit status word inside the workspace and the bytes that follow it
 // (status, abort flag, two detail words). 0 after a successful launch.
