@@ -1314,6 +1314,15 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       p.topk_weights[t * TOP_K + lane] = my_w;
       if (lid >= 0) hist[warp * E + lid] += 1;  // ids of one token are distinct: no conflict
     }
+    if constexpr (!SORTED && !EP_BUILD) {
+      // A slot without an expert (a token with fewer than eight selectable ones) has no row; the slot sum takes all eight of a
+      // token here, so it finds zeros. (With positions, or experts on other ranks, it looks for itself.)
+      for (uint32_t none = __ballot_sync(0xFFFFFFFFu, lane < TOP_K && my_id < 0); none != 0u; none &= none - 1u) {
+        uint4* row = reinterpret_cast<uint4*>(p.partial + static_cast<size_t>(t * TOP_K + __ffs(none) - 1) * NCH * H_DIM);
+#pragma unroll 1
+        for (int i = lane; i < NCH * H_DIM / 8; i += 32) row[i] = make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
     __syncwarp();  // the next token's increments may hit the same counters from other lanes
     float gdot = 0.f;
     auto quantise = [&](auto gate) {
