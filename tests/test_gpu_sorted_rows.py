@@ -4,7 +4,7 @@ left behind the full rounds: split where every CTA gets one pass of the up proje
 import pytest
 import torch
 
-from unimonomoe_b200 import MonoKernel, loader, synth, variant_path
+from unimonomoe_b200 import MonoKernel, build as kbuild, loader, synth, variant_path
 from unimonomoe_b200.loader import prepare_shared_expert
 
 pytestmark = pytest.mark.gpu
@@ -78,3 +78,21 @@ def test_sorted_rows_give_the_bits_of_slot_order(build, T, skew, residual, monke
         room = units // 148 + 2 <= mk._int_symbol("max_tiles") // 148
         assert split == (variant in PASSES and 0 < left <= 148 // PASSES[variant] // chunks * chunks and room)
     assert int(mk.workspace_view(flat["workspace"])["phase_ns"][6]) == 0
+
+
+def test_the_build_without_row_stores_measures_the_sorted_form():
+    """The development build that leaves the row stores out: large batches run the sorted form there as well (the positions
+    are written), and none of its row stores."""
+    mk, T = MonoKernel(kbuild.build_variant("qwen_w1_abl4")), 4096
+    layer = synth.make_layer(synth.QWEN, seed=5, device=DEV, with_shared=False)
+    batch = synth.make_batch(synth.QWEN, layer, T, seed=T, device=DEV)
+    sc = mk._allocate_scratch(T, DEV)
+    behind = -(-mk._int_symbol("workspace_min_bytes") // 256) * 256
+    sc["partial"].fill_(float("nan"))
+    sc["workspace"][behind:].fill_(0xEE)
+    out = torch.empty(T, 2048, dtype=torch.bfloat16, device=DEV)
+    mk.prefill_impl(batch["hs"], batch["logits"], layer["w13"], layer["w13_scale"], layer["w2"], layer["w2_scale"], 8, True, None,
+                    out, scratch=sc, check=True)
+    pos = sc["workspace"][behind:behind + T * 32].view(torch.int32)
+    assert torch.equal(torch.sort(pos).values, torch.arange(T * 8, dtype=torch.int32, device=DEV))
+    assert bool(sc["partial"].isnan().all())

@@ -71,7 +71,8 @@
 // results are then wrong) so that its share of the run time can be measured by difference.
 //   1: no TMEM read-out / promotion   2: no SiLU / requantisation arithmetic   4: no partial-row stores
 //   8: no activation gather copies    16: no weight TMA loads
-//   256: no lane exchange before the partial-row stores (same bytes, wrong columns)
+//   256: no lane exchange before the partial-row stores (same bytes, wrong columns; of rows in sorted order, those that a warp
+//   stores itself)
 //   128: every slab step issues its four MMAs twice (1024 tensor-core cycles per step: is a step bound by latency or by issue?)
 //   64: no operand hand-shake at all (producers idle; the MMA warp waits only for accumulator buffers)
 //   32: the intermediate's passes alias one 16 KB slot, which leaves room for four-deep operand rings
@@ -209,7 +210,8 @@ constexpr int MAX_TILES = MAX_MY_TILES * kGrid;
 // counter, every (unit, 256-column pass of the down projection). The intermediate leaves shared memory, and the weight
 // ring takes its place. The operations on a row and their order are those of the whole unit: the same bits come out.
 // (With one pass of the up projection per unit there is too little to cut: no number of units makes it pay.)
-// Profiling and ablation builds compute whole units: the stall counters and the switches are in that loop only.
+// Profiling and ablation builds compute whole units (of large batches with sorted rows too): the stall counters and the
+// switches are in that loop only.
 #ifdef MONO_PROFILE
 constexpr bool PROFILE_BUILD = true;
 #else
@@ -2208,7 +2210,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             // The last passes leave the activation stages to the gather warps, which refill them: the last one goes through
             // the intermediate, which nothing reads any more, or where that is too small the last two are stored directly.
             constexpr int RING_PASSES = LAST_IN_INTER ? NHB - 1 : NHB - 2;
-            const bool staged = box_full && alive_w && (hb < RING_PASSES || LAST_IN_INTER);
+            const bool staged = box_full && alive_w && (hb < RING_PASSES || LAST_IN_INTER) && (MONO_ABLATE & 4) == 0;
             const uint32_t slot = hb < RING_PASSES ? ring_slot : inter_slot;
             if (lane == 0) {
               bulk_wait_read<0>();   // the previous pass's box has left its slot
@@ -2236,7 +2238,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
                 tma_store_3d_stream(&p.tm_rows, 0, static_cast<uint32_t>(tile_row + q * 32), static_cast<uint32_t>((hb * 256 + h * WC) / ROW_BOX), slot);
                 bulk_commit();
               }
-            } else if (alive_w) {
+            } else if (alive_w && (MONO_ABLATE & 4) == 0) {
               store_direct(std::integral_constant<int, 0>(), prow, 1, 0);
             }
           } else if (alive_w && (MONO_ABLATE & 4) == 0) {
@@ -2727,10 +2729,14 @@ using namespace mono;
 
 extern "C" {
 
-// What every launch needs (sizeof(Workspace)) and, behind it, the intermediate rows of the split form. A workspace that
-// holds only the needed part is accepted: its launches compute whole units.
+// What every launch needs (sizeof(Workspace)) and, behind it, the intermediate rows of the split form, or the slots' positions
+// in a large batch. A workspace that holds only the needed part is accepted: its launches compute whole units, with their
+// partial rows in the slots' order.
 constexpr size_t kSplitOffset = (sizeof(Workspace) + 255) / 256 * 256;
-size_t prefill_wgmma_workspace_bytes() { return kSplitOffset + SPLIT_ROWS * SPLIT_ROW_BYTES; }
+// (Profiling and ablation builds have no split form, but the sorted rows of large batches: room for the positions alone.)
+constexpr size_t POS_BYTES = SORTED_BUILD ? size_t{MAX_TILES} / NCH * TILE_M * sizeof(int32_t) : 0;
+constexpr size_t BEHIND_BYTES = SPLIT_ROWS * SPLIT_ROW_BYTES > POS_BYTES ? SPLIT_ROWS * SPLIT_ROW_BYTES : POS_BYTES;
+size_t prefill_wgmma_workspace_bytes() { return kSplitOffset + BEHIND_BYTES; }
 size_t prefill_wgmma_workspace_min_bytes() { return sizeof(Workspace); }
 int prefill_wgmma_num_experts() { return E; }
 int prefill_wgmma_num_experts_local() { return E_LOCAL; }
