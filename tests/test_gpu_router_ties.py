@@ -1,5 +1,6 @@
-"""(Up to eight tokens every CTA routes and sorts the batch for itself.) Routing where scores tie inside a lane's experts, between lanes and between groups, with zeros of both signs and masked experts,
-and activation scales of tokens whose columns are zero, subnormal or huge: the same bits as the oracle, in every router mode."""
+"""Routing where scores tie inside a lane's experts, between lanes and between groups, with zeros of both signs and masked
+experts, and activation scales of tokens whose columns are zero, subnormal or huge: the same bits as the oracle, in every router
+mode, on both sides of eight tokens (up to which every CTA routes and sorts the whole batch for itself)."""
 import pytest
 import torch
 

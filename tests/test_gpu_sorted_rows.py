@@ -1,6 +1,7 @@
 """Partial rows in sorted order (large batches) against slot order (the same launch with a workspace that has no room for the
 slots' positions): the outputs have to be the same bits, and the positions the inverse of the sort. And the units that are
-left behind the full rounds: split where every CTA gets one pass of the up projection at most."""
+left behind the full rounds: split where every CTA gets one pass of the up projection at most, a batch of less than one round
+where the busiest CTA's steps are few enough, and neither where the workspace holds the positions alone."""
 import pytest
 import torch
 
@@ -9,26 +10,30 @@ from unimonomoe_b200.loader import prepare_shared_expert
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
-# (binary, layer, intermediate columns, local experts, shared expert), tokens, skew, residual: the smallest batch that has
-# sorted rows and the largest that has not, ragged tiles, ranks that own a part of the experts, three and four blocks a box,
-# intermediates too small for the last pass's box, units in chunks, the shared expert's rows behind the routed ones
-CASES = [(("qwen_w1", synth.QWEN, 512, 256, False), T, skew, False) for T, skew in ((4095, 0.0), (4096, 0.0), (5003, 1.0))]
-CASES += [(("qwen_w1", synth.QWEN, 512, 256, True), 4157, 0.5, True), (("qwen_tp2", synth.QWEN, 256, 256, False), 4111, 0.5, False),
-          (("qwen_ep4", synth.QWEN, 512, 64, False), 11003, 1.0, False), (("ds_tp8", synth.DEEPSEEK, 256, 256, False), 4099, 0.5, False),
-          (("ds_tp4", synth.DEEPSEEK, 512, 256, False), 4096, 1.0, False), (("ds_ep8", synth.DEEPSEEK, 2048, 32, True), 4133, 0.5, False)]
-# a few units left behind one round or several, the shared expert's among them, chunks, more than are split, none, less than one round
-CASES += [(("qwen_ep4", synth.QWEN, 512, 64, False), 8192, 0.5, False), (("qwen_ep4", synth.QWEN, 512, 64, False), 7500, 0.0, False),
-          (("qwen_ep8", synth.QWEN, 512, 32, True), 18000, 0.0, False), (("qwen_ep8", synth.QWEN, 512, 32, False), 6000, 0.0, False),
-          (("qwen_w1", synth.QWEN, 512, 256, False), 10000, 0.0, False), (("ds_tp8", synth.DEEPSEEK, 256, 256, False), 8192, 0.0, False),
-          (("ds_ep8", synth.DEEPSEEK, 2048, 32, False), 8000, 0.0, False)]
+# (binary, layer, intermediate columns, local experts, shared expert), tokens, skew, residual, units behind the full rounds
+# split?: the smallest batch that has sorted rows and the largest that has not, ragged tiles, ranks that own a part of the
+# experts, three and four blocks a box, intermediates too small for the last pass's box, units in chunks, the shared expert's
+# rows behind the routed ones
+CASES = [(("qwen_w1", synth.QWEN, 512, 256, False), 4095, 0.0, False, False), (("qwen_w1", synth.QWEN, 512, 256, False), 4096, 0.0, False, False),
+         (("qwen_w1", synth.QWEN, 512, 256, False), 5003, 1.0, False, False), (("qwen_w1", synth.QWEN, 512, 256, True), 4157, 0.5, True, False),
+         (("qwen_tp2", synth.QWEN, 256, 256, False), 4111, 0.5, False, False), (("qwen_ep4", synth.QWEN, 512, 64, False), 11003, 1.0, False, False),
+         (("ds_tp8", synth.DEEPSEEK, 256, 256, False), 4099, 0.5, False, False), (("ds_tp4", synth.DEEPSEEK, 512, 256, False), 4096, 1.0, False, False),
+         (("ds_ep8", synth.DEEPSEEK, 2048, 32, True), 4133, 0.5, False, False)]
+# more units left behind one round than are split, less than one round, likewise, a few left, the shared expert's among them;
+# few in less than one round, behind several, in chunks
+CASES += [(("qwen_ep4", synth.QWEN, 512, 64, False), 8192, 0.5, False, False), (("qwen_ep4", synth.QWEN, 512, 64, False), 7500, 0.0, False, False),
+          (("qwen_ep8", synth.QWEN, 512, 32, True), 18000, 0.0, False, True), (("qwen_ep8", synth.QWEN, 512, 32, False), 6000, 0.0, False, True),
+          (("qwen_w1", synth.QWEN, 512, 256, False), 10000, 0.0, False, True), (("ds_tp8", synth.DEEPSEEK, 256, 256, False), 8192, 0.0, False, True),
+          (("ds_ep8", synth.DEEPSEEK, 2048, 32, False), 8000, 0.0, False, True)]
 # the most tokens that the C entries take (the Python entries have a cap of their own): 31 full rounds, and no room in the
 # CTAs' lists for a part of the units behind them
-CASES += [(("qwen_w1", synth.QWEN, 512, 256, False), 71680, 0.0, False)]
+CASES += [(("qwen_w1", synth.QWEN, 512, 256, False), 71680, 0.0, False, False)]
 PASSES = {"qwen_w1": 4, "qwen_ep4": 4, "qwen_ep8": 4, "ds_tp8": 2, "ds_tp4": 4, "ds_ep8": 4}   # of a unit's up projection, where units are long
+MOST = {"qwen_w1": 74, "qwen_ep4": 74, "qwen_ep8": 74, "ds_tp8": 74, "ds_tp4": 111, "ds_ep8": 111}   # of less than a round that are split
 
 
-@pytest.mark.parametrize("build,T,skew,residual", CASES, ids=[f"{b[0]}{'-shared' if b[4] else ''}-{T}" for b, T, _, _ in CASES])
-def test_sorted_rows_give_the_bits_of_slot_order(build, T, skew, residual, monkeypatch):
+@pytest.mark.parametrize("build,T,skew,residual,splits", CASES, ids=[f"{c[0][0]}{'-shared' if c[0][4] else ''}-{c[1]}" for c in CASES])
+def test_sorted_rows_give_the_bits_of_slot_order(build, T, skew, residual, splits, monkeypatch):
     variant, spec, width, local, shared = build
     monkeypatch.setattr(loader, "MOE_MONOKERNEL_PREFILL_MAX_TOKENS", max(T, loader.MOE_MONOKERNEL_PREFILL_MAX_TOKENS))
     mk = MonoKernel(variant_path(variant))
@@ -44,40 +49,40 @@ def test_sorted_rows_give_the_bits_of_slot_order(build, T, skew, residual, monke
         kw["residual"] = torch.randn(T, spec.hidden, device=DEV).to(torch.bfloat16)
     needed = mk._int_symbol("workspace_min_bytes")
     behind = -(-needed // 256) * 256
+    positions = -(-T * 32 // 256) * 256
     got = []
-    for small in (False, True):
+    for size in (None, behind + positions, needed):   # all of it, the positions alone, neither
         sc = mk._allocate_scratch(T, DEV)
         sc["partial"].fill_(float("nan"))
         sc["sorted_ids"].fill_(-1)
-        if small:
-            sc["workspace"] = sc["workspace"][:needed]
-        else:
-            sc["workspace"][behind:behind + T * 32].fill_(0xEE)
+        sc["workspace"][behind:behind + positions].fill_(0xEE)
+        sc["workspace"] = sc["workspace"][:size]
         out = torch.full((T, spec.hidden), float("nan"), dtype=torch.bfloat16, device=DEV)
         mk.prefill_impl(batch["hs"], batch["logits"], layer["w13"], layer["w13_scale"], layer["w2"], layer["w2_scale"], 8,
                         True, layer["bias"], out, scratch=sc, check=True, **kw)
-        got.append((out.view(torch.int16), sc))
-    (a, sc), (b, flat) = got
-    assert torch.equal(a, b)
+        view = mk.workspace_view(sc["workspace"])
+        got.append((out.view(torch.int16), sc, view["total_tiles"], int(view["phase_ns"][6]) != 0))
+        sc["partial"] = None
+    (a, sc, units, split), (b, some, _, some_split), (c, _, _, no_split) = got
+    assert torch.equal(a, b) and torch.equal(a, c)
     assert bool(torch.isfinite(a.view(torch.bfloat16).float()).all())
-    pos = sc["workspace"][behind:behind + T * 32].view(torch.int32)
+    assert not no_split
     if T < 4096:
-        assert bool((pos.view(torch.uint8) == 0xEE).all())
+        assert all(bool((x["workspace"][behind:behind + T * 32] == 0xEE).all()) for x in (sc, some))
         return
-    rows = int((sc["topk_ids"] >= 0).sum())
     here = sc["topk_ids"].flatten() >= 0
-    assert bool((pos[~here] == -1).all())
-    assert torch.equal(sc["sorted_ids"][pos[here].long()], here.nonzero()[:, 0].int())
-    assert int(pos.max()) == rows - 1
+    for x in (sc, some):
+        pos = x["workspace"][behind:behind + T * 32].view(torch.int32)
+        assert bool((pos[~here] == -1).all())
+        assert torch.equal(x["sorted_ids"][pos[here].long()], here.nonzero()[:, 0].int())
+        assert int(pos.max()) == int(here.sum()) - 1
     # units behind the full rounds: split or not
-    view, chunks = mk.workspace_view(sc["workspace"]), max(width // 512, 1)
-    units = view["total_tiles"] + (-(-(-(-T // 128)) // (256 // local)) * chunks if shared else 0)
-    left = units % 148 if units > 148 else 0
-    split = int(view["phase_ns"][6]) != 0
-    if units > 148:
-        room = units // 148 + 2 <= mk._int_symbol("max_tiles") // 148
-        assert split == (variant in PASSES and 0 < left <= 148 // PASSES[variant] // chunks * chunks and room)
-    assert int(mk.workspace_view(flat["workspace"])["phase_ns"][6]) == 0
+    chunks = max(width // 512, 1)
+    units += -(-(-(-T // 128)) // (256 // local)) * chunks if shared else 0
+    most = 0 if variant not in PASSES else MOST[variant] if units < 148 else 148 // PASSES[variant] // chunks * chunks
+    room = units // 148 + 2 <= mk._int_symbol("max_tiles") // 148
+    assert split == splits == (0 < units % 148 <= most and room)
+    assert not some_split
 
 
 def test_the_build_without_row_stores_measures_the_sorted_form():

@@ -26,9 +26,13 @@ CASES += [(SHARED, 3, 0.5, None), (SHARED, 32, 0.0, None)]
 CASES += [(("ds_tp8", synth.DEEPSEEK, 256, 256, False), T, 0.5, None) for T in (1, 4)]
 CASES += [(("ds_ep8", synth.DEEPSEEK, 2048, 32, True), T, 0.5, None) for T in (8, 20)]
 CASES += [(("wide_ep8", WIDE, 256, 32, False), T, 0.5, None) for T in (3, 16)]
-# two waves of units through the intermediate: more rows than it holds; the shared expert's units in the second wave, and
-# units in chunks (2600 of the tokens on two local experts: 42 tiles)
+# from 4096 tokens on: whole units, and those behind the full round of 148 split, the shared expert's among them
 CASES += [(("qwen_ep8", synth.QWEN, 512, 32, True), 18000, 0.0, None)]
+# two waves of units through the intermediate: more rows than it holds. 2600 of the tokens on eight local experts: 168 units
+# with 20800 of the 18944 rows that it has room for, and the shared expert's 13 units at the end of the second wave; and units
+# in chunks (2600 of the tokens on two local experts: 42 tiles)
+CASES += [(("qwen_ep2", synth.QWEN, 512, 128, True), 3300, 0.0,
+           (2600, (1, 17, 40, 41, 77, 78, 100, 101), (130, 150, 170, 190, 200, 210, 220, 230)))]
 CASES += [(("ds_ep8", synth.DEEPSEEK, 2048, 32, False), 3200, 0.0,
            (2600, (3, 17, 40, 41, 77, 78, 100, 101), (40, 41, 77, 78, 100, 101, 130, 131)))]
 _layers = {}
@@ -83,8 +87,9 @@ def _run(build, T, skew, experts=None):
 
 @pytest.mark.parametrize("build,T,skew,experts", CASES, ids=[f"{b[0]}{'-shared' if b[4] else ''}-{T}" for b, T, _, _ in CASES])
 def test_split_units_give_the_bits_of_whole_units(build, T, skew, experts):
-    (a, a_split, _), (b, b_split, _) = _run(build, T, skew, experts)
+    (a, a_split, units), (b, b_split, _) = _run(build, T, skew, experts)
     assert (a_split, b_split) == (True, False)
+    assert not isinstance(experts, tuple) or units > 148
     assert torch.equal(a, b)
     assert bool(torch.isfinite(a.view(torch.bfloat16).float()).all())
 
@@ -104,12 +109,14 @@ def test_the_time_stamp_tells_which_form_ran():
 
 
 # 148 units fill one round of whole units, in which splitting does not pay from about 75 on (where a unit is long, H =
-# 7168 and 512 columns, from 112 on, and with a few rows a tile it pays throughout): up to there, and from 149 to about 203, the split form. 32 tokens reach 169 experts at even routing,
-# 124 at skew 0.5, 69 at skew 1.0.
-EP4, TP4 = ("qwen_ep4", synth.QWEN, 512, 64, False), ("ds_tp4", synth.DEEPSEEK, 512, 256, False)
+# 7168 and 512 columns, from 112 on, and with a few rows a tile it pays throughout): up to there, and from 149 to about 203,
+# the split form. 32 tokens reach 169 experts at even routing, 124 at skew 0.5, 69 at skew 1.0. From 4096 tokens on whole
+# units fill the round, and up to 37 behind it are split: 149 to 185.
+EP2, EP4, TP4 = ("qwen_ep2", synth.QWEN, 512, 128, False), ("qwen_ep4", synth.QWEN, 512, 64, False), ("ds_tp4", synth.DEEPSEEK, 512, 256, False)
 CHOICES = [(W1, 32, 0.0, None, (149, 203), True), (W1, 32, 0.5, None, (76, 148), False), (W1, 32, 1.0, None, (1, 74), True),
            (W1, 16, 0.0, None, (76, 148), False), (EP4, 7500, 0.0, None, (76, 148), False),
-           (EP4, 8192, 0.0, None, (149, 203), True), (TP4, 12, 0.0, "apart", (96, 96), True),
+           (EP2, 3850, 0.0, None, (149, 203), True), (EP4, 8192, 0.0, None, (149, 185), True),
+           (EP4, 10200, 0.0, None, (186, 203), False), (TP4, 12, 0.0, "apart", (96, 96), True),
            (TP4, 28, 0.5, None, (112, 148), True), (W1, 9, 0.0, "apart", (72, 72), True)]
 
 
