@@ -145,7 +145,7 @@ static_assert(E == 256, "routing keeps 8 logits per lane: exactly 256 experts");
 static_assert(E_LOCAL > 0 && E_LOCAL <= E, "local experts are a subset");
 static_assert(K_DIM % 128 == 0 && N_HALF % 128 == 0 && H_DIM % 256 == 0, "geometry must tile by 128/256");
 static_assert(ROUTER_MODE >= 0 && ROUTER_MODE <= 2, "unknown router mode");
-static_assert(NK % 2 == 0, "activation quantisation pairs two 128-column groups per warp");
+static_assert(NK % 4 == 0, "activation quantisation: the four quarter-warps have as many 128-column groups each");
 static_assert(ROUTER_MODE != 2 || N_GROUP * 32 == E, "grouped routing assumes 32 experts per group");
 
 // ------------------------------------------------------------------ launch shape
@@ -209,7 +209,7 @@ constexpr int MAX_TILES = MAX_MY_TILES * kGrid;
 // 128-column pass of the up projection), whose e4m3 result and scales go to global memory; then, behind a grid-wide
 // counter, every (unit, 256-column pass of the down projection). The intermediate leaves shared memory, and the weight
 // ring takes its place. The operations on a row and their order are those of the whole unit: the same bits come out.
-// (With one pass of the up projection per unit there is too little to cut: no number of units makes it pay.)
+// (With one pass of the up projection per unit there is too little to cut in two halves: SHARE_BUILD below.)
 // Profiling and ablation builds compute whole units (of large batches with sorted rows too): the stall counters and the
 // switches are in that loop only.
 #ifdef MONO_PROFILE
@@ -306,7 +306,9 @@ constexpr int RK = K_DIM / 64;
 constexpr int kDirectTokens = 256;
 // Smallest batch whose partial rows are in sorted order: an expert then has a full tile on average. Launch in us, slot order ->
 // sorted, H=2048 I=512: 2048 tokens 193 -> 198, 3000 215 -> 221, 4096 298 -> 298, 5000 371 -> 361; H=7168 I=256: 2500 503 -> 508,
-// 4096 614 -> 609, 6000 824 -> 813; 128 of 256 experts: 4096 tokens 197 -> 191.
+// 4096 614 -> 609, 6000 824 -> 813. Ranks with a part of the experts have longer units then: 128 of 256 experts 4096 tokens
+// (192 units) 197 -> 182, 64 of 256 9600 (190, before in the split form) 238 -> 211, 10800 (196) 245 -> 221, 32 of 256 23000 (203)
+// 322 -> 286, 32 of 256 at H=7168 in four chunks 4300 (196) 791 -> 766 (all with the changes to routing and SiLU).
 constexpr int kSortedTokens = 4096;
 // Largest batch that every CTA routes for itself. Launch in us, dealt over the CTAs -> by each: 1 token 35.2 -> 31.8, 4 39.0 -> 35.3,
 // 64 of 256 experts 9 35.6 -> 34.8, 12 tokens 74.1 -> 74.9 (a warp's token takes longer with all warps of the SM at it); H=7168
@@ -1108,7 +1110,8 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
         for (int i = 0; i < TCOLS / 2; ++i) acc[i] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int dk = 0; dk < NP; ++dk) promote(acc, sc[dk], sc[dk], down_col);
-        const int prow = fi < 0 ? -1 : SORTED ? ti.chunk * (numel + (p.sh_on ? p.num_tokens : 0)) + (sh ? numel : 0) + ti.row0 + r : fi * NCH + ti.chunk;
+        const int rows = numel + (p.sh_on ? p.num_tokens : 0);   // of a chunk, in sorted order
+        const int prow = fi < 0 ? -1 : SORTED ? ti.chunk * rows + (sh ? numel : 0) + ti.row0 + r : fi * NCH + ti.chunk;
         store_rows(p, acc, prow, make_float2(rw, rw), hb * 256 + h * WC, !dead);
       }
       if (w + 1 < waves) meet(static_cast<uint32_t>((2 * w + 2) * kGrid));  // the intermediate may be overwritten
@@ -1117,8 +1120,9 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
 }
 
 // ------------------------------------------------------------------ the kernel
-// FORM_SORTED: whole units with the partial rows in sorted order (and the split form for those behind the full rounds), an instance of its own because its store section changes
-// the registers of the slab loop (the others take 2 to 5 % longer with both in one).
+// FORM_SORTED: whole units with the partial rows in sorted order (and the split form for those behind the full rounds), an
+// instance of its own because its store section changes the registers of the slab loop (the others take 2 to 5 % longer with
+// both in one).
 // FORM_SHORT: the instance for batches that are expected to be short. It holds both forms of the expert phase and takes one of
 // them by the units that phase 1 counts. FORM_WHOLE computes whole units only, and computes them faster: inside
 // the first one they take 2 to 4 us more a launch (16 tokens 85 -> 88 us, 64 of 256 experts at 7500 tokens 153 -> 157).
@@ -2633,7 +2637,8 @@ int make_bf16_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
-// Sorted partial rows [rows, H] bf16 as blocks of 32 columns: a box is 32 rows of ROW_BLOCKS neighbouring blocks.
+// Sorted partial rows [rows, H] bf16 as blocks of 32 columns: a box is 32 rows of ROW_BLOCKS neighbouring blocks. Encoded at
+// every launch that has them: its base and rows are those of the caller's scratch and batch.
 int make_rows_map(CUtensorMap* m, void* base, uint64_t rows) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return -1;
@@ -2649,7 +2654,7 @@ int make_rows_map(CUtensorMap* m, void* base, uint64_t rows) {
 // Plan / run split. What a launch needs besides its arguments depends only on the device (the kernel's
 // shared-memory attribute) and on the weight tensors (their TMA descriptors: base address + the compiled
 // extents). Both are made once and kept: a descriptor per (kind, base address, rows) in a small table, the
-// attribute once per device. The reference re-encodes both descriptors and re-sets the attribute on every
+// attribute once per device. (The descriptor of sorted partial rows is not among them.) The reference re-encodes both descriptors and re-sets the attribute on every
 // call (kernel/qwen_tp/src/prefill_mono_final_nb.cu:1611-1639, :1655).
 struct MapKey {
   const void* base;
