@@ -239,7 +239,8 @@ int prefill_wgmma_cta_pair(void);
  * enough for 1 or 2 chunks). */
 int prefill_wgmma_partial_chunks(void);
 int prefill_wgmma_block_threads(void);        /* threads per CTA */
-int prefill_wgmma_list_places(int units);     /* longest per-CTA unit list of a large batch; at most max_tiles / grid_size */
+int prefill_wgmma_list_places(int units);     /* longest per-CTA unit list of a large batch */
+int prefill_wgmma_list_room(void);            /* places of a list: never fewer */
 int prefill_wgmma_stable_sort(void);          /* 1 = sorted_token_ids is deterministic (stable) */
 /* The workspace that every launch accepts (230 KB); the rest of prefill_wgmma_workspace_bytes() is the intermediate of
  * the split form: 10 MB, 5 MB at N_HALF = 256, none at 128 and in the two-CTA build, which have no split form. */

@@ -101,3 +101,26 @@ def test_the_build_without_row_stores_measures_the_sorted_form():
     pos = sc["workspace"][behind:behind + T * 32].view(torch.int32)
     assert torch.equal(torch.sort(pos).values, torch.arange(T * 8, dtype=torch.int32, device=DEV))
     assert bool(sc["partial"].isnan().all())
+
+
+def test_the_largest_batch_in_pairs_of_tiles(monkeypatch):
+    """More than 32 pairs for a cluster: one ragged pair per expert behind the full ones. Same bits as the build that deals tiles."""
+    T = 71680
+    monkeypatch.setattr(loader, "MOE_MONOKERNEL_PREFILL_MAX_TOKENS", T)
+    layer = synth.make_layer(synth.QWEN, seed=5, device=DEV, with_shared=False)
+    for seed in range(40):
+        batch = synth.make_batch(synth.QWEN, layer, T, seed=seed, device=DEV)
+        pairs = int((torch.bincount(batch["logits"].topk(8, dim=-1).indices.flatten(), minlength=256) + 255).div(256, rounding_mode="floor").sum())
+        if pairs > 32 * 74:
+            break
+    got = []
+    for variant in ("qwen_w1_pair", "qwen_w1"):
+        mk = MonoKernel(variant_path(variant))
+        sc = mk._allocate_scratch(T, DEV)
+        out = torch.full((T, 2048), float("nan"), dtype=torch.bfloat16, device=DEV)
+        mk.prefill_impl(batch["hs"], batch["logits"], layer["w13"], layer["w13_scale"], layer["w2"], layer["w2_scale"], 8, True,
+                        None, out, scratch=sc, check=True)
+        got.append((out.view(torch.int16), mk.workspace_view(sc["workspace"])["total_tiles"]))
+    assert got[0][1] == pairs > 32 * 74
+    assert torch.equal(got[0][0], got[1][0])
+    assert bool(torch.isfinite(got[0][0].view(torch.bfloat16).float()).all())

@@ -198,8 +198,9 @@ constexpr int BLOCK = 128 + N_EPI;
 constexpr int NWARPS = BLOCK / 32;
 constexpr int WARP_TMA = 0, WARP_MMA = 1, WARP_GATHER0 = 2;  // warps 2,3 gather; warps 4.. epilogue
 constexpr int N_GATHER = 64;
-constexpr int MAX_MY_TILES = 32 * NCH;
-constexpr int MAX_TILES = MAX_MY_TILES * kGrid;
+constexpr int MAX_TILES = 32 * NCH * kGrid;   // tiles that a launch is accepted with
+// Places of a CTA's list of them. Pairs: half as many rows' worth to a list, but still a ragged one per expert.
+constexpr int MAX_MY_TILES = PAIR ? ((MAX_TILES - E_LOCAL) / 2 + E_LOCAL + kGrid / 2 - 1) / (kGrid / 2) : 32 * NCH;
 
 // ------------------------------------------------------------------ the split form of the expert phase
 // A unit of the schedule (one tile, all of its passes) keeps one CTA busy for NP * NK + NHB * NP slab steps. That is
@@ -781,7 +782,8 @@ __host__ __device__ constexpr int rest_units(int units) {
 // Places that the longest list of a CTA takes up in a large batch: its whole units, and its share of those that are split.
 constexpr int list_places(int units) {
   const int rest = REST_BUILD ? rest_units(units) : 0, whole = units - rest;
-  int most = (whole + kGrid - 1) / kGrid;
+  constexpr int LISTS = PAIR ? kGrid / 2 : kGrid;   // a pair of tiles is dealt to a cluster of two CTAs
+  int most = (whole + LISTS - 1) / LISTS;
   for (int cta = 0; cta < kGrid; ++cta) {
     const SplitShare s = split_share(rest, cta);
     if (s.hi > s.lo && whole / kGrid + s.hi - s.lo > most) most = whole / kGrid + s.hi - s.lo;
@@ -2779,8 +2781,9 @@ int prefill_wgmma_cta_pair() { return PAIR ? 1 : 0; }
 // allocation is large enough, beyond that the caller sizes it from this accessor.
 int prefill_wgmma_partial_chunks() { return NCH; }
 int prefill_wgmma_block_threads() { return BLOCK; }
-// Places of the longest per-CTA unit list of a large batch of `units` units; a list has max_tiles / grid_size of them.
+// Places of the longest per-CTA unit list of a large batch of `units` units, and those that a list has.
 int prefill_wgmma_list_places(int units) { return list_places(units); }
+int prefill_wgmma_list_room() { return MAX_MY_TILES; }
 int prefill_wgmma_stable_sort() { return 1; }
 // Byte offset of the 32-bit status word inside the workspace and the bytes that follow it
 // (status, abort flag, two detail words). 0 after a successful launch.
