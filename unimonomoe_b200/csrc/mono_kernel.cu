@@ -299,9 +299,9 @@ static_assert(!SORTED_BUILD || ROW_SLOT_BYTES * (N_EPI / 32) <= SA * A_STAGE_BYT
 // The slot sum reads each partial row once. Loads of 384 threads keep 48 KB an SM on their way, and that bounds them where a
 // token's rows are neighbours, in slot order; the copy engine keeps 200 KB on its way, in stages of SUM_COLS columns of them. Sum in
 // us, loads -> copies, H=2048 I=128: 2960 tokens 18.7 -> 16.7 (launch 101.8 -> 100.8), 4000 29.8 -> 23.2 (130.3 -> 125.8), 8192 59 -> 47
-// (213.3 -> 205.8; with a shared expert 240.6 -> 226.6), 20000 136 -> 107 (470 -> 463). Not for rows all over the buffer, where memory pages bound both
-// (sorted rows, 8192 tokens 60 -> 65, H=7168 16384 393 -> 429), nor for ranks that have two rows of eight (33 -> 48). Two or three
-// vectors a thread instead: no difference, slower. An instance of its own, FORM_COPIES: with this code in it too the other one takes
+// (213.3 -> 205.8; with a shared expert 240.6 -> 226.6), 20000 136 -> 107 (470 -> 463). Not for rows all over the buffer, where
+// memory pages bound both (sorted rows, 8192 tokens 60 -> 65, H=7168 16384 393 -> 429), nor for ranks that have two rows of eight
+// (33 -> 48). Two or three vectors a thread instead: no difference, slower. An instance of its own, FORM_COPIES: with this code in it too the other one takes
 // 2 to 4 us more a launch at every size (60 tokens 57.7 -> 59.9), for instructions that it fetches and does not need.
 constexpr bool COPIES_BUILD = !SORTED_BUILD && !EP_BUILD && !PAIR;
 constexpr int sum_cols() {   // the largest part of a row that makes a stage of 32 KB at most, in 16-byte vectors for 256 threads
@@ -409,7 +409,7 @@ struct alignas(16) TileInfo {   // read as one 16-byte word
 };
 constexpr int SHARED_E = E_LOCAL;
 
-enum Form { FORM_WHOLE, FORM_SHORT, FORM_SORTED, FORM_COPIES };   // instances of the kernel
+enum Form { FORM_WHOLE, FORM_SHORT, FORM_SORTED, FORM_COPIES, FORM_SOLO };   // instances of the kernel
 
 // ------------------------------------------------------------------ small helpers
 __device__ __forceinline__ uint32_t float_key(float f) {
@@ -1167,7 +1167,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   const int T = p.num_tokens;
   const int numel = T * TOP_K;
 
-  constexpr bool CAN_SPLIT = FORM == FORM_SHORT && SPLIT_BUILD;
+  constexpr bool SOLO = FORM == FORM_SOLO && SPLIT_BUILD;   // a few tokens: routed by every CTA, in the split form, nothing reduced
+  constexpr bool CAN_SPLIT = (FORM == FORM_SHORT || SOLO) && SPLIT_BUILD;
   constexpr bool SORTED = FORM == FORM_SORTED && SORTED_BUILD;
   constexpr bool COPIES = FORM == FORM_COPIES && COPIES_BUILD;   // the slot sum's rows come through shared memory
   constexpr bool SHARE = (FORM == FORM_WHOLE || COPIES) && SHARE_BUILD;   // units behind the full rounds are shared by several CTAs
@@ -1195,7 +1196,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   // launch sequence of the tensor-parallel epilogue: a device counter outside the
   // workspace (which is zeroed every launch) so that CUDA-graph replays advance it
   // (kernel/qwen_tp/src/prefill_mono_final_nb.cu:985-1016)
-  const bool tp_on = (p.tp_mc != nullptr) && (p.tp_pads != nullptr) && (p.tp_ncomm > 0);
+  const bool tp_on = !SOLO && (p.tp_mc != nullptr) && (p.tp_pads != nullptr) && (p.tp_ncomm > 0);
   if (tp_on && p.tp_seqctr != nullptr && bid == 0 && tid == 0) {
     const uint32_t sq = atomicAdd(p.tp_seqctr, 1u) + 1u;
     atomicExch(&ws->tp_seq_pub, sq);
@@ -1206,7 +1207,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   // (routing and quantisation of 200 tokens 5.8 -> 5.2 us, of 777 at H = 7168 16.2 -> 14.5).
   // A batch of a few tokens is routed and sorted by every CTA for itself: all of them write the same bytes, each reads what it
   // wrote, and the two grid barriers in front of the expert phase are not needed.
-  const bool solo = !PAIR && T <= kSoloTokens && p.logits_out == nullptr;
+  const bool solo = SOLO || (!PAIR && T <= kSoloTokens && p.logits_out == nullptr);
   const int cta_t0 = solo ? 0 : static_cast<int>(static_cast<long long>(bid) * T / kGrid);
   const int cta_t1 = solo ? T : static_cast<int>(static_cast<long long>(bid + 1) * T / kGrid);
   const int t_begin = cta_t0 + warp * (cta_t1 - cta_t0) / NWARPS, t_end = cta_t0 + (warp + 1) * (cta_t1 - cta_t0) / NWARPS;
@@ -1217,7 +1218,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   // core's fp32 accumulator over K slabs of 64 in ascending order (its order inside one instruction is
   // the hardware's). One accumulator of 128 tokens x 256 experts in tensor memory; TMA brings one
   // [128 x 64] slab of x and one [256 x 64] slab of W_r per stage, both in the 128-byte swizzle.
-  const bool gemv = !PAIR && p.logits_out != nullptr;  // the pair build keeps every tcgen05 instruction at cta_group::2
+  const bool gemv = !PAIR && !SOLO && p.logits_out != nullptr;  // the pair build keeps every tcgen05 instruction at cta_group::2
   if (gemv) {
     if (tid == 0) {
       for (int s = 0; s < RS; ++s) { mbar_init(&S.rfull[s], 1); mbar_init(&S.rempty[s], 1); }
@@ -1459,11 +1460,11 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     // Split form: in one wave every row of the batch has its place in the intermediate (its sorted position); in waves of
     // kGrid units the place is that of the unit in its wave.
     const int units = tt_routed + sh_units;
-    const bool one_wave = rows_routed + sh_units / NCH * TILE_M <= p.sp_rows;
+    const bool one_wave = SOLO || rows_routed + sh_units / NCH * TILE_M <= p.sp_rows;
     bool split = false;
     int lo = 0, hi = 0;       // this CTA's units of the last wave
     if constexpr (CAN_SPLIT) {
-      split = units > 0 && split_pays(units, rows_routed * NCH <= FEW_ROWS * tt_routed, one_wave);
+      split = SOLO || (units > 0 && split_pays(units, rows_routed * NCH <= FEW_ROWS * tt_routed, one_wave));
       const SplitShare mine = split_share(one_wave ? units : units - kGrid, bid);
       lo = mine.lo;
       hi = mine.hi;
@@ -1600,14 +1601,14 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   // inter_ready barriers collect the epilogue warps of both CTAs.
   const uint32_t crank = PAIR ? cluster_ctarank() : 0u;
   const bool leader = crank == 0u;
-  const bool split = CAN_SPLIT && alive && S.sp_waves != 0;
+  const bool split = SOLO || (CAN_SPLIT && alive && S.sp_waves != 0);
   if (tid == 0) {
     const uint32_t both = PAIR ? 2u : 1u;
-    for (int s = 0; s < SA; ++s) {
+    for (int s = 0; !SOLO && s < SA; ++s) {
       mbar_init(&S.fullA[s], N_GATHER + ((PAIR && leader) ? 1u : 0u));
       mbar_init(&S.emptyA[s], 1);
     }
-    for (int s = 0; s < SB; ++s) { mbar_init(&S.fullB[s], 1); mbar_init(&S.emptyB[s], 1); }
+    for (int s = 0; !SOLO && s < SB; ++s) { mbar_init(&S.fullB[s], 1); mbar_init(&S.emptyB[s], 1); }
     if constexpr (CAN_SPLIT || REST) {
       for (int s = 0; s < SPLIT_SA; ++s) { mbar_init(&S.sp.fullA[s], N_GATHER); mbar_init(&S.sp.emptyA[s], 1); }
       for (int s = 0; s < SPLIT_SB; ++s) { mbar_init(&S.sp.fullB[s], 1); mbar_init(&S.sp.emptyB[s], 1); }
@@ -1617,7 +1618,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
 #ifdef MONO_PROFILE
     for (int i = 0; i < 48; ++i) (&S.whist[0][0])[i] = 0ull;
 #endif
-    for (int s = 0; s < NP; ++s) mbar_init(&S.inter_ready[s], both * (N_EPI / 32));
+    for (int s = 0; !SOLO && s < NP; ++s) mbar_init(&S.inter_ready[s], both * (N_EPI / 32));
     mbar_init(&S.rows_read, N_EPI / 32);
     mbar_init_fence();
   }
@@ -2811,6 +2812,16 @@ bool short_expected(int num_tokens, int sh_units) {
   return units <= most1 || (units > kGrid && units <= kGrid + most2);
 }
 
+// Batches that every CTA routes for itself and that the split form is faster for whatever they reach: at most an expert a slot (and
+// the shared expert's `sh_units`). They have an instance with nothing else in it: routing, scan and sum are shorter where the compiler
+// knows what is not asked for (one token 2.8 + 1.6 + 1.8 -> 2.5 + 1.2 + 0.9 us). Launch in us, FORM_SHORT -> FORM_SOLO: 1 token 30.7 ->
+// 29.1, 4 39.0 -> 36.0, with the shared expert 43.9 -> 38.8, 8 59.0 -> 53.7; 64 of 256 experts 8 tokens 32.8 -> 30.8; H=7168 I=256 1 59.4
+// -> 57.4, 8 92.1 -> 86.4, 32 of 256 experts in chunks 8 94.6 -> 87.9.
+bool solo_split(int num_tokens, int sh_units) {
+  const int most = (num_tokens * TOP_K < E_LOCAL ? num_tokens * TOP_K : E_LOCAL) * NCH + sh_units;
+  return num_tokens <= kSoloTokens && (most <= SPLIT_MOST_1 || (LONG_UNITS && most <= kGrid));
+}
+
 cudaError_t ensure_kernel_attribute(int dev) {
   std::lock_guard<std::mutex> lock(g_plan_mutex);
   if (dev >= 0 && dev < 64 && g_attr_set[dev]) return cudaSuccess;
@@ -2826,6 +2837,8 @@ cudaError_t ensure_kernel_attribute(int dev) {
   if constexpr (SPLIT_BUILD) {
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(moe_prefill_kernel<FORM_SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SHORT_DYN_SMEM);
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(moe_prefill_kernel<FORM_SOLO>, cudaFuncAttributeMaxDynamicSharedMemorySize, SHORT_DYN_SMEM);
   }
   if (err == cudaSuccess && dev >= 0 && dev < 64) g_attr_set[dev] = true;
   return err;
@@ -3141,14 +3154,18 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
     }
     return 0;
   }
+  const bool reduces = p.tp_mc != nullptr && p.tp_pads != nullptr && p.tp_ncomm > 0;
   if constexpr (SPLIT_BUILD) {
-    if (short_batch) moe_prefill_kernel<FORM_SHORT><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
+    if (short_batch && !reduces && router_w == nullptr && solo_split(num_tokens, static_cast<int>(sh_tiles) * NCH)) {
+      moe_prefill_kernel<FORM_SOLO><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
+    } else if (short_batch) {
+      moe_prefill_kernel<FORM_SHORT><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
+    }
   }
   if constexpr (SORTED_BUILD) {
     if (p.slot_pos != nullptr) moe_prefill_kernel<FORM_SORTED><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
   }
   // (not with the in-kernel reduce, whose transfer follows the chunks of the loop over the output)
-  const bool reduces = p.tp_mc != nullptr && p.tp_pads != nullptr && p.tp_ncomm > 0;
   const bool copies = COPIES_BUILD && !reduces && static_cast<uint32_t>(num_tokens) * SUM_PARTS >= kSumItems;
   if constexpr (COPIES_BUILD) {
     if (copies) moe_prefill_kernel<FORM_COPIES><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
