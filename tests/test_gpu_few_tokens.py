@@ -41,3 +41,20 @@ def test_no_expert_of_this_rank(T):
     mk.prefill_impl(batch["hs"], logits, layer["w13"], layer["w13_scale"], layer["w2"], layer["w2_scale"], 8, True, layer["bias"], out,
                     scratch=mk._allocate_scratch(T, DEV), check=True, expert_map=synth.expert_map(spec, 0, 8, device=DEV))
     assert torch.equal(out, torch.zeros_like(out))
+
+
+@pytest.mark.parametrize("T", [9, 300, 2048, 2049])
+def test_scales_from_global_memory(T):
+    """K = 7168 beside an intermediate of 512 columns: a token's output is the same bits with the activation scales in shared memory
+    (from 2049 tokens on) and loaded from global memory (below)."""
+    spec, first = synth.DEEPSEEK, 2049
+    mk = MonoKernel(variant_path("ds_ep8"))
+    layer = synth.make_layer(spec, seed=4, device=DEV, expert_slice=(0, 32), with_shared=False)
+    batch = synth.make_batch(spec, layer, first, seed=4, device=DEV)
+    emap = synth.expert_map(spec, 0, 8, device=DEV)
+    out = {}
+    for n in (T, first):   # a token's output does not depend on the batch that it is in
+        out[n] = torch.full((n, spec.hidden), float("nan"), dtype=torch.bfloat16, device=DEV)
+        mk.prefill_impl(batch["hs"][:n], batch["logits"][:n], layer["w13"], layer["w13_scale"], layer["w2"], layer["w2_scale"], 8, True,
+                        layer["bias"], out[n], scratch=mk._allocate_scratch(n, DEV), check=True, expert_map=emap)
+    assert torch.equal(out[T], out[first][:T])

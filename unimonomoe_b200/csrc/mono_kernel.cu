@@ -253,13 +253,27 @@ constexpr int SA = SA_RAW > STAGE_CAP ? STAGE_CAP : SA_RAW;
 static_assert(SB >= 2 && SA >= 2, "intermediate too wide for shared memory: shard N_HALF further");
 constexpr int DYN_SMEM = 1024 + INTER_BYTES + SA * A_STAGE_BYTES + SB * B_STAGE_BYTES + SCALE_BYTES;
 static_assert(NWARPS * E * 4 <= SA * A_STAGE_BYTES, "phase-0 histograms live in the activation ring");
+// Beside an intermediate of 512 columns the activation scales of K = 7168 (28 KB) take the room of a third weight stage, and two
+// stages keep 64 KB of weights on their way where memory wants 96. Where tiles have few rows (FORM_SHORT, FORM_FEW) a thread loads its
+// row's scales from global memory instead, two slab steps ahead. Launch in us, two stages -> three, H=7168, I=512: 64 tokens 606 ->
+// 543, 777 714 -> 642; 32 of 256 experts, I=2048 in chunks: 40 tokens 307 -> 266, 200 350 -> 307, 800 384 -> 342, 2048 418 -> 387, with
+// the shared expert 446 -> 419. With full tiles the loads cost what the stage gives: I=512 2500 tokens 817 -> 833, 4095 1126 -> 1208,
+// 8192 (sorted rows) 1789 -> 1917; 32 of 256 experts 3900 763 -> 742. At I=256 a fourth stage is all there is to gain: 777 tokens 343 ->
+// 346, 2500 418 -> 442.
+constexpr int kFewTokens = 2048;   // half a tile to an expert
+constexpr int SCALE_BYTES_AG = ((2 * WSU_N + 2 * WSD_N) * 4 + 1023) / 1024 * 1024;
+constexpr int SB_AG = (SMEM_AVAIL + SCALE_BYTES - SCALE_BYTES_AG - SA * A_STAGE_BYTES) / B_STAGE_BYTES;
+constexpr bool AS_GLOBAL = SB == 2 && SB_AG > SB && MONO_ABLATE == 0;
+constexpr int FEW_DYN_SMEM = AS_GLOBAL ? 1024 + INTER_BYTES + SA * A_STAGE_BYTES + SB_AG * B_STAGE_BYTES + SCALE_BYTES_AG : DYN_SMEM;
 // split form: no intermediate and no scale staging in shared memory, so the weight ring is deeper
 constexpr int SPLIT_SA = 3;
 constexpr int SPLIT_SB = (SMEM_CAP - SMEM_STATIC_RESERVE - 1024 - SPLIT_SA * A_STAGE_BYTES) / B_STAGE_BYTES;
 constexpr int SPLIT_SMEM = 1024 + SPLIT_SA * A_STAGE_BYTES + SPLIT_SB * B_STAGE_BYTES;
-constexpr int SHORT_DYN_SMEM = (SPLIT_BUILD && SPLIT_SMEM > DYN_SMEM) ? SPLIT_SMEM : DYN_SMEM;  // either form
+constexpr int EITHER_SMEM = FEW_DYN_SMEM > DYN_SMEM ? FEW_DYN_SMEM : DYN_SMEM;
+constexpr int SHORT_DYN_SMEM = (SPLIT_BUILD && SPLIT_SMEM > EITHER_SMEM) ? SPLIT_SMEM : EITHER_SMEM;  // either form
 constexpr int A_STAGE_CAP = SPLIT_SA > STAGE_CAP ? SPLIT_SA : STAGE_CAP;
 constexpr int B_STAGE_CAP = SPLIT_SB > STAGE_CAP ? SPLIT_SB : STAGE_CAP;
+static_assert(!AS_GLOBAL || SB_AG <= B_STAGE_CAP, "barriers of the weight stages");
 static_assert(!SPLIT_BUILD || SPLIT_SB >= 3, "the split form needs a weight ring of at least three stages");
 
 // Register budget (setmaxnreg). The kernel launches with REGS_LAUNCH registers per thread; the
@@ -409,7 +423,7 @@ struct alignas(16) TileInfo {   // read as one 16-byte word
 };
 constexpr int SHARED_E = E_LOCAL;
 
-enum Form { FORM_WHOLE, FORM_SHORT, FORM_SORTED, FORM_COPIES, FORM_SOLO };   // instances of the kernel
+enum Form { FORM_WHOLE, FORM_SHORT, FORM_SORTED, FORM_COPIES, FORM_SOLO, FORM_FEW };   // instances of the kernel
 
 // ------------------------------------------------------------------ small helpers
 __device__ __forceinline__ uint32_t float_key(float f) {
@@ -1173,6 +1187,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   constexpr bool COPIES = FORM == FORM_COPIES && COPIES_BUILD;   // the slot sum's rows come through shared memory
   constexpr bool SHARE = (FORM == FORM_WHOLE || COPIES) && SHARE_BUILD;   // units behind the full rounds are shared by several CTAs
   constexpr bool REST = SORTED && REST_BUILD;   // what is left behind the full rounds of units can be split
+  constexpr bool AS_GLOBAL = (FORM == FORM_SHORT || FORM == FORM_FEW) && mono::AS_GLOBAL;   // activation scales from global memory, and a weight stage more
+  constexpr int SB = AS_GLOBAL ? SB_AG : mono::SB;
   constexpr int RS = (SA < SB) ? SA : SB;  // stages of the router linear's ring
   // 1024-byte aligned base of the operand buffers
   const uint32_t dyn_u32 = (smem_u32(dyn_raw) + 1023u) & ~1023u;
@@ -1181,7 +1197,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   uint8_t* a_ring = dyn + INTER_BYTES;
   uint8_t* b_ring = a_ring + SA * A_STAGE_BYTES;
   float* as_sm = reinterpret_cast<float*>(b_ring + SB * B_STAGE_BYTES);  // [NK][128]
-  float* wsu_sm = as_sm + NK * TILE_M;                                    // [2][WSU_N]
+  float* wsu_sm = as_sm + (AS_GLOBAL ? 0 : NK * TILE_M);                  // [2][WSU_N]
   float* wsd_sm = wsu_sm + 2 * WSU_N;                                     // [2][WSD_N]
   int* hist = reinterpret_cast<int*>(a_ring);  // [NWARPS][E], phases 0-1 only
   int* scan_cnt = reinterpret_cast<int*>(b_ring);  // phase 1 only: four arrays of E ints
@@ -2067,7 +2083,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       if (n_my > 0) {
         stage_ids(0);
         stage_weight_store(0);
-        for (int j = 0; j < AS_PIECES; ++j) { as_piece_load(j); as_piece_store(j); }
+        for (int j = 0; !AS_GLOBAL && j < AS_PIECES; ++j) { as_piece_load(j); as_piece_store(j); }
       }
 
       for (int it = 0; it < n_my; ++it) {
@@ -2082,6 +2098,10 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
         const int tile_row = SORTED ? ti.chunk * (numel + (p.sh_on ? T : 0)) + (ti.e == SHARED_E ? numel : 0) + ti.row0 : 0;
         const int prow = fi < 0 ? -1 : tile_row + r;
         const bool box_full = SORTED && __all_sync(0xFFFFFFFFu, fi >= 0);
+        // the row's scales of the next slab and the one behind it; a pass begins with those that the one before it has loaded
+        const float* as_row = p.act_scales + static_cast<size_t>(fi < 0 ? 0 : ntok) * NK;
+        float a_n1 = 0.f, a_n2 = 0.f;
+        if (AS_GLOBAL && fi >= 0) { a_n1 = __ldcg(as_row); a_n2 = __ldcg(as_row + 1); }
         float iscale[NP];
         { PROF_T0();
         named_bar_sync(1, N_EPI);  // this tile's staged scales are visible to all epilogue threads
@@ -2094,7 +2114,14 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
           for (int i = 0; i < TCOLS / 2; ++i) acc[i] = make_float2(0.f, 0.f);
           PROF_ADD(pe_zero); }
           for (int ks = 0; ks < NK; ++ks) {
-            const float a_s = as_sm[ks * TILE_M + r];
+            float a_s;
+            if constexpr (AS_GLOBAL) {
+              a_s = a_n1;
+              a_n1 = a_n2;
+              if (fi >= 0) a_n2 = __ldcg(as_row + (ks + 2 < NK ? ks + 2 : ks + 2 - NK));
+            } else {
+              a_s = as_sm[ks * TILE_M + r];
+            }
             const float s_g = __fmul_rn(wsu_t[ps * NK + ks], a_s), s_u = __fmul_rn(wsu_t[(NP + ps) * NK + ks], a_s);
 #pragma unroll
             for (int j = 0; j < NSPLIT; ++j) {
@@ -2181,7 +2208,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
           for (int i = 0; i < TCOLS / 2; ++i) acc[i] = make_float2(0.f, 0.f);
           if (has_next) {
             if (hb == 1) stage_weight_store(it + 1);
-            if (hb >= 1 && hb - 1 < AS_PIECES) as_piece_load(hb - 1);
+            if (!AS_GLOBAL && hb >= 1 && hb - 1 < AS_PIECES) as_piece_load(hb - 1);
           }
 #pragma unroll
           for (int dk = 0; dk < NP; ++dk) {
@@ -2279,7 +2306,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
           } else if (alive_w && (MONO_ABLATE & 4) == 0) {
             store_direct(std::integral_constant<int, 0>(), fi, NCH, ti.chunk);
           }
-          if (has_next && hb >= 1 && hb - 1 < AS_PIECES) as_piece_store(hb - 1);
+          if (!AS_GLOBAL && has_next && hb >= 1 && hb - 1 < AS_PIECES) as_piece_store(hb - 1);
           PROF_ADD(pe_store);
         }
       }
@@ -2826,6 +2853,10 @@ cudaError_t ensure_kernel_attribute(int dev) {
   std::lock_guard<std::mutex> lock(g_plan_mutex);
   if (dev >= 0 && dev < 64 && g_attr_set[dev]) return cudaSuccess;
   cudaError_t err = cudaFuncSetAttribute(moe_prefill_kernel<FORM_WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM);
+  if constexpr (AS_GLOBAL) {
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(moe_prefill_kernel<FORM_FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_DYN_SMEM);
+  }
   if constexpr (COPIES_BUILD) {
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(moe_prefill_kernel<FORM_COPIES>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM);
@@ -3170,7 +3201,13 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
   if constexpr (COPIES_BUILD) {
     if (copies) moe_prefill_kernel<FORM_COPIES><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
   }
-  if (!short_batch && p.slot_pos == nullptr && !copies) moe_prefill_kernel<FORM_WHOLE><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
+  const bool few = AS_GLOBAL && num_tokens <= kFewTokens;
+  if (!short_batch && p.slot_pos == nullptr && !copies) {
+    if constexpr (AS_GLOBAL) {
+      if (few) moe_prefill_kernel<FORM_FEW><<<kGrid, BLOCK, FEW_DYN_SMEM, stream>>>(p);
+    }
+    if (!few) moe_prefill_kernel<FORM_WHOLE><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
+  }
   err = cudaGetLastError();
   if (err != cudaSuccess) {
     fprintf(stderr, "kernel launch failed: %s\n", cudaGetErrorString(err));
