@@ -1200,10 +1200,11 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   float* wsu_sm = as_sm + (AS_GLOBAL ? 0 : NK * TILE_M);                  // [2][WSU_N]
   float* wsd_sm = wsu_sm + 2 * WSU_N;                                     // [2][WSD_N]
   int* hist = reinterpret_cast<int*>(a_ring);  // [NWARPS][E], phases 0-1 only
-  int* scan_cnt = reinterpret_cast<int*>(b_ring);  // phase 1 only: four arrays of E ints
+  int* scan_cnt = reinterpret_cast<int*>(b_ring);  // phase 1 only: four arrays of E ints and the warps' sums
   int* scan_tile = scan_cnt + E;
   int* ph1_tot = scan_tile + E;
   int* ph1_pre = ph1_tot + E;
+  int* scan_warp = ph1_pre + E;
 
   if (bid == 0 && tid == 0) {
     ws->phase_ns[0] = globaltimer_ns();
@@ -1455,17 +1456,28 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     if (tid < E) {
       cnt = ph1_tot[tid];
       tiles_e = (cnt + SCHED_ROWS - 1) / SCHED_ROWS * NCH;  // units of work: (tile, chunk), chunk fastest
-      scan_cnt[tid] = cnt;
-      scan_tile[tid] = tiles_e;
+    }
+    // inclusive sums over the experts: within the eight warps that hold them, then over the warps before
+    // (a chain of shuffles and two barriers; eight rounds through shared memory, two barriers each, before. Scan in us 1.2 -> 0.9 at
+    // one token, 6.4 -> 6.1 at 1000; launch, 128-column shard 60 tokens 58.3 -> 57.5, 300 68.7 -> 67.8, 64 of 256 experts 500 74.9 ->
+    // 73.1, together with the slot sum's ranges without a division where there is one)
+    int sum_c = cnt, sum_t = tiles_e;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int vc = __shfl_up_sync(0xFFFFFFFFu, sum_c, d), vt = __shfl_up_sync(0xFFFFFFFFu, sum_t, d);
+      if (lane >= d) { sum_c += vc; sum_t += vt; }
+    }
+    if (warp < E / 32 && lane == 31) { scan_warp[warp] = sum_c; scan_warp[E / 32 + warp] = sum_t; }
+    __syncthreads();
+    if (warp < E / 32) {
+#pragma unroll
+      for (int w = 0; w < E / 32; ++w) {
+        if (w < warp) { sum_c += scan_warp[w]; sum_t += scan_warp[E / 32 + w]; }
+      }
+      scan_cnt[tid] = sum_c;
+      scan_tile[tid] = sum_t;
     }
     __syncthreads();
-    for (int d = 1; d < E; d <<= 1) {
-      int vc = 0, vt = 0;
-      if (tid < E && tid >= d) { vc = scan_cnt[tid - d]; vt = scan_tile[tid - d]; }
-      __syncthreads();
-      if (tid < E) { scan_cnt[tid] += vc; scan_tile[tid] += vt; }
-      __syncthreads();
-    }
     // the shared expert's units follow the routed ones in the deal: token tile j (128 tokens), chunk fastest
     int sh_units = 0;
     if (p.sh_on) {
@@ -2576,7 +2588,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     } else if (!tp_on || bid < ncomp) {
       const uint32_t stride = static_cast<uint32_t>(ncomp) * BLOCK;
       for (int c = 0; c < nchunk; ++c) {
-        const uint32_t c_lo = static_cast<uint32_t>(out_vec * c / nchunk), c_hi = static_cast<uint32_t>(out_vec * (c + 1) / nchunk);
+        const uint32_t c_lo = nchunk == 1 ? 0u : static_cast<uint32_t>(out_vec * c / nchunk);
+        const uint32_t c_hi = static_cast<uint32_t>(nchunk == 1 ? out_vec : out_vec * (c + 1) / nchunk);
         int next[TOP_K];
         uint32_t iv = c_lo + static_cast<uint32_t>(bid) * BLOCK + tid;
         if (BY_SLOTS && iv < c_hi) slots_of(iv / HV, next);
