@@ -315,8 +315,8 @@ static_assert(!SORTED_BUILD || ROW_SLOT_BYTES * (N_EPI / 32) <= SA * A_STAGE_BYT
 // us, loads -> copies, H=2048 I=128: 2960 tokens 18.7 -> 16.7 (launch 101.8 -> 100.8), 4000 29.8 -> 23.2 (130.3 -> 125.8), 8192 59 -> 47
 // (213.3 -> 205.8; with a shared expert 240.6 -> 226.6), 20000 136 -> 107 (470 -> 463). Not for rows all over the buffer, where
 // memory pages bound both (sorted rows, 8192 tokens 60 -> 65, H=7168 16384 393 -> 429), nor for ranks that have two rows of eight
-// (33 -> 48). Two or three vectors a thread instead: no difference, slower. An instance of its own, FORM_COPIES: with this code in it too the other one takes
-// 2 to 4 us more a launch at every size (60 tokens 57.7 -> 59.9), for instructions that it fetches and does not need.
+// (33 -> 48). Two or three vectors a thread instead: no difference, slower. An instance of its own, FORM_COPIES: with this code in it
+// too the other one takes 2 to 4 us more a launch at every size (60 tokens 57.7 -> 59.9).
 constexpr bool COPIES_BUILD = !SORTED_BUILD && !EP_BUILD && !PAIR;
 constexpr int sum_cols() {   // the largest part of a row that makes a stage of 32 KB at most, in 16-byte vectors for 256 threads
   int d = 1;
@@ -1169,6 +1169,8 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
 // FORM_SHORT: the instance for batches that are expected to be short. It holds both forms of the expert phase and takes one of
 // them by the units that phase 1 counts. FORM_WHOLE computes whole units only, and computes them faster: inside
 // the first one they take 2 to 4 us more a launch (16 tokens 85 -> 88 us, 64 of 256 experts at 7500 tokens 153 -> 157).
+// FORM_SOLO: a few tokens, the split form alone (solo_split). FORM_COPIES: whole units of 128-column shards, the slot sum through
+// shared memory (COPIES_BUILD). FORM_FEW: whole units of few rows with a weight stage more (AS_GLOBAL).
 template <int FORM>
 __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t dyn_raw[];
@@ -1187,7 +1189,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   constexpr bool COPIES = FORM == FORM_COPIES && COPIES_BUILD;   // the slot sum's rows come through shared memory
   constexpr bool SHARE = (FORM == FORM_WHOLE || COPIES) && SHARE_BUILD;   // units behind the full rounds are shared by several CTAs
   constexpr bool REST = SORTED && REST_BUILD;   // what is left behind the full rounds of units can be split
-  constexpr bool AS_GLOBAL = (FORM == FORM_SHORT || FORM == FORM_FEW) && mono::AS_GLOBAL;   // activation scales from global memory, and a weight stage more
+  // activation scales from global memory, and a weight stage more
+  constexpr bool AS_GLOBAL = (FORM == FORM_SHORT || FORM == FORM_FEW) && mono::AS_GLOBAL;
   constexpr int SB = AS_GLOBAL ? SB_AG : mono::SB;
   constexpr int RS = (SA < SB) ? SA : SB;  // stages of the router linear's ring
   // 1024-byte aligned base of the operand buffers
