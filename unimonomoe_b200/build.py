@@ -56,7 +56,7 @@ DEV_VARIANTS = {
     **{f"qwen_w1_abl{m}": dict(QWEN, N_HALF=512, E_LOCAL=256, ABLATE=m) for m in (1, 4, 7, 15, 23, 31, 39, 71, 199, 256)},
 }
 
-SOURCES = ["mono_kernel.cu", "ptx_sm100.cuh", "pair_sm100.cuh", "bounded_wait.cuh", "route_math.cuh"]
+SOURCES = ["mono_kernel.cu", "ptx_sm100.cuh", "pair_sm100.cuh", "bounded_wait.cuh", "route_math.cuh", "slot_copies.cuh"]
 
 
 def lib_path(variant: str) -> str:

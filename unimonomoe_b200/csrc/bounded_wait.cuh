@@ -28,6 +28,12 @@ enum StatusCode : uint32_t {
   kErrBounds = 6,        // an index computed on the device fell outside its buffer
 };
 
+// wait sites reported in the status word
+enum Site : uint32_t {
+  kSiteEmptyB = 1, kSiteFullB, kSiteFullA, kSiteEmptyA, kSiteTmemEmpty, kSiteTmemFull, kSiteInterReady,
+  kSiteRouterEmpty, kSiteRouterFull, kSiteRouterAccEmpty, kSiteRouterAccFull, kSiteRowsRead, kSiteSumFull, kSiteSumEmpty,
+};
+
 // Everything is a 4-byte word except the 8-byte time stamps at the (8-byte aligned) end. The words a launch
 // needs at zero come first (kWorkspaceZeroBytes of them): the launcher clears only those; everything behind
 // them is written in full by the kernel before it is read.

@@ -50,6 +50,7 @@
 #include "pair_sm100.cuh"
 #include "ptx_sm100.cuh"
 #include "route_math.cuh"
+#include "slot_copies.cuh"
 
 #ifndef MONO_K_DIM
 #define MONO_K_DIM 2048
@@ -311,26 +312,15 @@ static_assert(!SORTED_BUILD || ROW_SLOT_BYTES * (N_EPI / 32) <= SA * A_STAGE_BYT
 
 // ------------------------------------------------------------------ slot sum through shared memory
 // The slot sum reads each partial row once. Loads of 384 threads keep 48 KB an SM on their way, and that bounds them where a
-// token's rows are neighbours, in slot order; the copy engine keeps 200 KB on its way, in stages of SUM_COLS columns of them. Sum in
+// token's rows are neighbours, in slot order; the copy engine keeps 200 KB on its way, a token's rows (32 to 40 KB) to a stage. Sum in
 // us, loads -> copies, H=2048 I=128: 2960 tokens 18.7 -> 16.7 (launch 101.8 -> 100.8), 4000 29.8 -> 23.2 (130.3 -> 125.8), 8192 59 -> 47
 // (213.3 -> 205.8; with a shared expert 240.6 -> 226.6), 20000 136 -> 107 (470 -> 463). Not for rows all over the buffer, where
 // memory pages bound both (sorted rows, 8192 tokens 60 -> 65, H=7168 16384 393 -> 429), nor for ranks that have two rows of eight
 // (33 -> 48). Two or three vectors a thread instead: no difference, slower. An instance of its own, FORM_COPIES: with this code in it
 // too the other one takes 2 to 4 us more a launch at every size (60 tokens 57.7 -> 59.9).
-constexpr bool COPIES_BUILD = !SORTED_BUILD && !EP_BUILD && !PAIR;
-constexpr int sum_cols() {   // the largest part of a row that makes a stage of 32 KB at most, in 16-byte vectors for 256 threads
-  int d = 1;
-  while (H_DIM % d != 0 || H_DIM / d % 8 != 0 || H_DIM / d * NCH > 2048) ++d;
-  return H_DIM / d;
-}
-constexpr uint32_t kSumItems = 20 * kGrid;   // stages of a launch from which it pays: see above
-constexpr int SUM_COLS = sum_cols(), SUM_PARTS = H_DIM / SUM_COLS;
-constexpr int SUM_ROW_BYTES = SUM_COLS * 2;
-constexpr int SUM_STAGES = 8;             // at most
-constexpr int SUM_WARPS = 8;              // that sum; another one requests the rows
-static_assert(SUM_COLS / 8 <= SUM_WARPS * 32, "a thread has one vector of a part");
-static_assert(TOP_K * NCH <= 32, "a lane requests one row");
-static_assert(2 * ((TOP_K + 1) * NCH + 1) * SUM_ROW_BYTES <= DYN_SMEM - 1024, "two stages at least");
+constexpr bool COPIES_BUILD = ONE_BOX && NP == 1 && NCH == 1 && !EP_BUILD && H_DIM <= 2048;
+constexpr int kCopyTokens = 20 * kGrid;   // smallest batch, measured at H=2048: see above
+static_assert(!COPIES_BUILD || 2 * (TOP_K + 2) * H_DIM * 2 <= DYN_SMEM - 1024, "two stages at least");
 
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t IDESC = umma_idesc_e4m3_f32(PAIR ? 256 : 128, BC);
@@ -353,12 +343,6 @@ constexpr int kSortedTokens = 4096;
 // 1 token 61.6 -> 59.4, 8 90.4 -> 89.7. Not with the router linear inside: 5 tokens 57.7 -> 63.5.
 constexpr int kSoloTokens = 8;
 constexpr uint32_t kSplitCounter = 3;  // workspace counter between the halves of the split form (0-2: grid barriers)
-
-// wait sites reported in the status word
-enum Site : uint32_t {
-  kSiteEmptyB = 1, kSiteFullB, kSiteFullA, kSiteEmptyA, kSiteTmemEmpty, kSiteTmemFull, kSiteInterReady,
-  kSiteRouterEmpty, kSiteRouterFull, kSiteRouterAccEmpty, kSiteRouterAccFull, kSiteRowsRead, kSiteSumFull, kSiteSumEmpty,
-};
 
 struct Params {
   const float* logits;
@@ -657,9 +641,6 @@ __device__ __forceinline__ size_t wsd_index(int e, int chunk, int i) {
 // ------------------------------------------------------------------ shared state
 struct SplitBars {   // split form; its own, since the last arrivals of whole units before it may still be on their way
   uint64_t fullA[SPLIT_SA], emptyA[SPLIT_SA], fullB[SPLIT_SB], emptyB[SPLIT_SB], tmem_full[NBUF], tmem_empty[NBUF];
-};
-struct SumBars {   // slot sum; in the place of gather_tok
-  uint64_t full[SUM_STAGES], empty[SUM_STAGES];
 };
 struct __align__(16) SharedState {
   uint64_t fullA[A_STAGE_CAP], emptyA[A_STAGE_CAP], fullB[B_STAGE_CAP], emptyB[B_STAGE_CAP];
@@ -2372,9 +2353,9 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     else tmem_dealloc(tmem_base, TMEM_COLS);
   }
 
-  SumBars& sum = *reinterpret_cast<SumBars*>(&S.gather_tok);
+  SumBars& sum_bars = *reinterpret_cast<SumBars*>(&S.gather_tok);
   if (COPIES && tid == 0) {   // (nothing of the gather is left)
-    for (int s = 0; s < SUM_STAGES; ++s) { mbar_init(&sum.full[s], 1); mbar_init(&sum.empty[s], SUM_WARPS); }
+    for (int s = 0; s < kSumStages; ++s) { mbar_init(&sum_bars.full[s], 1); mbar_init(&sum_bars.empty[s], kSumWarps); }
     mbar_init_fence();
   }
   alive = grid_sync(wc, 2, &S.flag) && alive;
@@ -2524,68 +2505,10 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     const uint32_t chunk_step = SORTED ? static_cast<uint32_t>(numel + (p.sh_on ? T : 0)) : 1u;
 
     if constexpr (COPIES) {
-      const uint32_t tokens = static_cast<uint32_t>(T);
-      const int sh_rows = p.sh_on ? NCH : 0, stage_rows = TOP_K * NCH + sh_rows + (p.residual != nullptr ? 1 : 0);
-      const uint32_t stage_bytes = static_cast<uint32_t>(stage_rows) * SUM_ROW_BYTES;
-      const uint32_t stages = min(static_cast<uint32_t>(SUM_STAGES), static_cast<uint32_t>(DYN_SMEM - 1024) / stage_bytes);
-      const uint32_t items = tokens * SUM_PARTS;   // (token, part of its rows)
-      const bool sh_all = p.sh_on != 0;
-      auto shared_here = [&](uint32_t tok) { return sh_all && static_cast<int>(tok / TILE_M) % p.sh_parts == p.sh_part; };
+      const SlotCopies<H_DIM, TOP_K, TILE_M, Params> copies(p, sum_bars, wc, dyn, DYN_SMEM - 1024);
       bool ok = true;
-      if (warp == 0) {
-        // the rows were written by other SMs, some by ordinary stores; the copies read them through the async proxy
-        fence_proxy_async();
-        uint32_t n = 0;
-        for (uint32_t item = bid; item < items; item += kGrid, ++n) {
-          const uint32_t st = n % stages, tok = item / SUM_PARTS, col = item % SUM_PARTS * SUM_COLS;
-          const bool sh = shared_here(tok);
-          if (!mbar_wait_warp(&sum.empty[st], ((n / stages) & 1u) ^ 1u, wc, kSiteSumEmpty)) { ok = false; break; }
-          if (lane == 0) mbar_arrive_expect_tx(&sum.full[st], (TOP_K * NCH + (sh ? NCH : 0) + (p.residual != nullptr ? 1 : 0)) * SUM_ROW_BYTES);
-          __syncwarp();
-          const uint32_t dst = dyn_u32 + st * stage_bytes;
-          if (lane < TOP_K * NCH)   // a row each
-            bulk_load(dst + lane * SUM_ROW_BYTES, p.partial + (static_cast<size_t>(tok) * (TOP_K * NCH) + lane) * H_DIM + col, SUM_ROW_BYTES, &sum.full[st]);
-          if (sh && lane < NCH) {
-            const size_t srow = static_cast<size_t>(tokens) * TOP_K + tok;
-            bulk_load(dst + (TOP_K * NCH + lane) * SUM_ROW_BYTES, p.partial + (srow * NCH + lane) * H_DIM + col, SUM_ROW_BYTES, &sum.full[st]);
-          }
-          if (p.residual != nullptr && lane == 0)
-            bulk_load(dst + (TOP_K * NCH + sh_rows) * SUM_ROW_BYTES, p.residual + static_cast<size_t>(tok) * H_DIM + col, SUM_ROW_BYTES, &sum.full[st]);
-        }
-      } else if (warp >= NWARPS - SUM_WARPS) {
-        const int v = tid - (NWARPS - SUM_WARPS) * 32;   // this thread's vector of a part
-        uint32_t n = 0;
-        for (uint32_t item = bid; item < items; item += kGrid, ++n) {
-          const uint32_t st = n % stages, tok = item / SUM_PARTS;
-          if (!mbar_wait(&sum.full[st], (n / stages) & 1u, wc, kSiteSumFull)) { ok = false; break; }
-          if (v < SUM_COLS / W) {
-            const uint8_t* src = dyn + st * stage_bytes + v * 16;
-            float s[W], base[W];
-#pragma unroll
-            for (int i = 0; i < W; ++i) s[i] = base[i] = 0.f;
-            auto add = [&](float (&d)[W], int r) {
-              const uint4 raw = *reinterpret_cast<const uint4*>(src + r * SUM_ROW_BYTES);
-              const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(&raw);
-#pragma unroll
-              for (int i = 0; i < W; ++i) d[i] += __bfloat162float(b[i]);
-            };
-#pragma unroll
-            for (int r = 0; r < TOP_K * NCH; ++r) add(s, r);   // slot-major, chunk-minor
-            if (shared_here(tok)) {
-#pragma unroll
-              for (int c = 0; c < NCH; ++c) add(base, TOP_K * NCH + c);
-            }
-            if (p.residual != nullptr) add(base, TOP_K * NCH + sh_rows);
-            __nv_bfloat16 o[W];
-#pragma unroll
-            for (int i = 0; i < W; ++i)
-              o[i] = __float2bfloat16(sh_all || p.residual != nullptr ? __fmaf_rn(s[i], p.out_scale, base[i]) : __fmul_rn(s[i], p.out_scale));
-            *reinterpret_cast<uint4*>(p.out + static_cast<size_t>(tok) * H_DIM + item % SUM_PARTS * SUM_COLS + v * W) = *reinterpret_cast<const uint4*>(o);
-          }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sum.empty[st]);
-        }
-      }
+      if (warp == 0) ok = copies.request(bid, lane);
+      else if (warp >= NWARPS - kSumWarps) ok = copies.add(bid, tid - (NWARPS - kSumWarps) * 32, lane);
       if (!ok) __nanosleep(200000);   // aborting: copies in flight land
       __syncthreads();
     } else if (!tp_on || bid < ncomp) {
@@ -3213,7 +3136,7 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
     if (p.slot_pos != nullptr) moe_prefill_kernel<FORM_SORTED><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
   }
   // (not with the in-kernel reduce, whose transfer follows the chunks of the loop over the output)
-  const bool copies = COPIES_BUILD && !reduces && static_cast<uint32_t>(num_tokens) * SUM_PARTS >= kSumItems;
+  const bool copies = COPIES_BUILD && !reduces && num_tokens >= kCopyTokens;
   if constexpr (COPIES_BUILD) {
     if (copies) moe_prefill_kernel<FORM_COPIES><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
   }
