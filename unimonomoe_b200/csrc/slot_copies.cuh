@@ -66,7 +66,8 @@ struct SlotCopies {
     uint32_t n = 0;
     for (uint32_t tok = first; tok < tokens; tok += kGrid, ++n) {
       const uint32_t st = n % stages;
-      if (!mbar_wait(&bars.full[st], (n / stages) & 1u, wc, kSiteSumFull)) return false;
+      // the whole warp waits and gives up as one: lanes that left alone would be missed at the __syncwarp below
+      if (!mbar_wait_warp(&bars.full[st], (n / stages) & 1u, wc, kSiteSumFull)) return false;
       if (v < H / W) {
         const uint8_t* src = buf + st * stage_bytes + v * 16;
         float s[W], base[W];
