@@ -120,6 +120,16 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, c
   return true;
 }
 
+// Until this CTA's own copies have come in, `full` counting their bytes, stage n % stages for copy n: those of the last uses of the
+// stages, `used` in all. Whether or not the launch aborts, for a CTA that ended before them would leave its shared memory to them.
+// Nobody has a part in it and it takes microseconds; the limit is for a machine that has stopped answering.
+constexpr uint64_t kDrainNs = 1000000;
+__device__ __forceinline__ void drain_copies(uint64_t* full, uint32_t used, uint32_t stages) {
+  const uint64_t t0 = globaltimer_ns();
+  for (uint32_t n = used > stages ? used - stages : 0u; n < used; ++n)
+    while (!mbar_try_wait(&full[n % stages], (n / stages) & 1u) && globaltimer_ns() - t0 < kDrainNs) {}
+}
+
 // Spin until *p >= target (device scope). False on abort or time-out.
 __device__ __forceinline__ bool wait_counter_ge(const uint32_t* p, uint32_t target, const WaitCtx& c,
                                                 uint32_t code, uint32_t site) {

@@ -2506,10 +2506,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
 
     if constexpr (COPIES) {
       const SlotCopies<H_DIM, TOP_K, TILE_M, Params> copies(p, sum_bars, wc, dyn, DYN_SMEM - 1024);
-      bool ok = true;
-      if (warp == 0) ok = copies.request(bid, lane);
-      else if (warp >= NWARPS - kSumWarps) ok = copies.add(bid, tid - (NWARPS - kSumWarps) * 32, lane);
-      if (!ok) __nanosleep(200000);   // aborting: copies in flight land
+      if (warp == 0) copies.request(bid, lane);
+      else if (warp >= NWARPS - kSumWarps) copies.add(bid, tid - (NWARPS - kSumWarps) * 32, lane);
       __syncthreads();
     } else if (!tp_on || bid < ncomp) {
       const uint32_t stride = static_cast<uint32_t>(ncomp) * BLOCK;

@@ -35,8 +35,8 @@ struct SlotCopies {
     return p.sh_on && static_cast<int>(tok / TILE) % p.sh_parts == p.sh_part;
   }
 
-  // One warp: rows of tokens first, first + kGrid, ... False when the launch aborts.
-  __device__ __forceinline__ bool request(uint32_t first, int lane) const {
+  // One warp: rows of tokens first, first + kGrid, ... until the launch aborts. Behind it all of them have come in.
+  __device__ __forceinline__ void request(uint32_t first, int lane) const {
     static_assert(SLOTS <= 32, "a lane requests one row");
     const uint32_t tokens = static_cast<uint32_t>(p.num_tokens), buf_u32 = smem_u32(buf);
     // the rows were written by other SMs, some by ordinary stores; the copies read them through the async proxy
@@ -45,7 +45,7 @@ struct SlotCopies {
     for (uint32_t tok = first; tok < tokens; tok += kGrid, ++n) {
       const uint32_t st = n % stages;
       const bool sh = shared_row(tok);
-      if (!mbar_wait_warp(&bars.empty[st], ((n / stages) & 1u) ^ 1u, wc, kSiteSumEmpty)) return false;
+      if (!mbar_wait_warp(&bars.empty[st], ((n / stages) & 1u) ^ 1u, wc, kSiteSumEmpty)) break;
       if (lane == 0) mbar_arrive_expect_tx(&bars.full[st], (SLOTS + (sh ? 1 : 0) + (p.residual != nullptr ? 1 : 0)) * ROW_BYTES);
       __syncwarp();
       const uint32_t dst = buf_u32 + st * stage_bytes;
@@ -56,18 +56,18 @@ struct SlotCopies {
       if (p.residual != nullptr && lane == 0)
         bulk_load(dst + (SLOTS + (p.sh_on ? 1 : 0)) * ROW_BYTES, p.residual + static_cast<size_t>(tok) * H, ROW_BYTES, &bars.full[st]);
     }
-    return true;
+    drain_copies(bars.full, n, stages);
   }
 
-  // kSumWarps warps, thread v of them: vector v of the same tokens. False when the launch aborts.
-  __device__ __forceinline__ bool add(uint32_t first, int v, int lane) const {
+  // kSumWarps warps, thread v of them: vector v of the same tokens, until the launch aborts.
+  __device__ __forceinline__ void add(uint32_t first, int v, int lane) const {
     static_assert(H / W <= kSumWarps * 32, "a thread has one vector of a row");
     const uint32_t tokens = static_cast<uint32_t>(p.num_tokens);
     uint32_t n = 0;
     for (uint32_t tok = first; tok < tokens; tok += kGrid, ++n) {
       const uint32_t st = n % stages;
       // the whole warp waits and gives up as one: lanes that left alone would be missed at the __syncwarp below
-      if (!mbar_wait_warp(&bars.full[st], (n / stages) & 1u, wc, kSiteSumFull)) return false;
+      if (!mbar_wait_warp(&bars.full[st], (n / stages) & 1u, wc, kSiteSumFull)) return;
       if (v < H / W) {
         const uint8_t* src = buf + st * stage_bytes + v * 16;
         float s[W], base[W];
@@ -92,7 +92,6 @@ struct SlotCopies {
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars.empty[st]);
     }
-    return true;
   }
 };
 
