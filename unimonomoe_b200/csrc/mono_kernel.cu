@@ -1283,7 +1283,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       constexpr int RCOLS = E / EPI_WGS;
       const uint32_t t_lane = tmem_r + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(h * RCOLS);
       for (int rt = 0; rt < n_rt; ++rt) {
-        if (!mbar_wait(&S.racc_full, static_cast<uint32_t>(rt) & 1u, wc, kSiteRouterAccFull)) break;
+        if (!mbar_wait_warp(&S.racc_full, static_cast<uint32_t>(rt) & 1u, wc, kSiteRouterAccFull)) break;   // a warp's lanes together
         tc_fence_after();
         const int row = c0 + rt * TILE_M + r;
 #pragma unroll
@@ -1969,7 +1969,12 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
       auto up_col = [&](int c) -> uint32_t { return static_cast<uint32_t>(ONE_BOX ? h * HCB + c * (BC / 2) : h * WC + c * LDW); };
       auto down_col = [&](int c) -> uint32_t { return static_cast<uint32_t>(h * WC + c * LDW); };
       uint32_t nt = 0;
-      bool dead = false;  // after an abort: keep the loop structure (named barriers stay matched), skip the work
+      // After an abort: keep the loop structure (named barriers stay matched), skip the work. The lanes of a warp can come out of a
+      // wait with different answers, and the read-out behind it needs them all: one that has given up goes through it once more, and
+      // there the warp learns of it. (8192 tokens of a 128-column shard 204.8 -> 205.3 us, 1000 74.7 -> 75.1; 9 tokens of 256 experts
+      // 63.6 -> 62.2, 1000 160.6 -> 161.5. A wait that votes at every poll: 1000 162.2; a read-out without a branch around it: 500
+      // bytes of spills, 210.)
+      bool dead = false, given_up = false;
       // Accumulators, pairs of adjacent columns. Buffer j of a slab owns acc[j*WC/2, (j+1)*WC/2):
       // first the HCB gate columns (down projection: the first half of WC output columns), then the up columns.
       float2 acc[TCOLS / 2];
@@ -1989,6 +1994,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
         if constexpr ((MONO_ABLATE & 1) != 0) {
           tc_fence_before();
           __syncwarp();
+          dead = __any_sync(0xFFFFFFFFu, given_up);
           if (lane == 0) { if (PAIR && !leader) mbar_arrive_cluster(at_leader(&S.tmem_empty[buf])); else mbar_arrive(&S.tmem_empty[buf]); }
           return;
         }
@@ -2002,6 +2008,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             tc_fence_before();
             __syncwarp();
             if (lane == 0) { if (PAIR && !leader) mbar_arrive_cluster(at_leader(&S.tmem_empty[buf])); else mbar_arrive(&S.tmem_empty[buf]); }
+            dead = __any_sync(0xFFFFFFFFu, given_up);
             TRACE_E(2);
           }
 #pragma unroll
@@ -2124,7 +2131,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
               const uint32_t buf = nt % NBUF;
               TRACE_E(0);
               { PROF_T0();
-              if (!dead && !mbar_wait(&S.tmem_full[buf], (nt / NBUF) & 1u, wc, kSiteTmemFull)) dead = true;
+              if (!dead) given_up = !mbar_wait(&S.tmem_full[buf], (nt / NBUF) & 1u, wc, kSiteTmemFull);
               PROF_ADD(pe_wait); PROF_HIST(0, (ks < 16 ? ks : 15), et == 0); }
               TRACE_E(1);
               PROF_T0();
@@ -2215,7 +2222,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
               const uint32_t buf = nt % NBUF;
               TRACE_E(0);
               { PROF_T0();
-              if (!dead && !mbar_wait(&S.tmem_full[buf], (nt / NBUF) & 1u, wc, kSiteTmemFull)) dead = true;
+              if (!dead) given_up = !mbar_wait(&S.tmem_full[buf], (nt / NBUF) & 1u, wc, kSiteTmemFull);
               PROF_ADD(pe_wait); PROF_HIST(0, 16 + dk, et == 0); }
               TRACE_E(1);
               PROF_T0();
@@ -2226,7 +2233,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             }
           }
           PROF_T0();
-          const bool alive_w = !__any_sync(0xFFFFFFFFu, dead);
+          const bool alive_w = !dead;
           // Neighbouring lanes swap half of their 32-byte pieces first, so that in every store instruction
           // lanes 2i and 2i+1 write 64 contiguous bytes of ONE row: 16 lines per instruction instead of 32.
           // (only in warp-uniform branches: the shuffles need every lane of the warp.) `row`: this thread's partial row, or
