@@ -21,7 +21,7 @@ def emulation(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["sum", "lanes", "drain"])
+@pytest.mark.parametrize("case", ["sum", "lanes", "drain", "settle"])
 def test_every_lane_comes_to_the_end(emulation, case):
     r = subprocess.run([emulation, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout

@@ -51,3 +51,14 @@ def test_what_skips_a_read_out_is_voted_on():
 def test_mma_warp_waits_together():
     text = "".join(_code("mono_kernel.cu"))
     assert re.search(r"if constexpr \(MONO_MMA_WARP != 0\) return mbar_wait_warp\(bar, parity, wc, site\);", text)
+
+
+def test_announced_copies_are_waited_for():
+    """Every ring that copies are announced on is drained by the role that announced them, and an aborting CTA's pause is one that
+    lasts."""
+    for name in ("mono_kernel.cu", "slot_copies.cuh"):
+        text = "".join(_code(name))
+        announced = set(re.findall(r"mbar_arrive_expect_tx\(&([\w.]+)\[", text))
+        drained = set(re.findall(r"drain_copies\(([\w.]+),", text))
+        assert announced and announced == drained, (name, announced ^ drained)
+        assert "__nanosleep" not in text

@@ -3,6 +3,7 @@
 //   sum    the output is the sum of the rows
 //   lanes  the launch aborts while half of a summing warp sees its barrier complete and the other half does not yet
 //   drain  the launch aborts with copies on their way: none is left when the roles have returned
+//   settle an aborting CTA's pause lasts although the sleep in it ends at once
 // Exit status 0: right; 2: wrong; 3: a whole-warp operation waits for lanes that have left.
 #include <atomic>
 #include <chrono>
@@ -141,6 +142,11 @@ static __nv_bfloat16 value(size_t row, int col, int salt) { return __float2bfloa
 
 int main(int, char** argv) {
   g_case = argv[1];
+  if (g_case == "settle") {
+    const uint64_t t0 = globaltimer_ns();
+    settle();
+    return globaltimer_ns() - t0 >= 200000 ? 0 : 2;
+  }
   const uint32_t first = 77;
   std::vector<__nv_bfloat16> partial(size_t(T) * (SLOTS + 1) * H), residual(size_t(T) * H), out(size_t(T) * H);
   for (uint32_t tok = first; tok < T; tok += kGrid)

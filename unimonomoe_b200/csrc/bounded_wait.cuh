@@ -130,6 +130,13 @@ __device__ __forceinline__ void drain_copies(uint64_t* full, uint32_t used, uint
     while (!mbar_try_wait(&full[n % stages], (n / stages) & 1u) && globaltimer_ns() - t0 < kDrainNs) {}
 }
 
+// Time for what an aborting CTA has issued and nobody waits for; they take microseconds. (__nanosleep alone may return at once.)
+constexpr uint64_t kSettleNs = 200000;
+__device__ __forceinline__ void settle() {
+  const uint64_t t0 = globaltimer_ns();
+  while (globaltimer_ns() - t0 < kSettleNs) __nanosleep(10000);
+}
+
 // Spin until *p >= target (device scope). False on abort or time-out.
 __device__ __forceinline__ bool wait_counter_ge(const uint32_t* p, uint32_t target, const WaitCtx& c,
                                                 uint32_t code, uint32_t site) {

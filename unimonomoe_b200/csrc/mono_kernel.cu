@@ -869,6 +869,7 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
             }
           }
         }
+        drain_copies(S.sp.fullB, nb, SPLIT_SB);
       }
     } else if (warp == WARP_MMA) {
       int steps = 0;
@@ -1253,6 +1254,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             tma_load_2d(&p.tm_rw, static_cast<uint32_t>(ks * 64), 0u, b_ring + st * B_STAGE_BYTES, &S.rfull[st]);
           }
         }
+        drain_copies(S.rfull, n, RS);   // the histograms' memory next
       }
     } else if (warp == WARP_MMA) {
       if (lane == 0) {
@@ -1738,6 +1740,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             }
           }
         }
+        if (!PAIR || leader) drain_copies(S.fullB, nb, SB);   // (the leader's barriers count both halves)
         PROF_STORE(0, pw_emptyB);
       }
     } else if (warp == WARP_MMA) {
@@ -2344,8 +2347,8 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     }
   }
 
-  // teardown of phase 2: when aborting, give in-flight bulk copies and MMAs time to land
-  if (aborted(ws)) __nanosleep(200000);
+  // teardown of phase 2: when aborting, MMAs that nobody has waited for run out
+  if (aborted(ws)) settle();
   tc_fence_before();
   if constexpr (PAIR) cluster_sync_all();  // nothing of the peer is still signalling this CTA, or reading its tensor memory
   else __syncthreads();
