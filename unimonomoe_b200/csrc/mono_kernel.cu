@@ -255,12 +255,16 @@ static_assert(SB >= 2 && SA >= 2, "intermediate too wide for shared memory: shar
 constexpr int DYN_SMEM = 1024 + INTER_BYTES + SA * A_STAGE_BYTES + SB * B_STAGE_BYTES + SCALE_BYTES;
 static_assert(NWARPS * E * 4 <= SA * A_STAGE_BYTES, "phase-0 histograms live in the activation ring");
 // Beside an intermediate of 512 columns the activation scales of K = 7168 (28 KB) take the room of a third weight stage, and two
-// stages keep 64 KB of weights on their way where memory wants 96. Where tiles have few rows (FORM_SHORT, FORM_FEW) a thread loads its
+// stages keep 64 KB of weights on their way where memory wants 96. Where tiles have few rows (FORM_FEW) a thread loads its
 // row's scales from global memory instead, two slab steps ahead. Launch in us, two stages -> three, H=7168, I=512: 64 tokens 606 ->
 // 543, 777 714 -> 642; 32 of 256 experts, I=2048 in chunks: 40 tokens 307 -> 266, 200 350 -> 307, 800 384 -> 342, 2048 418 -> 387, with
 // the shared expert 446 -> 419. With full tiles the loads cost what the stage gives: I=512 2500 tokens 817 -> 833, 4095 1126 -> 1208,
 // 8192 (sorted rows) 1789 -> 1917; 32 of 256 experts 3900 763 -> 742. At I=256 a fourth stage is all there is to gain: 777 tokens 343 ->
 // 346, 2500 418 -> 442.
+// FORM_SHORT, whole units where the device declines the split form: ranks with a part of the experts have that in their second round,
+// with tiles that are full by then (32 of 256 experts 3100 tokens 469 -> 448, uneven 669 -> 650, 3400 uneven 658 -> 639). With all
+// experts its batches have a few tokens and are split, and the loop of the whole units beside it costs the split form registers
+// (I=512: 12 tokens 213 -> 217, 32 352 -> 361, 40 399 -> 408): two stages there.
 constexpr int kFewTokens = 2048;   // half a tile to an expert
 constexpr int SCALE_BYTES_AG = ((2 * WSU_N + 2 * WSD_N) * 4 + 1023) / 1024 * 1024;
 constexpr int SB_AG = (SMEM_AVAIL + SCALE_BYTES - SCALE_BYTES_AG - SA * A_STAGE_BYTES) / B_STAGE_BYTES;
@@ -1172,7 +1176,7 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
   constexpr bool SHARE = (FORM == FORM_WHOLE || COPIES) && SHARE_BUILD;   // units behind the full rounds are shared by several CTAs
   constexpr bool REST = SORTED && REST_BUILD;   // what is left behind the full rounds of units can be split
   // activation scales from global memory, and a weight stage more
-  constexpr bool AS_GLOBAL = (FORM == FORM_SHORT || FORM == FORM_FEW) && mono::AS_GLOBAL;
+  constexpr bool AS_GLOBAL = (FORM == FORM_FEW || (FORM == FORM_SHORT && EP_BUILD)) && mono::AS_GLOBAL;
   constexpr int SB = AS_GLOBAL ? SB_AG : mono::SB;
   constexpr int RS = (SA < SB) ? SA : SB;  // stages of the router linear's ring
   // 1024-byte aligned base of the operand buffers
