@@ -151,7 +151,7 @@ int prefill_wgmma_tp_has_devseq(void);        /* Q:1771 */
 int prefill_wgmma_tp_seq_bytes(void);         /* Q:1774 */
 int prefill_wgmma_tp_has_residual(void);      /* Q:1779 */
 int prefill_wgmma_tp_pad_words(int nchunk, int ncomm, int world); /* Q:1782-1784 */
-int prefill_wgmma_up_pipe(void);              /* Q:1786; weight ring depth */
+int prefill_wgmma_up_pipe(void);              /* Q:1786; weight ring depth of whole units (instances for short batches have more) */
 int prefill_wgmma_dn_pipe(void);              /* Q:1787; weight ring depth (one ring serves both phases) */
 int prefill_wgmma_a_stages(void);             /* Q:1788; activation ring depth */
 int prefill_wgmma_shm_total(void);            /* Q:1789 */
@@ -241,6 +241,9 @@ int prefill_wgmma_partial_chunks(void);
 int prefill_wgmma_block_threads(void);        /* threads per CTA */
 int prefill_wgmma_list_places(int units);     /* longest per-CTA unit list of a large batch */
 int prefill_wgmma_list_room(void);            /* places of a list: never fewer */
+/* The instance of the kernel that the calling thread's last launch ran: 0 whole units, 1 short batches, 2 sorted rows,
+ * 3 slot sum through shared memory, 4 a few tokens, 5 whole units of few rows; -1 before the first launch and after a refused one. */
+int prefill_wgmma_launched_form(void);
 int prefill_wgmma_stable_sort(void);          /* 1 = sorted_token_ids is deterministic (stable) */
 /* The workspace that every launch accepts (230 KB); the rest of prefill_wgmma_workspace_bytes() is the intermediate of
  * the split form: 10 MB, 5 MB at N_HALF = 256, none at 128 and in the two-CTA build, which have no split form. */

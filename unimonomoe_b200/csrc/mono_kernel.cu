@@ -2751,6 +2751,7 @@ std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;
 unsigned long long g_map_hits = 0, g_map_misses = 0;
 constexpr size_t kMaxCachedMaps = 4096;   // far more than the MoE layers of a model; beyond it the table restarts
 bool g_attr_set[64] = {};
+thread_local int t_form = -1;   // instance of this thread's last launch
 
 // Copies the cached descriptor into *dst, encoding it first if this tensor has not been seen.
 int cached_map(CUtensorMap* dst, int kind, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
@@ -2882,6 +2883,8 @@ int prefill_wgmma_block_threads() { return BLOCK; }
 int prefill_wgmma_list_places(int units) { return list_places(units); }
 int prefill_wgmma_list_room() { return MAX_MY_TILES; }
 int prefill_wgmma_stable_sort() { return 1; }
+// The instance that the calling thread's last launch ran (Form), -1 before the first and after one that was refused.
+int prefill_wgmma_launched_form() { return t_form; }
 // Byte offset of the 32-bit status word inside the workspace and the bytes that follow it
 // (status, abort flag, two detail words). 0 after a successful launch.
 int prefill_wgmma_status_offset() { return static_cast<int>(offsetof(Workspace, status)); }
@@ -2953,6 +2956,7 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
                                     const int32_t* expert_map, cudaStream_t stream,
                                     const SharedExpertArgs* sh = nullptr, void* tp_peers = nullptr) {
   (void)block_m;  // the tile height is the compiled TILE_M
+  t_form = -1;
   if (router_w != nullptr && PAIR) return -106;  // the pair build has no router linear
   if (sh != nullptr && PAIR) return -108;        // nor the shared expert
   if (router_w != nullptr) logits = logits_buf;
@@ -3130,6 +3134,7 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
       return -107;
     }
     err = cudaLaunchKernelEx(&cfg, moe_prefill_kernel<FORM_WHOLE>, p);
+    t_form = FORM_WHOLE;
     if (err != cudaSuccess) {
       fprintf(stderr, "kernel launch failed: %s\n", cudaGetErrorString(err));
       return static_cast<int>(err);
@@ -3137,28 +3142,31 @@ static int launch_common(const void* router_w, float* logits_buf, const float* l
     return 0;
   }
   const bool reduces = p.tp_mc != nullptr && p.tp_pads != nullptr && p.tp_ncomm > 0;
+  Form form = FORM_WHOLE;
+  if (p.slot_pos != nullptr) {
+    form = FORM_SORTED;
+  } else if (short_batch) {
+    form = !reduces && router_w == nullptr && solo_split(num_tokens, static_cast<int>(sh_tiles) * NCH) ? FORM_SOLO : FORM_SHORT;
+  } else if (COPIES_BUILD && !reduces && num_tokens >= kCopyTokens) {
+    form = FORM_COPIES;   // (not with the in-kernel reduce, whose transfer follows the chunks of the loop over the output)
+  } else if (AS_GLOBAL && num_tokens <= kFewTokens) {
+    form = FORM_FEW;
+  }
   if constexpr (SPLIT_BUILD) {
-    if (short_batch && !reduces && router_w == nullptr && solo_split(num_tokens, static_cast<int>(sh_tiles) * NCH)) {
-      moe_prefill_kernel<FORM_SOLO><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
-    } else if (short_batch) {
-      moe_prefill_kernel<FORM_SHORT><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
-    }
+    if (form == FORM_SOLO) moe_prefill_kernel<FORM_SOLO><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
+    if (form == FORM_SHORT) moe_prefill_kernel<FORM_SHORT><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
   }
   if constexpr (SORTED_BUILD) {
-    if (p.slot_pos != nullptr) moe_prefill_kernel<FORM_SORTED><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
+    if (form == FORM_SORTED) moe_prefill_kernel<FORM_SORTED><<<kGrid, BLOCK, SHORT_DYN_SMEM, stream>>>(p);
   }
-  // (not with the in-kernel reduce, whose transfer follows the chunks of the loop over the output)
-  const bool copies = COPIES_BUILD && !reduces && num_tokens >= kCopyTokens;
   if constexpr (COPIES_BUILD) {
-    if (copies) moe_prefill_kernel<FORM_COPIES><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
+    if (form == FORM_COPIES) moe_prefill_kernel<FORM_COPIES><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
   }
-  const bool few = AS_GLOBAL && num_tokens <= kFewTokens;
-  if (!short_batch && p.slot_pos == nullptr && !copies) {
-    if constexpr (AS_GLOBAL) {
-      if (few) moe_prefill_kernel<FORM_FEW><<<kGrid, BLOCK, FEW_DYN_SMEM, stream>>>(p);
-    }
-    if (!few) moe_prefill_kernel<FORM_WHOLE><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
+  if constexpr (AS_GLOBAL) {
+    if (form == FORM_FEW) moe_prefill_kernel<FORM_FEW><<<kGrid, BLOCK, FEW_DYN_SMEM, stream>>>(p);
   }
+  if (form == FORM_WHOLE) moe_prefill_kernel<FORM_WHOLE><<<kGrid, BLOCK, DYN_SMEM, stream>>>(p);
+  t_form = form;
   err = cudaGetLastError();
   if (err != cudaSuccess) {
     fprintf(stderr, "kernel launch failed: %s\n", cudaGetErrorString(err));
