@@ -873,7 +873,6 @@ __device__ __forceinline__ void split_phase(const Params& p, SharedState& S, con
             }
           }
         }
-        drain_copies(S.sp.fullB, nb, SPLIT_SB);
       }
     } else if (warp == WARP_MMA) {
       int steps = 0;
@@ -1744,7 +1743,6 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
             }
           }
         }
-        if (!PAIR || leader) drain_copies(S.fullB, nb, SB);   // (the leader's barriers count both halves)
         PROF_STORE(0, pw_emptyB);
       }
     } else if (warp == WARP_MMA) {
@@ -2351,7 +2349,9 @@ __global__ void __launch_bounds__(BLOCK, 1) moe_prefill_kernel(const __grid_cons
     }
   }
 
-  // teardown of phase 2: when aborting, MMAs that nobody has waited for run out
+  // Teardown of phase 2. Where a role has given up, the flag is up by now, and weight copies and MMAs that nobody waits for any more
+  // get the time that they take. (Weights waited for by the role that requests them, as in phase R: 64 of 256 experts 20 tokens 51.0
+  // -> 52.5 us, 1000 75.0 -> 76.1, in the mean over 28 sizes 0.5 %.)
   if (aborted(ws)) settle();
   tc_fence_before();
   if constexpr (PAIR) cluster_sync_all();  // nothing of the peer is still signalling this CTA, or reading its tensor memory
