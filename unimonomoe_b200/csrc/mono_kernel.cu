@@ -97,16 +97,15 @@
 
 #ifdef MONO_PROFILE
 #define PROF_DECL(n) long long n = 0
-#define PROF_T0() const long long prof_t0_ = clock64()
-#define PROF_ADD(n) n += clock64() - prof_t0_
-#ifdef MONO_TRACE
-#define PROF_STORE(slot, n)
-#else
-#define PROF_STORE(slot, n) p.ws->prof[blockIdx.x][slot] = static_cast<uint64_t>(n)
-#endif
-#define PROF_HIST(row, bin, who) do { if (who) S.whist[row][bin] += static_cast<unsigned long long>(clock64() - prof_t0_); } while (0)
 #else
 #define PROF_DECL(n)
+#endif
+#if defined(MONO_PROFILE) && !defined(MONO_TRACE)   // (a trace has its stamps and no counters beside them)
+#define PROF_T0() const long long prof_t0_ = clock64()
+#define PROF_ADD(n) n += clock64() - prof_t0_
+#define PROF_STORE(slot, n) p.ws->prof[blockIdx.x][slot] = static_cast<uint64_t>(n)
+#define PROF_HIST(row, bin, who) do { if (who) S.whist[row][bin] += static_cast<unsigned long long>(clock64() - prof_t0_); } while (0)
+#else
 #define PROF_T0()
 #define PROF_ADD(n)
 #define PROF_STORE(slot, n)
@@ -256,16 +255,18 @@ constexpr int DYN_SMEM = 1024 + INTER_BYTES + SA * A_STAGE_BYTES + SB * B_STAGE_
 static_assert(NWARPS * E * 4 <= SA * A_STAGE_BYTES, "phase-0 histograms live in the activation ring");
 // Beside an intermediate of 512 columns the activation scales of K = 7168 (28 KB) take the room of a third weight stage, and two
 // stages keep 64 KB of weights on their way where memory wants 96. Where tiles have few rows (FORM_FEW) a thread loads its
-// row's scales from global memory instead, two slab steps ahead. Launch in us, two stages -> three, H=7168, I=512: 64 tokens 606 ->
-// 543, 777 714 -> 642; 32 of 256 experts, I=2048 in chunks: 40 tokens 307 -> 266, 200 350 -> 307, 800 384 -> 342, 2048 418 -> 387, with
-// the shared expert 446 -> 419. With full tiles the loads cost what the stage gives: I=512 2500 tokens 817 -> 833, 4095 1126 -> 1208,
-// 8192 (sorted rows) 1789 -> 1917; 32 of 256 experts 3900 763 -> 742. At I=256 a fourth stage is all there is to gain: 777 tokens 343 ->
-// 346, 2500 418 -> 442.
+// row's scales from global memory instead, two slab steps ahead. Launch in us, two stages -> three, H=7168, I=512: 64 tokens 581 ->
+// 505, 777 663 -> 582, 2048 732 -> 649; 32 of 256 experts, I=2048 in chunks: 40 tokens 303 -> 232, 200 344 -> 274, 800 374 -> 309, 2048
+// with uneven routing 530 -> 468, with the shared expert 433 -> 411. kFewTokens is a bound for every geometry: beyond it all experts
+// gain for a while and then lose (I=512 2100 tokens 709 -> 664, 2500 747 -> 699, 3000 784 -> 773, uneven 995 -> 1009, 4000 1057 ->
+// 1088; with uneven routing 2048 831 to 866 -> 835 to 874), 32 of 256 experts gain up to the sorted rows (2100 422 -> 381, 3000 471 -> 444, 4000
+// 759 -> 760, uneven 741 -> 684). Sorted rows at I=512, 8192 tokens: 1789 -> 1917. At I=256 a fourth stage is all there is to gain: 777
+// tokens 343 -> 346, 2500 418 -> 442.
 // FORM_SHORT, whole units where the device declines the split form: ranks with a part of the experts have that in their second round,
 // with tiles that are full by then (32 of 256 experts 3100 tokens 469 -> 448, uneven 669 -> 650, 3400 uneven 658 -> 639). With all
 // experts its batches have a few tokens and are split, and the loop of the whole units beside it costs the split form registers
 // (I=512: 12 tokens 213 -> 217, 32 352 -> 361, 40 399 -> 408): two stages there.
-constexpr int kFewTokens = 2048;   // half a tile to an expert
+constexpr int kFewTokens = 2048;   // half a tile to an expert: see above
 constexpr int SCALE_BYTES_AG = ((2 * WSU_N + 2 * WSD_N) * 4 + 1023) / 1024 * 1024;
 constexpr int SB_AG = (SMEM_AVAIL + SCALE_BYTES - SCALE_BYTES_AG - SA * A_STAGE_BYTES) / B_STAGE_BYTES;
 constexpr bool AS_GLOBAL = SB == 2 && SB_AG > SB && MONO_ABLATE == 0;
@@ -318,7 +319,7 @@ static_assert(!SORTED_BUILD || ROW_SLOT_BYTES * (N_EPI / 32) <= SA * A_STAGE_BYT
 // The slot sum reads each partial row once. Loads of 384 threads keep 48 KB an SM on their way, and that bounds them where a
 // token's rows are neighbours, in slot order; the copy engine keeps 200 KB on its way, a token's rows (32 to 40 KB) to a stage. Sum in
 // us, loads -> copies, H=2048 I=128: 2960 tokens 18.7 -> 16.7 (launch 101.8 -> 100.8), 4000 29.8 -> 23.2 (130.3 -> 125.8), 8192 59 -> 47
-// (213.3 -> 205.8; with a shared expert 240.6 -> 226.6), 20000 136 -> 107 (470 -> 463). Not for rows all over the buffer, where
+// (213.3 -> 205.8; with a shared expert 240.6 -> 226.6), 20000 137 -> 103 (464 -> 461). Not for rows all over the buffer, where
 // memory pages bound both (sorted rows, 8192 tokens 60 -> 65, H=7168 16384 393 -> 429), nor for ranks that have two rows of eight
 // (33 -> 48). Two or three vectors a thread instead: no difference, slower. An instance of its own, FORM_COPIES: with this code in it
 // too the other one takes 2 to 4 us more a launch at every size (60 tokens 57.7 -> 59.9).
