@@ -43,7 +43,7 @@ static void __threadfence() {}
 static void __syncthreads() {}
 static void __nanosleep(unsigned) {}   // may end at once
 static uint64_t real_ns() { return std::chrono::steady_clock::now().time_since_epoch().count(); }
-static uint64_t globaltimer_ns() { return real_ns() / 1000; }   // so slow that no limit is met by the host's own pace
+static uint64_t globaltimer_ns() { return real_ns() / 5000; }   // so slow that no limit is met by the host's own pace
 
 // ---- warps
 struct Warp {
@@ -115,7 +115,7 @@ static bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     phase = g_bars[bar].phase;
     done = (phase & 1u) != parity;
   }
-  if (!done) std::this_thread::yield();
+  if (!done) std::this_thread::sleep_for(std::chrono::microseconds(50));
   if (bar == g_late && threadIdx.x / 32 == 6 && lane_ < 16 && phase >= 2) { raise_abort(); return false; }
   return done;
 }
@@ -177,11 +177,11 @@ int main(int, char** argv) {
       {
         std::lock_guard<std::mutex> l(g_m);
         // drain: what the third round of the stages asks for lands a while after the abort
-        const bool held = g_case == "drain" && landed >= 100 && (g_abort_ns == 0 || real_ns() - g_abort_ns < 50000000);
+        const bool held = g_case == "drain" && landed >= 100 && (g_abort_ns == 0 || real_ns() - g_abort_ns < 400000000);
         if (held && g_copies.size() >= 30) raise_abort();
         if (!held && !g_copies.empty()) { c = g_copies.back(); g_copies.pop_back(); }
       }
-      if (c.dst == nullptr) { std::this_thread::yield(); continue; }
+      if (c.dst == nullptr) { std::this_thread::sleep_for(std::chrono::microseconds(20)); continue; }
       memcpy(c.dst, c.src, c.bytes);
       ++landed;
       std::lock_guard<std::mutex> l(g_m);
